@@ -44,7 +44,8 @@ struct Geom {
   int32_t supp, nplanes, nbuckets;  // nbuckets = max(nplanes, 1)
   int32_t log2tile, ntu, ntv, L;    // L = tile + supp - 1
   // Sub-tiles of a tile, sube cells square: nsub_side along each side, nsub
-  // in all (sub-tile (a, b) of a tile is a * nsub_side + b).
+  // in all (the sub-tile a along u, b along v of a tile is b * nsub_side + a:
+  // consecutive bins run along u).
   int32_t sube, nsub_side, nsub;
   int32_t ne;                       // rows of even (and of odd) coefficients
   int32_t do_wgridding, shifting, lmshift, divide_by_n;

@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(F64_BATCH, 12)
 #pragma unroll
     for (int c = 0; c < 2; c++) acc[p][c][0] = acc[p][c][1] = 0.0;
   uint32_t gcur = INACTIVE;
-  int su0 = 0, sv0 = 0, mpc = 0;
+  int rb = 0, su0 = 0, sv0 = 0, mpc = 0;
 
   // This round's inputs are in pre (copied asynchronously); nidx is the next
   // round's index.
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(F64_BATCH, 12)
 #pragma unroll
           for (int c = 0; c < 2; c++) acc[p][c][0] = acc[p][c][1] = 0.0;
         gcur = gk;
-        window_of(g, gk, nbins, su0, sv0, mpc);
+        window_of(g, gk, nbins, rb, su0, sv0, mpc);
       }
       const unsigned m = __ballot_sync(0xffffffffu, lane >= q && lane < nb && st.key[lane] == gk);
       const int len = __popc(m);

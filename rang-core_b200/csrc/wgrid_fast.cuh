@@ -255,7 +255,7 @@ struct VisRecord {
   float x0, y0, xw;  // tap arguments (taps_uv, w_factor's locz of the first plane)
   uint32_t idx;      // visibility index, row * nchan + channel
   float ph_re, ph_im;  // shift phase (shift_phase with sign +1), (1, 0) without shifts
-  uint32_t meta;     // du | dv << 4 | (w was flipped) << 8 | first plane << 16
+  uint32_t meta;     // du | dv << 4 | (w was flipped) << 8 | su mod 8 << 9 | first plane << 16
   uint32_t bin;      // the sorted key (chunk * nbins + bin)
 };
 static_assert(sizeof(VisRecord) == 32, "records are one 32-byte sector");
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(256, COUNT_BLOCKS)
         const int mp = WPL ? minplane(g, w) : 0;
         // The key of bin_of_rc (Setup::locate refined by the sub-tile).
         k = (((su >> g.log2tile) * (uint32_t)g.ntv + (sv >> g.log2tile)) * (uint32_t)g.nbuckets + (uint32_t)mp) *
-                (uint32_t)g.nsub + sa * (uint32_t)g.nsub_side + sb;
+                (uint32_t)g.nsub + sb * (uint32_t)g.nsub_side + sa;
         if (CHUNKED) k += (rc.row / rows_per_chunk) * nbins;
         // The record's two 16-byte halves, formed in registers (VisRecord's
         // field order).
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(256, COUNT_BLOCKS)
           ph_im = ph.im;
         }
         const uint32_t meta = ((su & tmask) - sa * se) | (((sv & tmask) - sb * se) << 4) |
-                              (imflip < 0.0 ? 256u : 0u) | ((uint32_t)mp << 16);
+                              (imflip < 0.0 ? 256u : 0u) | ((su & 7u) << 9) | ((uint32_t)mp << 16);
         reinterpret_cast<uint4*>(rec + i)[0] =
             make_uint4(__float_as_uint(x0), __float_as_uint(y0), __float_as_uint(xw), (uint32_t)i);
         reinterpret_cast<uint4*>(rec + i)[1] = make_uint4(__float_as_uint(ph_re), __float_as_uint(ph_im), meta, k);
@@ -416,11 +416,13 @@ __device__ __forceinline__ cplx<float> record_value(const VisRecord& r, const In
   return {pr, pi * flip};
 }
 
-// The window of a bin key: the grid row and column of its cell (0, 0) (the
-// sub-tile's first cell; windows are 8 x 8) and its first plane.
+// The window of a bin key: its first row on the shifted indices (rb), the grid
+// row and column of its cell (0, 0) (the sub-tile's first cell; windows are
+// 8 x 8) and its first plane. Within a tile, first plane and sub-tile column
+// (a strip) the keys ascend along u.
 template <class T>
-__device__ __forceinline__ void window_of(const Geom<T>& g, uint32_t key, uint32_t nbins, int& su0, int& sv0,
-                                          int& mp) {
+__device__ __forceinline__ void window_of(const Geom<T>& g, uint32_t key, uint32_t nbins, int& rb, int& su0,
+                                          int& sv0, int& mp) {
   const uint32_t bin = key % nbins;
   const uint32_t sub = bin % (uint32_t)g.nsub, t = bin / (uint32_t)g.nsub;
   mp = (int)(t % (uint32_t)g.nbuckets);
@@ -428,10 +430,38 @@ __device__ __forceinline__ void window_of(const Geom<T>& g, uint32_t key, uint32
   const uint32_t tu = tile / (uint32_t)g.ntv, tv = tile - tu * (uint32_t)g.ntv;
   // Tiles are laid out on the shifted indices (i0 + n/2) mod n; the grid is
   // stored unshifted.
-  su0 = (int)(((tu << g.log2tile) + (sub / (uint32_t)g.nsub_side) * (uint32_t)g.sube + (uint32_t)(g.nu - g.nu / 2)) %
-              (uint32_t)g.nu);
-  sv0 = (int)(((tv << g.log2tile) + (sub % (uint32_t)g.nsub_side) * (uint32_t)g.sube + (uint32_t)(g.nv - g.nv / 2)) %
+  rb = (int)((tu << g.log2tile) + (sub % (uint32_t)g.nsub_side) * (uint32_t)g.sube);
+  su0 = (int)(((uint32_t)rb + (uint32_t)(g.nu - g.nu / 2)) % (uint32_t)g.nu);
+  sv0 = (int)(((tv << g.log2tile) + (sub / (uint32_t)g.nsub_side) * (uint32_t)g.sube + (uint32_t)(g.nv - g.nv / 2)) %
               (uint32_t)g.nv);
+}
+
+// A warp's window as it moves from bin to bin of the sorted order. Its rows
+// sit at u mod 8 (on the shifted indices), so that the next bin of the same
+// strip, a few rows further along u, keeps every row the two windows share in
+// place: only the rows that leave are written out (gridding), only those that
+// enter are read (degridding).
+struct Window {
+  uint32_t key = INACTIVE, strip = INACTIVE;  // the bin, and its strip (key / nsub_side)
+  int rb = 0, su0 = 0, sv0 = 0, mp = 0;       // window_of
+};
+// Moves to bin `key`; returns the rows the move leaves behind (8: all).
+template <class T>
+__device__ __forceinline__ int window_step(const Geom<T>& g, const Window& w, uint32_t key, uint32_t nbins,
+                                           Window& n) {
+  n.key = key;
+  n.strip = key / (uint32_t)g.nsub_side;
+  if (n.strip == w.strip) {
+    const int adv = (int)(key - w.key) * g.sube;
+    n.rb = w.rb + adv;
+    n.su0 = w.su0 + adv;
+    if (n.su0 >= g.nu) n.su0 -= g.nu;
+    n.sv0 = w.sv0;
+    n.mp = w.mp;
+    return min(adv, 8);
+  }
+  window_of(g, key, nbins, n.rb, n.su0, n.sv0, n.mp);
+  return 8;
 }
 
 // The taps t[0..S) placed at rows [off, off + S) of an 8-row window, zero
@@ -449,7 +479,20 @@ __device__ __forceinline__ void place8(const V (&t)[S], int off, V zero, V (&row
   }
 }
 
-// ------------------------------------------------------------------ integer gridder
+// The taps t[0..S) at rows (r + i) mod 8 of a window, zero elsewhere, in
+// registers (r is a runtime value: three conditional rotations).
+template <int S>
+__device__ __forceinline__ void rotate8(const float (&t)[S], int r, float (&row)[8]) {
+  float a[8], b[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) a[j] = j < S ? t[j < S ? j : 0] : 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; j++) b[j] = (r & 1) ? a[(j + 7) & 7] : a[j];
+#pragma unroll
+  for (int j = 0; j < 8; j++) a[j] = (r & 2) ? b[(j + 6) & 7] : b[j];
+#pragma unroll
+  for (int j = 0; j < 8; j++) row[j] = (r & 4) ? a[(j + 4) & 7] : a[j];
+}
 
 // ------------------------------------------------------------------ prefetch
 
@@ -528,17 +571,19 @@ __device__ __forceinline__ cplx<float> prefetched_vis(const Prefetched& p, const
 
 // ------------------------------------------------------------------ integer gridder
 
-constexpr int I8_BATCH = 32;         // records staged per round, one per lane
-constexpr uint32_t I8_CHUNK = 8192;  // sorted records per warp
+// Warps per block: each takes some of the support's plane pairs, and the block
+// stages its records once, one per thread.
+__host__ __device__ constexpr int i8_warps(int S) { return S >= 7 ? 2 : 1; }
+__host__ __device__ constexpr int i8_pairs(int S) { return ((S + 1) / 2 + i8_warps(S) - 1) / i8_warps(S); }
+__host__ __device__ constexpr int i8_blocks(int S) { return S <= 4 ? 16 : S <= 6 ? 12 : 9; }  // per SM
 constexpr float I8_ASCALE = 4194304.0f;  // 2^22
-// A's integers (w tap x u tap x 2^22, in [-2^16, 2^22 (1 + eps)]) are formed
-// without a conversion instruction: y = x + 2^23 + 2^16 + 0x8080 lies in
-// (2^23, 2^24), where FP32 spacing is 1, so the FFMA that forms x rounds it
-// to the nearest integer, and the bits of y are 0x4B010000 + rint(x) +
-// 0x8080: one IADD gives rint(x) with the offset the balanced limbs need.
-constexpr float I8_AOFF = 8487040.0f;      // 2^23 + 2^16 + 0x8080
-constexpr uint32_t I8_ABIAS = 0x4B010000u;  // bits of 2^23 + 2^16
-__device__ __forceinline__ uint32_t i8_aint(float y) { return __float_as_uint(y) - I8_ABIAS; }
+// A's integers (w tap x u tap x 2^22) are formed without a conversion
+// instruction: y = x + 2^23 + 0x8080 lies in [2^23, 2^24), where FP32 spacing is
+// 1, so the FFMA that forms x rounds it to the nearest integer, and the low
+// three bytes of y's bits are those of rint(x) + 0x8080, the offset the
+// balanced limbs need. The taps of every kernel of the table are positive on
+// [-1, 1] and at most 1 + eps, so x lies far inside [-0x8080, 2^23 - 0x8080).
+constexpr float I8_AOFF = 8421504.0f;  // 2^23 + 0x8080
 // Row strides (words) of the staging rows: with them the reads of the eight
 // records of a lane quad (slots 4 tq + j) fall in distinct banks.
 constexpr int I8_KU = 10;   // u taps placed on the window's 8 rows
@@ -547,21 +592,22 @@ constexpr int I8_KW = 10;   // w taps * 2^22 (8), as float2 pairs of planes
 
 // Staging of one round: per slot (record) the u taps and value * v taps
 // placed on the window's rows and columns (zero, or the offset, elsewhere),
-// the w taps times 2^22 and the key. Slot I8_BATCH stays zero.
+// the w taps times 2^22 and the key. Slot N, past the N records, stays zero.
+template <int N>
 struct I8Slots {
-  float* ku;      // [I8_BATCH + 1][I8_KU]
-  uint2* bv;      // [I8_BATCH + 1][I8_B]
-  float* kw;      // [I8_BATCH + 1][I8_KW]
-  uint32_t* key;  // [I8_BATCH + 1]
+  float* ku;      // [N + 1][I8_KU]
+  uint2* bv;      // [N + 1][I8_B]
+  float* kw;      // [N + 1][I8_KW]
+  uint32_t* key;  // [N + 1]
   __host__ __device__ static constexpr size_t bytes() {
-    return ((size_t)(I8_BATCH + 1) * (I8_B * 8 + I8_KU * 4 + I8_KW * 4 + 4) + 15) / 16 * 16;
+    return ((size_t)(N + 1) * (I8_B * 8 + I8_KU * 4 + I8_KW * 4 + 4) + 15) / 16 * 16;
   }
   // bv and kw are read as float2: both start on 8-byte boundaries.
   __device__ void carve(unsigned char* base) {
     bv = reinterpret_cast<uint2*>(base);
-    kw = reinterpret_cast<float*>(bv + (I8_BATCH + 1) * I8_B);
-    ku = kw + (I8_BATCH + 1) * I8_KW;
-    key = reinterpret_cast<uint32_t*>(ku + (I8_BATCH + 1) * I8_KU);
+    kw = reinterpret_cast<float*>(bv + (N + 1) * I8_B);
+    ku = kw + (N + 1) * I8_KW;
+    key = reinterpret_cast<uint32_t*>(ku + (N + 1) * I8_KU);
   }
 };
 
@@ -585,64 +631,169 @@ __device__ __forceinline__ void imma(int (&c)[4], uint32_t a0, uint32_t a1, uint
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Adds a bin's exact window sums to the fixed-point grid. acc[h][c][g][r]:
-// plane pair h, component c (re, im), limb group g (weights 2^32, 2^24,
-// 2^16: the grid unit is 2^16 of the products), fragment element r (rows
-// gq / gq + 8 are planes 2h / 2h + 1 at window row gq; columns 2tq, 2tq + 1).
-template <int NP>
-__device__ __forceinline__ void i8_flush(const Geom<float>& g, FixCell* __restrict__ grids, int pg0, int npg,
-                                         int su0, int sv0, int mp, const int (&acc)[NP][2][3][4]) {
-  const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
-  const size_t plane = (size_t)g.nu * g.nv;
-  int row = su0 + gq;
-  if (row >= g.nu) row -= g.nu;
-#pragma unroll
-  for (int h = 0; h < NP; h++)
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int p = mp + 2 * h + (r >> 1);
-      const long long re = ((long long)acc[h][0][0][r] << 16) + ((long long)acc[h][0][1][r] << 8) + acc[h][0][2][r];
-      const long long im = ((long long)acc[h][1][0][r] << 16) + ((long long)acc[h][1][1][r] << 8) + acc[h][1][2][r];
-      if ((re | im) == 0 || p < pg0 || p >= pg0 + npg) continue;
-      int col = sv0 + 2 * tq + (r & 1);
-      if (col >= g.nv) col -= g.nv;
-      fix_add(grids + (size_t)(p - pg0) * plane + (size_t)row * g.nv + col, re, im);
-    }
+__device__ __forceinline__ void imma16(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a0), "r"(a1), "r"(b0));
 }
 
-// Gridding of records [kbase, kend) (single precision): each warp takes
-// I8_CHUNK consecutive sorted records, stages I8_BATCH at a time, and per run
+// Adds the first `leave` rows of a window's exact sums to the fixed-point grid
+// and clears them. acc[h][c][g][r]: plane pair h0 + h, component c (re, im), limb
+// group g (weights 2^32, 2^24, 2^16: the grid unit is 2^16 of the products),
+// fragment element r (rows gq / gq + 8 of the MMA are planes 2h / 2h + 1 at the
+// window row that is gq mod 8; columns 2tq, 2tq + 1).
+//
+// The atomics are what bounds sparse bins: L2 takes about one 32-byte sector
+// per slice and clock, whatever the number of words added in it. Straight
+// from the fragments every 8-byte add was a sector of its own (8 x 8 cells of
+// every plane per bin: 19.6 ms for 1.8 M bins of support 8). Through `buf` a
+// half-warp adds one row of one plane, 128 contiguous bytes, and only the
+// rows the window leaves are added.
+constexpr int I8_FLUSH_BYTES = 8 * 2 * 8 * 16;  // [row][plane of the pair][column] cells
+template <int NP>
+__device__ __forceinline__ void i8_flush(const Geom<float>& g, FixCell* __restrict__ grids, int pg0, int npg,
+                                         const Window& w, int leave, int h0, int (&acc)[NP][2][3][4],
+                                         unsigned long long* buf) {
+  const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+  const int o = (gq - w.rb) & 7;  // this lane's row of the window
+  const int e = lane >> 4, word = lane & 15;
+  int col = w.sv0 + (word >> 1);
+  if (col >= g.nv) col -= g.nv;
+  const size_t plane = (size_t)g.nu * g.nv;
+#pragma unroll
+  for (int h = 0; h < NP; h++) {
+    if (o < leave) {
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const long long re = ((long long)acc[h][0][0][r] << 16) + ((long long)acc[h][0][1][r] << 8) + acc[h][0][2][r];
+        const long long im = ((long long)acc[h][1][0][r] << 16) + ((long long)acc[h][1][1][r] << 8) + acc[h][1][2][r];
+        reinterpret_cast<longlong2*>(buf)[(o * 2 + (r >> 1)) * 8 + 2 * tq + (r & 1)] = make_longlong2(re, im);
+#pragma unroll
+        for (int q = 0; q < 3; q++) acc[h][0][q][r] = acc[h][1][q][r] = 0;
+      }
+    }
+    __syncwarp();
+    const int p = w.mp + 2 * (h0 + h) + e;
+    const bool ok = p >= pg0 && p < pg0 + npg;
+    unsigned long long* base = reinterpret_cast<unsigned long long*>(grids + (size_t)(ok ? p - pg0 : 0) * plane + col) +
+                               (word & 1);
+    for (int i = 0; i < leave; i++) {
+      const unsigned long long v = buf[i * 32 + lane];
+      int row = w.su0 + i;
+      if (row >= g.nu) row -= g.nu;
+      if (ok && v) atomicAdd(base + (size_t)row * g.nv * 2, v);
+    }
+    __syncwarp();
+  }
+}
+
+// The limb products of a run's first 16 HF records (slots q .. q + len - 1 of
+// bin run; the zero slot past them) added to the window's fragments.
+template <int NP, int HF, int N>
+__device__ __forceinline__ void i8_contract(const I8Slots<N>& st, int q, int len, int h0, int (&acc)[NP][2][3][4]) {
+  const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+  // This lane's records: k = 4tq + j and 16 + 4tq + j, j < 4.
+  int slot[4 * HF];
+#pragma unroll
+  for (int j = 0; j < 4 * HF; j++) {
+    const int k = (j < 4 ? 4 * tq : 16 + 4 * tq) + (j & 3);
+    slot[j] = k < len ? q + k : N;
+  }
+  float kuv[4 * HF];
+  uint32_t b[2][3][HF];  // B limbs per component: registers for k 4tq.. and 16 + 4tq..
+#pragma unroll
+  for (int hf = 0; hf < HF; hf++) {
+    uint2 bvv[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      kuv[4 * hf + j] = st.ku[slot[4 * hf + j] * I8_KU + gq];
+      bvv[j] = st.bv[slot[4 * hf + j] * I8_B + gq];
+    }
+    limbs4(bvv[0].x, bvv[1].x, bvv[2].x, bvv[3].x, b[0][0][hf], b[0][1][hf], b[0][2][hf]);
+    limbs4(bvv[0].y, bvv[1].y, bvv[2].y, bvv[3].y, b[1][0][hf], b[1][1][hf], b[1][2][hf]);
+  }
+#pragma unroll
+  for (int h = 0; h < NP; h++) {
+    uint32_t a[3][2 * HF];  // per limb: rows gq (plane 2h), gq + 8 (plane 2h + 1) x k halves
+#pragma unroll
+    for (int hf = 0; hf < HF; hf++) {
+      float2 w[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        w[j] = *reinterpret_cast<const float2*>(st.kw + slot[4 * hf + j] * I8_KW + 2 * (h0 + h));
+      uint32_t x[4], y[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        x[j] = __float_as_uint(fmaf(w[j].x, kuv[4 * hf + j], I8_AOFF));
+        y[j] = __float_as_uint(fmaf(w[j].y, kuv[4 * hf + j], I8_AOFF));
+      }
+      limbs4(x[0], x[1], x[2], x[3], a[0][2 * hf], a[1][2 * hf], a[2][2 * hf]);
+      limbs4(y[0], y[1], y[2], y[3], a[0][2 * hf + 1], a[1][2 * hf + 1], a[2][2 * hf + 1]);
+    }
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      // weight 2^32: a2 b2; 2^24: a2 b1 + a1 b2; 2^16: a2 b0 + a1 b1 + a0 b2
+#pragma unroll
+      for (int gr = 0; gr < 3; gr++)
+#pragma unroll
+        for (int i = 0; i <= gr; i++) {
+          const uint32_t (&av)[2 * HF] = a[2 - i];
+          const uint32_t (&bl)[HF] = b[c][2 - gr + i];
+          if constexpr (HF == 2)
+            imma(acc[h][c][gr], av[0], av[1], av[2], av[3], bl[0], bl[1]);
+          else
+            imma16(acc[h][c][gr], av[0], av[1], bl[0]);
+        }
+    }
+  }
+}
+
+// A barrier of W warps.
+template <int W>
+__device__ __forceinline__ void block_sync() {
+  if constexpr (W == 1)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
+// Gridding of records [kbase, kend) (single precision): each block takes
+// `chunk` consecutive sorted records, stages one per thread at a time, and per run
 // of one bin forms the integer limbs of A (rows: w tap x placed u tap of
 // planes 2h and 2h + 1, columns: the run's records) and B (rows: records,
 // columns: value x placed v tap) and adds their limb products into int32
-// fragments on the tensor cores; at the end of a bin the fragments are
-// combined into int64 and added to the grid. Records outside the run read
-// the zero slot. The next round's records and values are loaded while the
+// fragments on the tensor cores; when the window moves to the next bin, the
+// rows it leaves are combined into int64 and added to the grid. Records
+// outside the run read the zero slot; runs of at most 16 take the MMAs of
+// half the depth. The next round's records and values are loaded while the
 // current round is contracted.
 template <int S>
-__global__ void __launch_bounds__(I8_BATCH, S <= 4 ? 16 : S <= 6 ? 12 : 8)
+__global__ void __launch_bounds__(32 * i8_warps(S), i8_blocks(S))
     k_grid_i8(const __grid_constant__ Geom<float> g, Inputs in, int mode, const VisRecord* __restrict__ rec,
-              const uint32_t* __restrict__ sorted, uint64_t kbase, uint64_t kend, uint32_t nbins,
+              const uint32_t* __restrict__ sorted, uint64_t kbase, uint64_t kend, uint32_t chunk, uint32_t nbins,
               FixCell* __restrict__ grids, int pg0, int npg, FixScale* __restrict__ fs,
               const int* __restrict__ run) {
   static_assert(S >= 1 && S <= 8, "8 x 8 windows");
   if (run && *run == 0) return;  // a speculative pass's regridding, not needed
-  constexpr int NP = (S + 1) / 2;  // plane pairs
+  constexpr int W = i8_warps(S), N = 32 * W;
+  constexpr int NP = i8_pairs(S);  // plane pairs of each warp
   extern __shared__ __align__(16) unsigned char smem[];
-  I8Slots st;
-  st.carve(smem);
-  const int lane = threadIdx.x, gq = lane >> 2, tq = lane & 3;
+  const int tid = threadIdx.x, lane = tid & 31, h0 = (tid >> 5) * NP;
+  unsigned long long* flush_buf = reinterpret_cast<unsigned long long*>(smem + (tid >> 5) * I8_FLUSH_BYTES);
+  I8Slots<N> st;
+  st.carve(smem + W * I8_FLUSH_BYTES);
   {  // the zero slot: u and w taps 0, B rows at the offset (value 0)
-    float* zk = st.ku + I8_BATCH * I8_KU;
-    uint2* zb = st.bv + I8_BATCH * I8_B;
-    float* zw = st.kw + I8_BATCH * I8_KW;
-    if (lane < I8_KU) zk[lane] = 0.0f;
-    if (lane < I8_B) zb[lane] = make_uint2(0x8080u, 0x8080u);
-    if (lane < I8_KW) zw[lane] = 0.0f;
-    if (lane == 0) st.key[I8_BATCH] = INACTIVE;
+    float* zk = st.ku + N * I8_KU;
+    uint2* zb = st.bv + N * I8_B;
+    float* zw = st.kw + N * I8_KW;
+    if (tid < I8_KU) zk[tid] = 0.0f;
+    if (tid < I8_B) zb[tid] = make_uint2(0x8080u, 0x8080u);
+    if (tid < I8_KW) zw[tid] = 0.0f;
+    if (tid == 0) st.key[N] = INACTIVE;
   }
-  const uint64_t k0 = kbase + (uint64_t)blockIdx.x * I8_CHUNK;
-  const uint64_t k1 = min(kend, k0 + I8_CHUNK);
+  const uint64_t k0 = kbase + (uint64_t)blockIdx.x * chunk;
+  const uint64_t k1 = min(kend, k0 + chunk);
   const float bscale = ldexpf(1.0f, fs->sb);
   bool bad = false;
 
@@ -655,22 +806,21 @@ __global__ void __launch_bounds__(I8_BATCH, S <= 4 ? 16 : S <= 6 ? 12 : 8)
       for (int q = 0; q < 3; q++)
 #pragma unroll
         for (int r = 0; r < 4; r++) acc[h][c][q][r] = 0;
-  uint32_t gcur = INACTIVE;
-  int su0 = 0, sv0 = 0, mpc = 0;
+  Window win;
 
   // Rounds ahead: this round's inputs are in pre (copied asynchronously),
   // nidx is the next round's index.
-  Prefetched* pre = reinterpret_cast<Prefetched*>(smem + I8Slots::bytes()) + lane;
+  Prefetched* pre = reinterpret_cast<Prefetched*>(smem + W * I8_FLUSH_BYTES + I8Slots<N>::bytes()) + tid;
   const bool with_vis = mode == VALUE_DATA && in.vis_kind != VIS_UNIT, with_wgt = in.wgt_kind != WGT_NONE;
-  if (k0 + lane < k1) prefetch(pre, rec, in, with_vis, with_wgt, sorted[k0 + lane], k0 + lane);
+  if (k0 + tid < k1) prefetch(pre, rec, in, with_vis, with_wgt, sorted[k0 + tid], k0 + tid);
   cp_async_commit();
-  uint32_t nidx = (k0 + I8_BATCH + lane < k1) ? sorted[k0 + I8_BATCH + lane] : 0u;
+  uint32_t nidx = (k0 + N + tid < k1) ? sorted[k0 + N + tid] : 0u;
 
-  for (uint64_t kb = k0; kb < k1; kb += I8_BATCH) {
-    const int nb = (int)min((uint64_t)I8_BATCH, k1 - kb);
+  for (uint64_t kb = k0; kb < k1; kb += N) {
+    const int nb = (int)min((uint64_t)N, k1 - kb);
     cp_async_wait_all();
-    __syncwarp();
-    if (lane < nb) {  // staging, one record per lane
+    block_sync<W>();
+    if (tid < nb) {  // staging, one record per thread
       const VisRecord r = prefetched_record(*pre);
       const float wt = prefetched_wgt(*pre, in);
       const cplx<float> vv = with_vis ? prefetched_vis(*pre, in) : cplx<float>{1.0f, 0.0f};
@@ -682,7 +832,7 @@ __global__ void __launch_bounds__(I8_BATCH, S <= 4 ? 16 : S <= 6 ? 12 : 8)
       const float pr = r.ph_re * wt, pi = r.ph_im * wt;
       const float vr = vv.re * pr - vv.im * pi, vi = (vv.re * pi + vv.im * pr) * flip;
       bad |= !isfinite(vr) || !isfinite(vi) || !isfinite(r.x0) || !isfinite(r.y0) || !isfinite(r.xw);
-      const int mp = (int)(r.meta >> 16), du = (int)(r.meta & 15u), dv = (int)((r.meta >> 4) & 15u);
+      const int mp = (int)(r.meta >> 16), ur = (int)((r.meta >> 9) & 7u), dv = (int)((r.meta >> 4) & 15u);
       const float br = vr * bscale, bi = vi * bscale;
       uint2 bt[S];
 #pragma unroll
@@ -690,7 +840,7 @@ __global__ void __launch_bounds__(I8_BATCH, S <= 4 ? 16 : S <= 6 ? 12 : 8)
         bt[i] = make_uint2((uint32_t)(__float2int_rn(br * kv[i]) + 0x8080), (uint32_t)(__float2int_rn(bi * kv[i]) + 0x8080));
       float urow[8];
       uint2 brow[8];
-      place8<S>(ku, du, 0.0f, urow);
+      rotate8<S>(ku, ur, urow);
       place8<S>(bt, dv, make_uint2(0x8080u, 0x8080u), brow);
       float wrow[8];
 #pragma unroll
@@ -703,9 +853,9 @@ __global__ void __launch_bounds__(I8_BATCH, S <= 4 ? 16 : S <= 6 ? 12 : 8)
         }
         wrow[j] = w;
       }
-      float2* cu = reinterpret_cast<float2*>(st.ku + lane * I8_KU);
-      uint2* cb = st.bv + lane * I8_B;
-      float2* cw = reinterpret_cast<float2*>(st.kw + lane * I8_KW);
+      float2* cu = reinterpret_cast<float2*>(st.ku + tid * I8_KU);
+      uint2* cb = st.bv + tid * I8_B;
+      float2* cw = reinterpret_cast<float2*>(st.kw + tid * I8_KW);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         cu[j] = make_float2(urow[2 * j], urow[2 * j + 1]);
@@ -713,84 +863,33 @@ __global__ void __launch_bounds__(I8_BATCH, S <= 4 ? 16 : S <= 6 ? 12 : 8)
       }
 #pragma unroll
       for (int j = 0; j < 8; j++) cb[j] = brow[j];
-      st.key[lane] = r.bin;
+      st.key[tid] = r.bin;
     }
     // The next round's record and value, in flight while this one is contracted.
-    __syncwarp();
-    if (kb + I8_BATCH + lane < k1) prefetch(pre, rec, in, with_vis, with_wgt, nidx, kb + I8_BATCH + lane);
+    block_sync<W>();
+    if (kb + N + tid < k1) prefetch(pre, rec, in, with_vis, with_wgt, nidx, kb + N + tid);
     cp_async_commit();
-    if (kb + 2 * I8_BATCH + lane < k1) nidx = sorted[kb + 2 * I8_BATCH + lane];
+    if (kb + 2 * N + tid < k1) nidx = sorted[kb + 2 * N + tid];
     int q = 0;
     while (q < nb) {
       const uint32_t gk = st.key[q];
-      if (gk != gcur) {
-        if (gcur != INACTIVE) i8_flush<NP>(g, grids, pg0, npg, su0, sv0, mpc, acc);
-#pragma unroll
-        for (int h = 0; h < NP; h++)
-#pragma unroll
-          for (int c = 0; c < 2; c++)
-#pragma unroll
-            for (int qq = 0; qq < 3; qq++)
-#pragma unroll
-              for (int r = 0; r < 4; r++) acc[h][c][qq][r] = 0;
-        gcur = gk;
-        window_of(g, gk, nbins, su0, sv0, mpc);
+      if (gk != win.key) {
+        Window next;
+        const int leave = window_step(g, win, gk, nbins, next);
+        if (win.key != INACTIVE) i8_flush<NP>(g, grids, pg0, npg, win, leave, h0, acc, flush_buf);
+        win = next;
       }
-      // The run: slots [q, q + len) of bin gk.
-      const unsigned m = __ballot_sync(0xffffffffu, lane >= q && lane < nb && st.key[lane] == gk);
+      // The run: slots [q, q + len) of bin gk, at most 32.
+      const unsigned m = __ballot_sync(0xffffffffu, q + lane < nb && st.key[q + lane] == gk);
       const int len = __popc(m);
-      // This lane's eight records: k = 4tq + j and 16 + 4tq + j, j < 4.
-      int slot[8];
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int k = (j < 4 ? 4 * tq : 16 + 4 * tq) + (j & 3);
-        slot[j] = (k >= q && k < q + len) ? k : I8_BATCH;
-      }
-      float kuv[8];
-      uint32_t b[2][3][2];  // B limbs per component: registers for k 4tq.. and 16 + 4tq..
-#pragma unroll
-      for (int hf = 0; hf < 2; hf++) {
-        uint2 bvv[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          kuv[4 * hf + j] = st.ku[slot[4 * hf + j] * I8_KU + gq];
-          bvv[j] = st.bv[slot[4 * hf + j] * I8_B + gq];
-        }
-        limbs4(bvv[0].x, bvv[1].x, bvv[2].x, bvv[3].x, b[0][0][hf], b[0][1][hf], b[0][2][hf]);
-        limbs4(bvv[0].y, bvv[1].y, bvv[2].y, bvv[3].y, b[1][0][hf], b[1][1][hf], b[1][2][hf]);
-      }
-#pragma unroll
-      for (int h = 0; h < NP; h++) {
-        uint32_t a[3][4];  // per limb: rows gq (plane 2h), gq + 8 (plane 2h + 1) x k halves
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-          float2 w[4];
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            w[j] = 2 * h < S ? *reinterpret_cast<const float2*>(st.kw + slot[4 * hf + j] * I8_KW + 2 * h)
-                             : make_float2(0.0f, 0.0f);
-          limbs4(i8_aint(fmaf(w[0].x, kuv[4 * hf], I8_AOFF)), i8_aint(fmaf(w[1].x, kuv[4 * hf + 1], I8_AOFF)),
-                 i8_aint(fmaf(w[2].x, kuv[4 * hf + 2], I8_AOFF)), i8_aint(fmaf(w[3].x, kuv[4 * hf + 3], I8_AOFF)),
-                 a[0][2 * hf], a[1][2 * hf], a[2][2 * hf]);
-          limbs4(i8_aint(fmaf(w[0].y, kuv[4 * hf], I8_AOFF)), i8_aint(fmaf(w[1].y, kuv[4 * hf + 1], I8_AOFF)),
-                 i8_aint(fmaf(w[2].y, kuv[4 * hf + 2], I8_AOFF)), i8_aint(fmaf(w[3].y, kuv[4 * hf + 3], I8_AOFF)),
-                 a[0][2 * hf + 1], a[1][2 * hf + 1], a[2][2 * hf + 1]);
-        }
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-          // weight 2^32: a2 b2; 2^24: a2 b1 + a1 b2; 2^16: a2 b0 + a1 b1 + a0 b2
-          imma(acc[h][c][0], a[2][0], a[2][1], a[2][2], a[2][3], b[c][2][0], b[c][2][1]);
-          imma(acc[h][c][1], a[2][0], a[2][1], a[2][2], a[2][3], b[c][1][0], b[c][1][1]);
-          imma(acc[h][c][1], a[1][0], a[1][1], a[1][2], a[1][3], b[c][2][0], b[c][2][1]);
-          imma(acc[h][c][2], a[2][0], a[2][1], a[2][2], a[2][3], b[c][0][0], b[c][0][1]);
-          imma(acc[h][c][2], a[1][0], a[1][1], a[1][2], a[1][3], b[c][1][0], b[c][1][1]);
-          imma(acc[h][c][2], a[0][0], a[0][1], a[0][2], a[0][3], b[c][2][0], b[c][2][1]);
-        }
-      }
+      if (len > 16)
+        i8_contract<NP, 2>(st, q, len, h0, acc);
+      else
+        i8_contract<NP, 1>(st, q, len, h0, acc);
       q += len;
     }
   }
-  if (gcur != INACTIVE) i8_flush<NP>(g, grids, pg0, npg, su0, sv0, mpc, acc);
+  if (win.key != INACTIVE) i8_flush<NP>(g, grids, pg0, npg, win, 8, h0, acc, flush_buf);
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&fs->nonfinite, 1);
 }
 
@@ -972,8 +1071,8 @@ __global__ void __launch_bounds__(H16_BATCH, S <= 6 ? 24 : 12)
       const uint32_t gk = st.key[q];
       if (gk != gcur) {  // load the window of bin gk as FP16 fragments
         gcur = gk;
-        int su0, sv0, mp;
-        window_of(g, gk, nbins, su0, sv0, mp);
+        int rb, su0, sv0, mp;
+        window_of(g, gk, nbins, rb, su0, sv0, mp);
         int row = su0 + gq;
         if (row >= g.nu) row -= g.nu;
         int c0 = sv0 + 2 * tq, c1 = c0 + 1;

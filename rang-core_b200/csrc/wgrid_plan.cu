@@ -389,7 +389,7 @@ __device__ __forceinline__ uint32_t bin_of_rc(const Geom<T>& g, const double* __
   const uint32_t su = (uint32_t)shifted(iu0, g.nu), sv = (uint32_t)shifted(iv0, g.nv);
   const uint32_t tu = su >> g.log2tile, tv = sv >> g.log2tile;
   const uint32_t mask = (1u << g.log2tile) - 1u;
-  const uint32_t sub = ((su & mask) / (uint32_t)g.sube) * (uint32_t)g.nsub_side + (sv & mask) / (uint32_t)g.sube;
+  const uint32_t sub = ((sv & mask) / (uint32_t)g.sube) * (uint32_t)g.nsub_side + (su & mask) / (uint32_t)g.sube;
   if (piu0) *piu0 = iu0;
   if (piv0) *piv0 = iv0;
   return ((tu * (uint32_t)g.ntv + tv) * (uint32_t)g.nbuckets + (uint32_t)minplane(g, w)) * (uint32_t)g.nsub + sub;
@@ -987,9 +987,9 @@ __device__ __forceinline__ void tc_decode(const Geom<float>& g, uint32_t key, in
   const uint32_t tu = tile / (uint32_t)g.ntv, tv = tile - tu * (uint32_t)g.ntv;
   // Tiles are laid out on the shifted indices (i0 + n/2) mod n; the grid
   // itself is stored unshifted.
-  su0 = (int)(((tu << g.log2tile) + (sub / (uint32_t)g.nsub_side) * (uint32_t)g.sube + (uint32_t)(g.nu - g.nu / 2)) %
+  su0 = (int)(((tu << g.log2tile) + (sub % (uint32_t)g.nsub_side) * (uint32_t)g.sube + (uint32_t)(g.nu - g.nu / 2)) %
               (uint32_t)g.nu);
-  sv0 = (int)(((tv << g.log2tile) + (sub % (uint32_t)g.nsub_side) * (uint32_t)g.sube + (uint32_t)(g.nv - g.nv / 2)) %
+  sv0 = (int)(((tv << g.log2tile) + (sub / (uint32_t)g.nsub_side) * (uint32_t)g.sube + (uint32_t)(g.nv - g.nv / 2)) %
               (uint32_t)g.nv);
 }
 
@@ -1068,7 +1068,7 @@ __global__ void __launch_bounds__(TC_BATCH, S <= 6 ? 20 : 12)
         const uint32_t su = (uint32_t)shifted(iu0, g.nu), sv = (uint32_t)shifted(iv0, g.nv);
         const uint32_t sa = (su & tmask) / se, sb = (sv & tmask) / se;
         key = (((su >> g.log2tile) * (uint32_t)g.ntv + (sv >> g.log2tile)) * (uint32_t)g.nbuckets + (uint32_t)mp) *
-                  (uint32_t)g.nsub + sa * (uint32_t)g.nsub_side + sb;
+                  (uint32_t)g.nsub + sb * (uint32_t)g.nsub_side + sa;
         duv = ((su & tmask) - sa * se) | (((sv & tmask) - sb * se) << 8);
         float ku[S], kv[S];
         const float x0 = (float)(-uf * 2.0 + ((double)S - 1.0));
@@ -1277,7 +1277,7 @@ __global__ void __launch_bounds__(TC_BATCH, S <= 5 ? 20 : S == 6 ? 16 : 12)
         const uint32_t su = (uint32_t)shifted(iu0, g.nu), sv = (uint32_t)shifted(iv0, g.nv);
         const uint32_t sa = (su & tmask) / se, sb = (sv & tmask) / se;
         key = (((su >> g.log2tile) * (uint32_t)g.ntv + (sv >> g.log2tile)) * (uint32_t)g.nbuckets + (uint32_t)mp) *
-                  (uint32_t)g.nsub + sa * (uint32_t)g.nsub_side + sb;
+                  (uint32_t)g.nsub + sb * (uint32_t)g.nsub_side + sa;
         duv = ((su & tmask) - sa * se) | (((sv & tmask) - sb * se) << 8);
         float ku[S], kv[S];
         const float x0 = (float)(-uf * 2.0 + ((double)S - 1.0));
@@ -1964,18 +1964,33 @@ void launch_count_rec(const Geom<float>& g, const double4* rowc, const double* f
   }
 }
 
+// Sorted records per block of a kernel whose SMs hold `blocks` of them: sixteen
+// waves where there are records enough, in whole rounds of 32 between 64 and
+// 1024. A block in a sparse region of the uv plane costs several times one in
+// the dense core, so that few long blocks leave the chip idle at the end:
+// 66 M visibilities, 2048^2, support 6: 3.80 ms at 8192 records a block, 3.24
+// at 2048, 3.06 at 1024, 3.09 at 512, 3.45 at 256; support 8, 54 M: 8.7, 6.9,
+// 6.3, 6.1, 6.2 ms. Dense data pay the shorter blocks' starts: 1.06 G
+// visibilities 30.0, 29.7, 30.3, 31.9, 35.4 ms.
+uint32_t warp_chunk(uint64_t n, unsigned blocks) {
+  const uint64_t c = n / (148ull * blocks * 16ull) / 32 * 32;
+  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(c, 64), 1024);
+}
+
 template <int S>
 void launch_grid_i8(cudaStream_t s, const Geom<float>& g, const Inputs& in, int mode, const fast::VisRecord* rec,
                     const uint32_t* sorted, uint64_t kbase, uint64_t kend, uint32_t nbins, fast::FixCell* grids,
                     int pg0, int npg, fast::FixScale* fs, const int* run = nullptr) {
   if (kend <= kbase) return;
-  const int smem = (int)(fast::I8Slots::bytes() + fast::I8_BATCH * sizeof(fast::Prefetched));
-  const unsigned nblocks = (unsigned)((kend - kbase + fast::I8_CHUNK - 1) / fast::I8_CHUNK);
+  constexpr int W = fast::i8_warps(S);
+  const int smem = (int)(W * fast::I8_FLUSH_BYTES + fast::I8Slots<32 * W>::bytes() + 32 * W * sizeof(fast::Prefetched));
+  const uint32_t chunk = warp_chunk(kend - kbase, fast::i8_blocks(S));
+  const unsigned nblocks = (unsigned)((kend - kbase + chunk - 1) / chunk);
   check_cuda(cudaFuncSetAttribute(fast::k_grid_i8<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem");
   {
     StageTimer timer_(ST_GRID, s);
-    fast::k_grid_i8<S><<<nblocks, fast::I8_BATCH, smem, s>>>(g, in, mode, rec, sorted, kbase, kend, nbins, grids,
-                                                             pg0, npg, fs, run);
+    fast::k_grid_i8<S><<<nblocks, 32 * W, smem, s>>>(g, in, mode, rec, sorted, kbase, kend, chunk, nbins,
+                                                             grids, pg0, npg, fs, run);
   }
   check_cuda(cudaGetLastError(), "grid kernel (integer tensor cores)");
 }

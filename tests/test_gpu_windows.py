@@ -1,0 +1,58 @@
+"""The moving windows of the tensor-core gridders and degridders: every
+support they take, visibility counts around a round and a block of records,
+and visibilities spread over the whole grid (sparse bins, tile edges, the
+wrap of rows and columns at the grid's edge), against the CPU oracle."""
+
+import numpy as np
+import pytest
+
+import oracle
+from rang import gridder, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _kernel(supp, single):
+    """A w-gridding kernel row of support `supp` whose oversampling is near 2."""
+    rows = [(abs(r[1] - 2.0), i) for i, r in enumerate(gridder.kernel_table())
+            if r[0] == supp and r[5] == 3 and r[6] == single]
+    return min(rows)[1]
+
+
+def _uv(n, nu, nv, cell, seed):
+    """`n` rows whose u, v cover the grid evenly with clusters at a tile corner
+    and at the grid's edge, and a few w."""
+    rng = np.random.default_rng(seed)
+    u, v = rng.uniform(-0.5, 0.5, n), rng.uniform(-0.5, 0.5, n)
+    k = n // 4
+    u[:k], v[:k] = 0.5 - rng.uniform(0, 4.0 / nu, k), rng.uniform(-2.0, 2.0, k) / nv
+    u[k:2 * k], v[k:2 * k] = (32 + rng.uniform(-4, 4, k)) / nu, (32 + rng.uniform(-4, 4, k)) / nv
+    uvw = np.stack([u / cell, v / cell, rng.uniform(-40.0, 40.0, n)], axis=1)
+    return uvw * (synth.C_LIGHT / 1e9)  # wavelengths at 1 GHz
+
+
+@pytest.mark.parametrize("single", [True, False])
+@pytest.mark.parametrize("supp", [4, 5, 6, 7, 8])
+@pytest.mark.parametrize("n", [1, 33, 64, 65, 1025, 40000])
+def test_windows_match_the_oracle(single, supp, n):
+    nx, ny, cell = 96, 64, 2e-4
+    nu, nv = 216, 150  # neither a multiple of the tile
+    uvw = _uv(n, nu, nv, cell, 17 * supp + n)
+    freq = np.array([1e9])
+    rng = np.random.default_rng(n)
+    vis = rng.standard_normal((n, 1)) + 1j * rng.standard_normal((n, 1))
+    img = rng.standard_normal((nx, ny))
+    wgt = rng.uniform(0.5, 1.5, (n, 1))
+    if single:
+        vis, img, wgt = vis.astype(np.complex64), img.astype(np.float32), wgt.astype(np.float32)
+    kw = dict(uvw=uvw, freq=freq, wgt=wgt, pixsize_x=cell, pixsize_y=cell, epsilon=1e-3,
+              kernel=(_kernel(supp, single), nu, nv))
+    got = gridder.vis2dirty(vis=vis, npix_x=nx, npix_y=ny, **kw)
+    ref = oracle.vis2dirty(vis=vis, npix_x=nx, npix_y=ny, **kw)
+    # The parity tests' bounds: factors in 23 bits (single) or float64, random
+    # signs, no wide-field correction at this field.
+    tol = 2e-5 if single else 1e-9
+    assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+    got = gridder.dirty2vis(dirty=img, **kw)
+    ref = oracle.dirty2vis(dirty=img, **kw)
+    assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
