@@ -255,7 +255,7 @@ struct VisRecord {
   float x0, y0, xw;  // tap arguments (taps_uv, w_factor's locz of the first plane)
   uint32_t idx;      // visibility index, row * nchan + channel
   float ph_re, ph_im;  // shift phase (shift_phase with sign +1), (1, 0) without shifts
-  uint32_t meta;     // du | dv << 4 | (w was flipped) << 8 | su mod 8 << 9 | first plane << 16
+  uint32_t meta;     // dv << 4 | (w was flipped) << 8 | su mod 8 << 9 | first plane << 16
   uint32_t bin;      // the sorted key (chunk * nbins + bin)
 };
 static_assert(sizeof(VisRecord) == 32, "records are one 32-byte sector");
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256, COUNT_BLOCKS)
           ph_re = ph.re;
           ph_im = ph.im;
         }
-        const uint32_t meta = ((su & tmask) - sa * se) | (((sv & tmask) - sb * se) << 4) |
+        const uint32_t meta = (((sv & tmask) - sb * se) << 4) |
                               (imflip < 0.0 ? 256u : 0u) | ((su & 7u) << 9) | ((uint32_t)mp << 16);
         reinterpret_cast<uint4*>(rec + i)[0] =
             make_uint4(__float_as_uint(x0), __float_as_uint(y0), __float_as_uint(xw), (uint32_t)i);
@@ -896,8 +896,8 @@ __global__ void __launch_bounds__(32 * i8_warps(S), i8_blocks(S))
 // ------------------------------------------------------------------ tensor-core degridder
 
 constexpr int H16_BATCH = 32;
-constexpr uint32_t H16_CHUNK = 8192;
 constexpr float H16_BSCALE = 16384.0f;  // 2^14: v taps stay clear of FP16 subnormals
+constexpr int h16_blocks(int S) { return S <= 6 ? 24 : 12; }  // one-warp blocks per SM
 constexpr int H16_KU = 10;  // u taps placed on the window's 8 rows (read as float2)
 constexpr int H16_KV = 10;  // v taps * 2^14 placed on the 8 columns (read as float2)
 constexpr int H16_KW = 12;  // w taps (8, read as float4)
@@ -964,34 +964,35 @@ struct DegridOut {
 };
 
 // Degridding of records [kbase, kend) (single precision, degrid_task_body,
-// wgridder.rs:2793-2901): per bin the warp holds the bin's 8 x 8 window of
-// each plane as FP16 hi + lo fragments (scaled by a power of two to the
-// window's largest value); per block of sixteen records the v contraction
-// T[k][u] = sum_v kv_k[v - dv_k] G_p[u][v] of each plane runs on the tensor
-// cores as hi*hi + hi*lo + lo*hi (mma.sync m16n8k8, records along M, window
-// rows along N, FP32 accumulation, each block from zero); the u and w
+// wgridder.rs:2793-2901): the warp holds the current bin's 8 x 8 window of
+// each plane as FP16 hi + lo fragments, each row (of all planes) scaled by a
+// power of two to its largest value; per block of sixteen records the v
+// contraction T[k][u] = sum_v kv_k[v - dv_k] G_p[u][v] of each plane runs on
+// the tensor cores as hi*hi + hi*lo + lo*hi (mma.sync m16n8k8, records along M,
+// window rows along N, FP32 accumulation, each block from zero); the u and w
 // contractions and the final phase and weight (wgridder.rs:3146-3159) run on
 // the CUDA cores, reduced over the four lanes that hold a record's window
-// rows. Each output depends only on its own record and the window, so the
-// result does not depend on the grouping. With plane groups (first / last)
-// the partial sums accumulate in `vis` and the final factor is applied with
-// the last group. The next round's records are copied while the current
-// round is contracted. `out` says where the results go (DegridOut). Up to
-// support 6, 24 warps per SM (80 registers) measured 4 % faster than 16 (122
+// rows. Window rows sit at u mod 8, so the next bin of a strip reads only the
+// rows it adds. Each output depends only on its own record and its window
+// rows, so the result does not depend on the grouping. With plane groups
+// (first / last) the partial sums accumulate in `vis` and the final factor is
+// applied with the last group. The next round's records are copied while the
+// current round is contracted. `out` says where the results go (DegridOut). Up
+// to support 6, 24 warps per SM (80 registers) measured 4 % faster than 16 (122
 // registers) and 20 (96), and as fast as 28. The w contraction before the u
 // taps and one output lane per record (two lanes of each quad) measured 10 %
 // faster than u first and one lane writing both records.
 template <int S>
-__global__ void __launch_bounds__(H16_BATCH, S <= 6 ? 24 : 12)
+__global__ void __launch_bounds__(H16_BATCH, h16_blocks(S))
     k_degrid_h(const __grid_constant__ Geom<float> g, Inputs wts, const VisRecord* __restrict__ rec,
-               const uint32_t* __restrict__ sorted, uint64_t kbase, uint64_t kend, uint32_t nbins,
+               const uint32_t* __restrict__ sorted, uint64_t kbase, uint64_t kend, uint32_t chunk, uint32_t nbins,
                const cplx<float>* __restrict__ grids, int pg0, int npg, const __grid_constant__ DegridOut out,
                int first, int last, const uint32_t* __restrict__ kb_ptr, const uint32_t* __restrict__ ke_ptr) {
   static_assert(S >= 1 && S <= 8, "8 x 8 windows");
   if (kb_ptr) {  // a range the device computed: the grid covers its largest size
     kbase = *kb_ptr;
     kend = *ke_ptr;
-    if (kbase + (uint64_t)blockIdx.x * H16_CHUNK >= kend) return;
+    if (kbase + (uint64_t)blockIdx.x * chunk >= kend) return;
   }
   extern __shared__ __align__(16) unsigned char smem[];
   H16Slots st;
@@ -1006,13 +1007,14 @@ __global__ void __launch_bounds__(H16_BATCH, S <= 6 ? 24 : 12)
       st.out[H16_BATCH] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   }
-  const uint64_t k0 = kbase + (uint64_t)blockIdx.x * H16_CHUNK;
-  const uint64_t k1 = min(kend, k0 + H16_CHUNK);
+  const uint64_t k0 = kbase + (uint64_t)blockIdx.x * chunk;
+  const uint64_t k1 = min(kend, k0 + chunk);
   const size_t plane = (size_t)g.nu * g.nv;
 
-  uint32_t bhi[S][2], blo[S][2];  // [plane][re/im]: window rows gq, columns 2tq, 2tq + 1
-  float inv = 0.0f;               // 1 / (window scale * 2^14)
-  uint32_t gcur = INACTIVE;
+  uint32_t bhi[S][2], blo[S][2];  // [plane][re/im]: window row gq (mod 8), columns 2tq, 2tq + 1
+  float inv = 0.0f;               // 1 / (row gq's scale * 2^14)
+  float2 invp = {0.0f, 0.0f};     // the same of rows 2tq, 2tq + 1
+  Window win;
   double part = 0.0, vmax = 0.0;  // the stored modes' misfit partial and largest |stored|
 
   Prefetched* pre = reinterpret_cast<Prefetched*>(smem + H16Slots::bytes()) + lane;
@@ -1031,11 +1033,11 @@ __global__ void __launch_bounds__(H16_BATCH, S <= 6 ? 24 : 12)
       float ku[S], kv[S], kw[S];
       eval_taps2<float, S>(g.coeff, g.ne, r.x0, r.y0, ku, kv);
       if (g.do_wgridding) eval_taps1<S>(g.coeff, r.xw, kw);
-      const int mp = (int)(r.meta >> 16), du = (int)(r.meta & 15u), dv = (int)((r.meta >> 4) & 15u);
+      const int mp = (int)(r.meta >> 16), ur = (int)((r.meta >> 9) & 7u), dv = (int)((r.meta >> 4) & 15u);
 #pragma unroll
       for (int i = 0; i < S; i++) kv[i] *= H16_BSCALE;
       float urow[8], vrow[8], wrow[8];
-      place8<S>(ku, du, 0.0f, urow);
+      rotate8<S>(ku, ur, urow);
       place8<S>(kv, dv, 0.0f, vrow);
 #pragma unroll
       for (int j = 0; j < 8; j++) {
@@ -1069,36 +1071,43 @@ __global__ void __launch_bounds__(H16_BATCH, S <= 6 ? 24 : 12)
     int q = 0;
     while (q < nb) {
       const uint32_t gk = st.key[q];
-      if (gk != gcur) {  // load the window of bin gk as FP16 fragments
-        gcur = gk;
-        int rb, su0, sv0, mp;
-        window_of(g, gk, nbins, rb, su0, sv0, mp);
-        int row = su0 + gq;
+      if (gk != win.key) {  // read the rows that bin gk adds to the window, as FP16 fragments
+        Window next;
+        const int enter = window_step(g, win, gk, nbins, next);
+        win = next;
+        const int o = (gq - win.rb) & 7;  // this lane's row of the window
+        const bool mine = o >= 8 - enter;
+        int row = win.su0 + o;
         if (row >= g.nu) row -= g.nu;
-        int c0 = sv0 + 2 * tq, c1 = c0 + 1;
+        int c0 = win.sv0 + 2 * tq, c1 = c0 + 1;
         if (c0 >= g.nv) c0 -= g.nv;
         if (c1 >= g.nv) c1 -= g.nv;
         cplx<float> v[S][2];  // [plane][column]
         float m = 0.0f;
 #pragma unroll
         for (int p = 0; p < S; p++) {
-          const int pp = mp + p;
-          const bool ok = pp >= pg0 && pp < pg0 + npg && (g.do_wgridding || pp == 0);
+          const int pp = win.mp + p;
+          const bool ok = mine && pp >= pg0 && pp < pg0 + npg && (g.do_wgridding || pp == 0);
           const cplx<float>* src = grids + (size_t)(ok ? pp - pg0 : 0) * plane + (size_t)row * g.nv;
           v[p][0] = ok ? src[c0] : cplx<float>{0.0f, 0.0f};
           v[p][1] = ok ? src[c1] : cplx<float>{0.0f, 0.0f};
           m = fmaxf(m, fmaxf(fmaxf(fabsf(v[p][0].re), fabsf(v[p][0].im)), fmaxf(fabsf(v[p][1].re), fabsf(v[p][1].im))));
         }
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        // Largest window value to about 2^14 (FP16 tops out at 65504).
-        const int e = (m > 0.0f && isfinite(m)) ? ilogbf(m) : 0;
-        const float sc = ldexpf(1.0f, 14 - e);
-        inv = ldexpf(1.0f, e - 14) / H16_BSCALE;
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        if (mine) {
+          // The row's largest value to about 2^14 (FP16 tops out at 65504).
+          const int e = (m > 0.0f && isfinite(m)) ? max(ilogbf(m), -100) : 0;
+          const float sc = ldexpf(1.0f, 14 - e);
+          inv = ldexpf(1.0f, e - 14) / H16_BSCALE;
 #pragma unroll
-        for (int p = 0; p < S; p++) {
-          split_h2(v[p][0].re * sc, v[p][1].re * sc, bhi[p][0], blo[p][0]);
-          split_h2(v[p][0].im * sc, v[p][1].im * sc, bhi[p][1], blo[p][1]);
+          for (int p = 0; p < S; p++) {
+            split_h2(v[p][0].re * sc, v[p][1].re * sc, bhi[p][0], blo[p][0]);
+            split_h2(v[p][0].im * sc, v[p][1].im * sc, bhi[p][1], blo[p][1]);
+          }
         }
+        invp.x = __shfl_sync(0xffffffffu, inv, 8 * tq);
+        invp.y = __shfl_sync(0xffffffffu, inv, 8 * tq + 4);
       }
       const unsigned mk = __ballot_sync(0xffffffffu, lane >= q && lane < nb && st.key[lane] == gk);
       const int len = __popc(mk);
@@ -1150,8 +1159,8 @@ __global__ void __launch_bounds__(H16_BATCH, S <= 6 ? 24 : 12)
         float tr[2], ti[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-          tr[h] = fmaf(kup[h].x, wr[h][0], kup[h].y * wr[h][1]);
-          ti[h] = fmaf(kup[h].x, wi[h][0], kup[h].y * wi[h][1]);
+          tr[h] = fmaf(kup[h].x, wr[h][0] * invp.x, kup[h].y * (wr[h][1] * invp.y));
+          ti[h] = fmaf(kup[h].x, wi[h][0] * invp.x, kup[h].y * (wi[h][1] * invp.y));
         }
 #pragma unroll
         for (int h = 0; h < 2; h++)
@@ -1168,7 +1177,7 @@ __global__ void __launch_bounds__(H16_BATCH, S <= 6 ? 24 : 12)
             const uint32_t idx = __float_as_uint(fo.w);
             const uint64_t k = kb + (uint64_t)slot;
             cplx<float>* dst = out.mode == DEGRID_TO_VIS ? out.vis + idx : out.stored + k;
-            cplx<float> accv{(tq ? tr[1] : tr[0]) * inv, (tq ? ti[1] : ti[0]) * inv * fo.z};
+            cplx<float> accv{tq ? tr[1] : tr[0], (tq ? ti[1] : ti[0]) * fo.z};
             if (!first) {
               const cplx<float> prev = *dst;
               accv = {accv.re + prev.re, accv.im + prev.im};
@@ -1252,6 +1261,7 @@ __global__ void __launch_bounds__(STORE_THREADS) k_sum_partials(const double* __
                                                                  double* out) {
   __shared__ double sh[STORE_THREADS];
   double v = 0.0;
+#pragma unroll 8
   for (uint32_t i = threadIdx.x; i < n; i += STORE_THREADS) v += partials[i];
   const double s = block_sum(v, sh);
   if (threadIdx.x == 0) *out = s;

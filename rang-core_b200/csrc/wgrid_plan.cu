@@ -1965,16 +1965,25 @@ void launch_count_rec(const Geom<float>& g, const double4* rowc, const double* f
 }
 
 // Sorted records per block of a kernel whose SMs hold `blocks` of them: sixteen
-// waves where there are records enough, in whole rounds of 32 between 64 and
-// 1024. A block in a sparse region of the uv plane costs several times one in
-// the dense core, so that few long blocks leave the chip idle at the end:
-// 66 M visibilities, 2048^2, support 6: 3.80 ms at 8192 records a block, 3.24
-// at 2048, 3.06 at 1024, 3.09 at 512, 3.45 at 256; support 8, 54 M: 8.7, 6.9,
-// 6.3, 6.1, 6.2 ms. Dense data pay the shorter blocks' starts: 1.06 G
-// visibilities 30.0, 29.7, 30.3, 31.9, 35.4 ms.
+// waves where there are records enough, up to 1024 records, and at most 128
+// waves, in whole rounds of 32 between 64 and 8192. A block in a sparse region
+// of the uv plane costs several times one in the dense core, so that a few long
+// blocks leave the chip idle at the end: gridding 66 M visibilities, 2048^2,
+// support 6, takes 3.80 ms at 8192 records a block, 3.24 at 2048, 3.06 at 1024,
+// 3.09 at 512, 3.45 at 256; support 8, 54 M: 8.7, 6.9, 6.3, 6.1, 6.2 ms. Larger
+// calls have blocks enough and pay the blocks' starts: 1.06 G visibilities 30.0,
+// 29.7, 30.3, 31.9, 35.4 ms.
 uint32_t warp_chunk(uint64_t n, unsigned blocks) {
-  const uint64_t c = n / (148ull * blocks * 16ull) / 32 * 32;
-  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(c, 64), 1024);
+  const uint64_t wave = 148ull * blocks;
+  const uint64_t c = std::max(std::min<uint64_t>(n / (wave * 16), 1024), n / (wave * 128)) / 32 * 32;
+  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(c, 64), 8192);
+}
+
+// The degridder's records per warp, and the blocks (partial sums) it takes for n.
+uint32_t degrid_chunk(int supp, uint64_t n) { return warp_chunk(n, fast::h16_blocks(supp)); }
+uint32_t degrid_parts(int supp, uint64_t n) {
+  const uint32_t c = degrid_chunk(supp, n);
+  return (uint32_t)((n + c - 1) / c);
 }
 
 template <int S>
@@ -2019,12 +2028,13 @@ void launch_degrid_h(cudaStream_t s, const Geom<float>& g, const Inputs& wts, co
   // then only bounds its size (the grid covers kend - kbase records).
   if (kend <= kbase) return;
   const int smem = (int)(fast::H16Slots::bytes() + fast::H16_BATCH * sizeof(fast::Prefetched));
-  const unsigned nblocks = (unsigned)((kend - kbase + fast::H16_CHUNK - 1) / fast::H16_CHUNK);
+  const uint32_t chunk = degrid_chunk(S, kend - kbase);
+  const unsigned nblocks = (unsigned)((kend - kbase + chunk - 1) / chunk);
   check_cuda(cudaFuncSetAttribute(fast::k_degrid_h<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem");
   {
     StageTimer timer_(ST_DEGRID, s);
-    fast::k_degrid_h<S><<<nblocks, fast::H16_BATCH, smem, s>>>(g, wts, rec, sorted, kbase, kend, nbins, grids, pg0,
-                                                               npg, out, first, last, kb_ptr, ke_ptr);
+    fast::k_degrid_h<S><<<nblocks, fast::H16_BATCH, smem, s>>>(g, wts, rec, sorted, kbase, kend, chunk, nbins, grids,
+                                                               pg0, npg, out, first, last, kb_ptr, ke_ptr);
   }
   check_cuda(cudaGetLastError(), "degrid kernel (tensor cores)");
 }
@@ -3006,7 +3016,7 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
           if (fused) {
             out = *static_cast<const fast::DegridOut*>(fused);
             out.block0 = block0;
-            block0 += (uint32_t)((chunk_sorted_[c + 1] - chunk_sorted_[c] + fast::H16_CHUNK - 1) / fast::H16_CHUNK);
+            block0 += degrid_parts(g_.supp, chunk_sorted_[c + 1] - chunk_sorted_[c]);
           } else {
             out.vis = reinterpret_cast<cplx<float>*>(vis);
           }
@@ -3097,9 +3107,11 @@ void Plan<T>::values_pass(bool gram, const Inputs& data, bool sorted_data, const
   }
   if (!sorted_.get()) throw InvalidArgument("this plan was made without the visibility layout");
   const uint64_t nblk = (nvis_ + fast::STORE_CHUNK - 1) / fast::STORE_CHUNK;
-  // Partial sums: one per block of the degridder (its chunks rounded up
-  // separately) or of the value kernels.
-  const size_t nparts_max = nblk + (size_t)nchunk_ + 1;
+  // Partial sums: one per block of the degridder (each row chunk's range
+  // split separately) or of the value kernels.
+  uint32_t ndegrid = 0;
+  for (int c = 0; c < nchunk_; c++) ndegrid += degrid_parts(g_.supp, chunk_sorted_[c + 1] - chunk_sorted_[c]);
+  const size_t nparts_max = std::max<size_t>(nblk, ndegrid);
   if (partials_.size() < nparts_max * sizeof(double)) partials_.alloc(nparts_max * sizeof(double), s);
   if (!res_bound_.get()) res_bound_.alloc(sizeof(fast::ValueBound), s);
   double* partials = partials_.as<double>();
@@ -3118,9 +3130,7 @@ void Plan<T>::values_pass(bool gram, const Inputs& data, bool sorted_data, const
       out.partials = partials;
       out.bound = res_bound_.as<fast::ValueBound>();
       degrid_to(model, none, nullptr, &out, s, nullptr);
-      nparts = 0;
-      for (int c = 0; c < nchunk_; c++)
-        nparts += (uint32_t)((chunk_sorted_[c + 1] - chunk_sorted_[c] + fast::H16_CHUNK - 1) / fast::H16_CHUNK);
+      nparts = ndegrid;
     } else {
       {
         StageTimer timer_(ST_OTHER, s);
