@@ -12,16 +12,19 @@
 // (mma.sync m8n8k4: rows the window's u cells, columns its v cells, k four
 // records: A = w tap x placed u taps, B = value x placed v taps), so the run's
 // sums are formed in one fixed order, in FP64 as the reference forms them.
-// At the end of a run the window is added to the 128-bit fixed-point grid
-// (each sum rounded once into the grid's unit; integer adds, exact in any
-// order), so the result does not depend on how the runs' atomic adds
-// interleave: a call is reproducible bit for bit.
+// When the window moves on, the rows it leaves are added to the 128-bit
+// fixed-point grid (each sum rounded once into the grid's unit; integer adds,
+// exact in any order), so the result does not depend on how the warps' atomic
+// adds interleave: a call is reproducible bit for bit.
 
 namespace fast {
 
 constexpr int F64_BATCH = 32;        // records staged per round, one per lane
-constexpr uint32_t F64_CHUNK = 2048;  // sorted records per warp
-constexpr int F64_ROW = 8;           // doubles per staged row (8 window cells)
+constexpr int F64_BLOCKS = 12;       // one-warp blocks per SM
+// Doubles per staged row of 8: the odd stride spreads the lanes' stores over
+// the banks; the w taps' rows are read as double2.
+constexpr int F64_ROW = 9, F64_KW = 10;
+constexpr int F64_FLUSH_BYTES = 2 * 8 * 8 * 32;  // two planes' cells, [plane][row][column]
 
 // Per slot (record): the u taps placed on the window's 8 rows, Re and Im of
 // value x v taps placed on its 8 columns, the w taps of the S planes (zero
@@ -33,14 +36,14 @@ struct F64Slots {
   double* kw;
   uint32_t* key;
   __host__ __device__ static constexpr size_t bytes() {
-    return ((size_t)(F64_BATCH + 1) * (4 * F64_ROW * 8 + 4) + 15) / 16 * 16;
+    return ((size_t)(F64_BATCH + 1) * ((3 * F64_ROW + F64_KW) * 8 + 4) + 15) / 16 * 16;
   }
   __device__ void carve(unsigned char* base) {
-    ku = reinterpret_cast<double*>(base);
+    kw = reinterpret_cast<double*>(base);
+    ku = kw + (F64_BATCH + 1) * F64_KW;
     bre = ku + (F64_BATCH + 1) * F64_ROW;
     bim = bre + (F64_BATCH + 1) * F64_ROW;
-    kw = bim + (F64_BATCH + 1) * F64_ROW;
-    key = reinterpret_cast<uint32_t*>(kw + (F64_BATCH + 1) * F64_ROW);
+    key = reinterpret_cast<uint32_t*>(bim + (F64_BATCH + 1) * F64_ROW);
   }
 };
 
@@ -112,56 +115,82 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// Adds a run's window sums to the 128-bit grid: acc[p][c][i] is plane
-// mp + p, component c, window row gq and column 2 tq + i.
+// Adds the first `leave` rows of a window's sums to the 128-bit grid and clears
+// them: acc[p][c][i] is plane mp + p, component c, column 2 tq + i of the window
+// row that is gq mod 8. As in i8_flush the adds go through shared memory, a
+// warp adding one row of one plane (256 contiguous bytes): straight from the
+// fragments each 8-byte add was a 32-byte sector of its own in L2, which
+// bound the kernel (4 x 512 adds per bin of support 8).
 template <int S>
 __device__ __forceinline__ void f64_flush(const Geom<double>& g, FixCell2* __restrict__ grids, int pg0, int npg,
-                                          int su0, int sv0, int mp, double sc, const double (&acc)[S][2][2]) {
+                                          const Window& w, int leave, double sc, double (&acc)[S][2][2],
+                                          unsigned long long* buf) {
   const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+  const int o = (gq - w.rb) & 7;  // this lane's row of the window
+  int col = w.sv0 + (lane >> 2);
+  if (col >= g.nv) col -= g.nv;
   const size_t plane = (size_t)g.nu * g.nv;
-  int row = su0 + gq;
-  if (row >= g.nu) row -= g.nu;
 #pragma unroll
-  for (int p = 0; p < S; p++) {
-    const int pp = mp + p;
-    if (pp < pg0 || pp >= pg0 + npg) continue;
+  for (int p2 = 0; p2 < S; p2 += 2) {
+    if (o < leave) {
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const double re = acc[p][0][i], im = acc[p][1][i];
-      if (re == 0.0 && im == 0.0) continue;
-      int col = sv0 + 2 * tq + i;
-      if (col >= g.nv) col -= g.nv;
-      FixTraits<double>::flush(grids + (size_t)(pp - pg0) * plane + (size_t)row * g.nv + col,
-                               FixTraits<double>::term(re, sc), FixTraits<double>::term(im, sc));
+      for (int e = 0; e < 2; e++) {
+        if (p2 + e >= S) break;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const FixWide re = FixTraits<double>::term(acc[p2 + e][0][i], sc);
+          const FixWide im = FixTraits<double>::term(acc[p2 + e][1][i], sc);
+          longlong2* d = reinterpret_cast<longlong2*>(buf + (e * 8 + o) * 32 + (2 * tq + i) * 4);
+          d[0] = make_longlong2(re.lo, re.hi);
+          d[1] = make_longlong2(im.lo, im.hi);
+          acc[p2 + e][0][i] = acc[p2 + e][1][i] = 0.0;
+        }
+      }
     }
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int p = w.mp + p2 + e;
+      if (p2 + e >= S || p < pg0 || p >= pg0 + npg) continue;
+      unsigned long long* base =
+          reinterpret_cast<unsigned long long*>(grids + (size_t)(p - pg0) * plane + col) + (lane & 3);
+      for (int i = 0; i < leave; i++) {
+        const unsigned long long v = buf[(e * 8 + i) * 32 + lane];
+        int row = w.su0 + i;
+        if (row >= g.nu) row -= g.nu;
+        if (v) atomicAdd(base + (size_t)row * g.nv * 4, v);
+      }
+    }
+    __syncwarp();
   }
 }
 
 // Gridding of sorted records [kbase, kend) in double precision (the
 // reference's grid_task_body, wgridder.rs:2102-2156, on windows): each warp
-// takes F64_CHUNK consecutive sorted visibilities, stages F64_BATCH at a time
+// takes `chunk` consecutive sorted visibilities, stages F64_BATCH at a time
 // (coordinates, taps and value from uvw and the data, as k_grid does) and
 // contracts each run of one bin four records at a time.
 template <int S>
-__global__ void __launch_bounds__(F64_BATCH, 12)
+__global__ void __launch_bounds__(F64_BATCH, F64_BLOCKS)
     k_grid_f64(const __grid_constant__ Geom<double> g, Inputs in, int mode, const double* __restrict__ uvw,
                const double* __restrict__ foc, const uint32_t* __restrict__ key, const uint32_t* __restrict__ sorted,
-               uint64_t kbase, uint64_t kend, uint32_t nbins, FixCell2* __restrict__ grids, int pg0, int npg,
+               uint64_t kbase, uint64_t kend, uint32_t chunk, uint32_t nbins, FixCell2* __restrict__ grids, int pg0, int npg,
                FixScale* __restrict__ fs) {
   static_assert(S >= 1 && S <= 8, "8 x 8 windows");
   extern __shared__ __align__(16) unsigned char smem[];
+  unsigned long long* flush_buf = reinterpret_cast<unsigned long long*>(smem);
   F64Slots st;
-  st.carve(smem);
+  st.carve(smem + F64_FLUSH_BYTES);
   const int lane = threadIdx.x, gq = lane >> 2, tq = lane & 3;
-  if (lane < F64_ROW) {
+  if (lane < 8) {
     st.ku[F64_BATCH * F64_ROW + lane] = 0.0;
     st.bre[F64_BATCH * F64_ROW + lane] = 0.0;
     st.bim[F64_BATCH * F64_ROW + lane] = 0.0;
-    st.kw[F64_BATCH * F64_ROW + lane] = 0.0;
+    st.kw[F64_BATCH * F64_KW + lane] = 0.0;
   }
   if (lane == 0) st.key[F64_BATCH] = INACTIVE;
-  const uint64_t k0 = kbase + (uint64_t)blockIdx.x * F64_CHUNK;
-  const uint64_t k1 = min(kend, k0 + F64_CHUNK);
+  const uint64_t k0 = kbase + (uint64_t)blockIdx.x * chunk;
+  const uint64_t k1 = min(kend, k0 + chunk);
   const double sc = FixTraits<double>::scale(fs->q);
   const uint32_t nchan = (uint32_t)g.nchan;
   const uint32_t tmask = (1u << g.log2tile) - 1u;
@@ -173,12 +202,11 @@ __global__ void __launch_bounds__(F64_BATCH, 12)
   for (int p = 0; p < S; p++)
 #pragma unroll
     for (int c = 0; c < 2; c++) acc[p][c][0] = acc[p][c][1] = 0.0;
-  uint32_t gcur = INACTIVE;
-  int rb = 0, su0 = 0, sv0 = 0, mpc = 0;
+  Window win;
 
   // This round's inputs are in pre (copied asynchronously); nidx is the next
   // round's index.
-  Prefetched64* pre = reinterpret_cast<Prefetched64*>(smem + F64Slots::bytes()) + lane;
+  Prefetched64* pre = reinterpret_cast<Prefetched64*>(smem + F64_FLUSH_BYTES + F64Slots::bytes()) + lane;
   const bool with_vis = mode == VALUE_DATA && in.vis_kind != VIS_UNIT;
   if (k0 + lane < k1) prefetch64(pre, uvw, foc, in, with_vis, with_wgt, key, sorted[k0 + lane], nchan);
   cp_async_commit();
@@ -199,7 +227,7 @@ __global__ void __launch_bounds__(F64_BATCH, 12)
       getpix(g, u, v, uf, vf, iu0, iv0);
       const int mp = minplane(g, w);
       const uint32_t su = (uint32_t)shifted(iu0, g.nu) & tmask, sv = (uint32_t)shifted(iv0, g.nv) & tmask;
-      const int du = (int)(su % (uint32_t)g.sube), dv = (int)(sv % (uint32_t)g.sube);
+      const int ur = (int)(su & 7u), dv = (int)(sv % (uint32_t)g.sube);
       double ku[S], kv[S];
       eval_taps2<double, S>(g.coeff, g.ne, -uf * 2.0 + ((double)S - 1.0), -vf * 2.0 + ((double)S - 1.0), ku, kv);
       cplx<double> val = unit_value<double>(g, b, imflip, f, with_wgt, prefetched_wgt64(pr, in));
@@ -208,29 +236,32 @@ __global__ void __launch_bounds__(F64_BATCH, 12)
       double* cu = st.ku + lane * F64_ROW;
       double* cr = st.bre + lane * F64_ROW;
       double* ci = st.bim + lane * F64_ROW;
-      double* cw = st.kw + lane * F64_ROW;
+      double* cw = st.kw + lane * F64_KW;
+      // The u taps at rows (su + i) mod 8, zero elsewhere.
 #pragma unroll
-      for (int j = 0; j < F64_ROW; j++) {
-        double a = 0.0, br = 0.0, bi = 0.0;
+      for (int j = 0; j < 8; j++) cu[(ur + j) & 7] = j < S ? ku[j < S ? j : 0] : 0.0;
+      double kwt[S];
+      if (g.do_wgridding) {  // the w taps from the first plane's argument (w_factor)
+        const double z = g.xdw * ((g.wmin + (double)mp * g.dw) - w);
+        eval_taps1<S>(g.coeff, z * 2.0 + ((double)S - 1.0), kwt);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        double br = 0.0, bi = 0.0;
 #pragma unroll
         for (int d = 0; d < 9 - S; d++) {
-          if (j - d >= 0 && j - d < S) {
+          if (j - d >= 0 && j - d < S && dv == d) {
             const int t = (j - d >= 0 && j - d < S) ? j - d : 0;
-            if (du == d) a = ku[t];
-            if (dv == d) {
-              br = val.re * kv[t];
-              bi = val.im * kv[t];
-            }
+            br = val.re * kv[t];
+            bi = val.im * kv[t];
           }
         }
-        cu[j] = a;
         cr[j] = br;
         ci[j] = bi;
         double kwj = 0.0;
         if (j < S) {
           if (g.do_wgridding) {
-            const int p = mp + j;
-            if (p >= pg0 && p < pg0 + npg) kwj = w_factor<double, S>(g, j, p, w);
+            if (mp + j >= pg0 && mp + j < pg0 + npg) kwj = kwt[j < S ? j : 0];
           } else if (j == 0 && pg0 == 0) {
             kwj = 1.0;
           }
@@ -247,14 +278,11 @@ __global__ void __launch_bounds__(F64_BATCH, 12)
     int q = 0;
     while (q < nb) {
       const uint32_t gk = st.key[q];
-      if (gk != gcur) {
-        if (gcur != INACTIVE) f64_flush<S>(g, grids, pg0, npg, su0, sv0, mpc, sc, acc);
-#pragma unroll
-        for (int p = 0; p < S; p++)
-#pragma unroll
-          for (int c = 0; c < 2; c++) acc[p][c][0] = acc[p][c][1] = 0.0;
-        gcur = gk;
-        window_of(g, gk, nbins, rb, su0, sv0, mpc);
+      if (gk != win.key) {
+        Window next;
+        const int leave = window_step(g, win, gk, nbins, next);
+        if (win.key != INACTIVE) f64_flush<S>(g, grids, pg0, npg, win, leave, sc, acc, flush_buf);
+        win = next;
       }
       const unsigned m = __ballot_sync(0xffffffffu, lane >= q && lane < nb && st.key[lane] == gk);
       const int len = __popc(m);
@@ -264,17 +292,24 @@ __global__ void __launch_bounds__(F64_BATCH, 12)
         const double kur = st.ku[slot * F64_ROW + gq];   // A: row gq, k tq
         const double bre = st.bre[slot * F64_ROW + gq];  // B: k tq, column gq
         const double bim = st.bim[slot * F64_ROW + gq];
+        const double2* kw2 = reinterpret_cast<const double2*>(st.kw + slot * F64_KW);
 #pragma unroll
-        for (int p = 0; p < S; p++) {
-          const double a = kur * st.kw[slot * F64_ROW + p];
-          dmma(acc[p][0], a, bre);
-          dmma(acc[p][1], a, bim);
+        for (int p = 0; p < S; p += 2) {
+          const double2 kw = kw2[p / 2];
+          const double a0 = kur * kw.x;
+          dmma(acc[p][0], a0, bre);
+          dmma(acc[p][1], a0, bim);
+          if (p + 1 < S) {
+            const double a1 = kur * kw.y;
+            dmma(acc[p + 1 < S ? p + 1 : 0][0], a1, bre);
+            dmma(acc[p + 1 < S ? p + 1 : 0][1], a1, bim);
+          }
         }
       }
       q += len;
     }
   }
-  if (gcur != INACTIVE) f64_flush<S>(g, grids, pg0, npg, su0, sv0, mpc, sc, acc);
+  if (win.key != INACTIVE) f64_flush<S>(g, grids, pg0, npg, win, 8, sc, acc, flush_buf);
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&fs->nonfinite, 1);
 }
 

@@ -373,12 +373,12 @@ __global__ void __launch_bounds__(256, COUNT_BLOCKS)
 
 // The taps of one axis at x (the reference's eval_taps, one of the two axes
 // of eval_taps2).
-template <int S>
-__device__ __forceinline__ void eval_taps1(const float* __restrict__ c, float x, float* r) {
+template <int S, class T>
+__device__ __forceinline__ void eval_taps1(const T* __restrict__ c, T x, T* r) {
   constexpr int ne = coeff_rows(S);
   constexpr int H = (S + 1) / 2;
-  const float x2 = x * x;
-  float e[H], o[H];
+  const T x2 = x * x;
+  T e[H], o[H];
 #pragma unroll
   for (int i = 0; i < H; i++) {
     e[i] = c[i];
@@ -388,13 +388,13 @@ __device__ __forceinline__ void eval_taps1(const float* __restrict__ c, float x,
   for (int k = 1; k < ne; k++)
 #pragma unroll
     for (int i = 0; i < H; i++) {
-      e[i] = fmaf(e[i], x2, c[k * S + i]);
-      o[i] = fmaf(o[i], x2, c[(ne + k) * S + i]);
+      e[i] = fma_t(e[i], x2, c[k * S + i]);
+      o[i] = fma_t(o[i], x2, c[(ne + k) * S + i]);
     }
 #pragma unroll
-  for (int i = 0; i < H; i++) r[i] = fmaf(o[i], x, e[i]);
+  for (int i = 0; i < H; i++) r[i] = fma_t(o[i], x, e[i]);
 #pragma unroll
-  for (int i = 0; i < S - H; i++) r[S - 1 - i] = fmaf(o[i], -x, e[i]);
+  for (int i = 0; i < S - H; i++) r[S - 1 - i] = fma_t(o[i], -x, e[i]);
 }
 
 // The stored value of a record's visibility (unit_value, data_value,

@@ -2009,11 +2009,13 @@ void launch_grid_f64(cudaStream_t s, const Geom<double>& g, const Inputs& in, in
                      const double* foc, const uint32_t* key, const uint32_t* sorted, uint64_t kbase, uint64_t kend,
                      uint32_t nbins, fast::FixCell2* grids, int pg0, int npg, fast::FixScale* fs) {
   if (kend <= kbase) return;
-  const int smem = (int)(fast::F64Slots::bytes() + fast::F64_BATCH * sizeof(fast::Prefetched64));
-  const unsigned nblocks = (unsigned)((kend - kbase + fast::F64_CHUNK - 1) / fast::F64_CHUNK);
+  const int smem =
+      (int)(fast::F64_FLUSH_BYTES + fast::F64Slots::bytes() + fast::F64_BATCH * sizeof(fast::Prefetched64));
+  const uint32_t chunk = warp_chunk(kend - kbase, fast::F64_BLOCKS);
+  const unsigned nblocks = (unsigned)((kend - kbase + chunk - 1) / chunk);
   {
     StageTimer timer_(ST_GRID, s);
-    fast::k_grid_f64<S><<<nblocks, fast::F64_BATCH, smem, s>>>(g, in, mode, uvw, foc, key, sorted, kbase, kend, nbins,
+    fast::k_grid_f64<S><<<nblocks, fast::F64_BATCH, smem, s>>>(g, in, mode, uvw, foc, key, sorted, kbase, kend, chunk, nbins,
                                                                grids, pg0, npg, fs);
   }
   check_cuda(cudaGetLastError(), "grid kernel (FP64 tensor cores)");
