@@ -41,7 +41,7 @@ template <class T>
 struct Geom {
   uint64_t nrow, nchan;
   int32_t nx, ny, nu, nv;
-  int32_t supp, nplanes, nbuckets;  // nbuckets = max(nplanes, 1)
+  int32_t supp, nplanes, nbuckets;  // nbuckets: first planes (make_geom)
   int32_t log2tile, ntu, ntv, L;    // L = tile + supp - 1
   // Sub-tiles of a tile, sube cells square: nsub_side along each side, nsub
   // in all (the sub-tile a along u, b along v of a tile is b * nsub_side + a:

@@ -569,23 +569,113 @@ __global__ void k_scan_add(uint32_t* __restrict__ out, uint64_t n, const uint32_
   if (i < n) out[i] += offs[i / SCAN_TILE];
 }
 
-// out[i] = sum of in[0..i) for i < n (in and out may alias).
-void exclusive_scan(const uint32_t* in, uint32_t* out, uint64_t n, cudaStream_t s) {
-  uint64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-  DevBuf sums(ntiles * 4, s);
-  {
-    StageTimer timer_(ST_PREFIX, s);
-    k_scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, s>>>(in, out, n, sums.as<uint32_t>());
+// The sums of PREFIX_TILE consecutive elements each; `vec`: 16-byte loads.
+constexpr int PREFIX_THREADS = 256, PREFIX_QUADS = 8;
+constexpr uint32_t PREFIX_TILE = PREFIX_THREADS * PREFIX_QUADS * 4;
+__device__ __forceinline__ uint4 prefix_load(const uint32_t* __restrict__ in, uint64_t i, uint64_t n, int vec) {
+  if (vec && i + 4 <= n) return *reinterpret_cast<const uint4*>(in + i);
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (i < n) v.x = in[i];
+  if (i + 1 < n) v.y = in[i + 1];
+  if (i + 2 < n) v.z = in[i + 2];
+  if (i + 3 < n) v.w = in[i + 3];
+  return v;
+}
+__device__ __forceinline__ void prefix_store(uint32_t* __restrict__ out, uint64_t i, uint64_t n, int vec, uint4 v) {
+  if (vec && i + 4 <= n) {
+    *reinterpret_cast<uint4*>(out + i) = v;
+    return;
   }
-  check_cuda(cudaGetLastError(), "scan");
-  if (ntiles > 1) {
-    exclusive_scan(sums.as<uint32_t>(), sums.as<uint32_t>(), ntiles, s);
-    {
-      StageTimer timer_(ST_PREFIX, s);
-      k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, n, sums.as<uint32_t>());
+  if (i < n) out[i] = v.x;
+  if (i + 1 < n) out[i + 1] = v.y;
+  if (i + 2 < n) out[i + 2] = v.z;
+  if (i + 3 < n) out[i + 3] = v.w;
+}
+__device__ __forceinline__ uint32_t block_sum_u32(uint32_t v) {  // the block's sum, in every thread
+  __shared__ uint32_t part[PREFIX_THREADS / 32];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  uint32_t s = 0;
+  for (int w = 0; w < PREFIX_THREADS / 32; w++) s += part[w];
+  __syncthreads();
+  return s;
+}
+__global__ void __launch_bounds__(PREFIX_THREADS) k_prefix_sums(const uint32_t* __restrict__ in, uint64_t n, int vec,
+                                                                uint32_t* __restrict__ sums) {
+  const uint64_t base = (uint64_t)blockIdx.x * PREFIX_TILE + threadIdx.x * 4;
+  uint32_t s = 0;
+#pragma unroll
+  for (int q = 0; q < PREFIX_QUADS; q++) {
+    const uint4 v = prefix_load(in, base + (uint64_t)q * PREFIX_THREADS * 4, n, vec);
+    s += v.x + v.y + v.z + v.w;
+  }
+  s = block_sum_u32(s);
+  if (threadIdx.x == 0) sums[blockIdx.x] = s;
+}
+// The exclusive scan of each tile from its offset, to `out` and (if given)
+// `out2`. `scanned`: sums holds the tiles' offsets; otherwise their sums, and
+// each block adds up those before its own.
+__global__ void __launch_bounds__(PREFIX_THREADS)
+    k_prefix_apply(const uint32_t* in, uint32_t* out, uint32_t* __restrict__ out2, uint64_t n, int vec,
+                   const uint32_t* __restrict__ sums, int scanned) {
+  __shared__ uint32_t warp_tot[PREFIX_THREADS / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t run = 0;
+  if (scanned) {
+    run = sums[blockIdx.x];
+  } else if (blockIdx.x) {
+    uint32_t s = 0;
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += PREFIX_THREADS) s += sums[i];
+    run = block_sum_u32(s);
+  }
+  const uint64_t base = (uint64_t)blockIdx.x * PREFIX_TILE + threadIdx.x * 4;
+  uint4 v[PREFIX_QUADS];
+#pragma unroll
+  for (int q = 0; q < PREFIX_QUADS; q++) v[q] = prefix_load(in, base + (uint64_t)q * PREFIX_THREADS * 4, n, vec);
+#pragma unroll
+  for (int q = 0; q < PREFIX_QUADS; q++) {  // 1024 consecutive elements, four a thread
+    const uint32_t mine = v[q].x + v[q].y + v[q].z + v[q].w;
+    uint32_t x = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
-    check_cuda(cudaGetLastError(), "scan");
+    if (lane == 31) warp_tot[wid] = x;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (int w = 0; w < PREFIX_THREADS / 32; w++) {
+      before += w < wid ? warp_tot[w] : 0u;
+      total += warp_tot[w];
+    }
+    __syncthreads();
+    const uint32_t e = run + before + x - mine;
+    const uint4 r = make_uint4(e, e + v[q].x, e + v[q].x + v[q].y, e + v[q].x + v[q].y + v[q].z);
+    const uint64_t i = base + (uint64_t)q * PREFIX_THREADS * 4;
+    prefix_store(out, i, n, vec, r);
+    if (out2) prefix_store(out2, i, n, vec, r);
+    run += total;
   }
+}
+
+// out[i] = sum of in[0..i) for i < n (in and out may alias), and the same in
+// out2 if given: the tiles' sums, then each tile again with its offset. The
+// elements are read twice and written once; the bin counts (4 bytes for every
+// bin, most of them empty) make this a pass over memory.
+void exclusive_scan(const uint32_t* in, uint32_t* out, uint64_t n, cudaStream_t s, uint32_t* out2 = nullptr) {
+  if (n == 0) return;
+  const uint64_t ntiles = (n + PREFIX_TILE - 1) / PREFIX_TILE;
+  const int vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) |
+                    reinterpret_cast<uintptr_t>(out2)) % 16) == 0;
+  DevBuf sums(ntiles * 4, s);
+  // Up to 2048 tiles each block adds up the sums before its own (8 KB from L2).
+  const bool two_level = ntiles > 2048;
+  StageTimer timer_(ST_PREFIX, s);
+  if (ntiles > 1) k_prefix_sums<<<(unsigned)ntiles, PREFIX_THREADS, 0, s>>>(in, n, vec, sums.as<uint32_t>());
+  if (two_level) exclusive_scan(sums.as<uint32_t>(), sums.as<uint32_t>(), ntiles, s);
+  k_prefix_apply<<<(unsigned)ntiles, PREFIX_THREADS, 0, s>>>(in, out, out2, n, vec, sums.as<uint32_t>(),
+                                                             two_level ? 1 : 0);
+  check_cuda(cudaGetLastError(), "scan");
 }
 
 // a[i] += base[c] for i < n, and base[c + 1] = the new a[n - 1]: one row
@@ -2428,7 +2518,9 @@ template <class T>
 void Plan<T>::build_layout(const Inputs& act, bool with_vis, const uint32_t* bits, cudaStream_t s) {
   ntiles_ = (size_t)g_.ntu * g_.ntv;
   nbins_ = ntiles_ * (size_t)g_.nbuckets * (size_t)g_.nsub;
-  if (nbins_ >= 0xffffffffull) throw InvalidArgument("too many uv tiles and w-planes for one call");
+  // The limit counts every plane as a first plane, as the keys of the binning's export do.
+  if (ntiles_ * (size_t)std::max(g_.nplanes, 1) * (size_t)g_.nsub >= 0xffffffffull)
+    throw InvalidArgument("too many uv tiles and w-planes for one call");
   if ((size_t)nchunk_ * nbins_ >= 0xffffffffull) {
     // Row chunks are an optimisation: as many as the 32-bit key space holds
     // (chunks x bins keys, below the inactive key), down to one.
@@ -2455,7 +2547,8 @@ void Plan<T>::build_layout(const Inputs& act, bool with_vis, const uint32_t* bit
                                                         bits);
   }
   check_cuda(cudaGetLastError(), "bin count");
-  exclusive_scan(starts_.as<uint32_t>(), starts_.as<uint32_t>(), nkeys + 1, s);
+  DevBuf cursor(sizeof(T) == 4 ? (nkeys + 1) * 4 : 0, s);  // the counting sort's
+  exclusive_scan(starts_.as<uint32_t>(), starts_.as<uint32_t>(), nkeys + 1, s, cursor.as<uint32_t>());
   if constexpr (sizeof(T) == 8) {
     // A stable radix sort of the visibility indices by bin key: inside a bin
     // the visibilities keep their index order (the reference's layout
@@ -2507,8 +2600,6 @@ void Plan<T>::build_layout(const Inputs& act, bool with_vis, const uint32_t* bit
       check_cuda(cudaMemcpyAsync(sorted_.get(), vals_out.get(), nvis_ * 4, cudaMemcpyDeviceToDevice, s), "copy");
     }
   } else {
-    DevBuf cursor((nkeys + 1) * 4, s);
-    check_cuda(cudaMemcpyAsync(cursor.get(), starts_.get(), (nkeys + 1) * 4, cudaMemcpyDeviceToDevice, s), "copy");
     sorted_.alloc(nvis_ * 4, s);
     {
       StageTimer timer_(ST_BIN_SCATTER, s);
@@ -3254,14 +3345,18 @@ void Plan<T>::export_binning(uint32_t* key_host, uint32_t* sorted_host, cudaStre
   if (nchunk_ != 1) throw DeviceError("binning export of a plan with row chunks");
   check_cuda(cudaMemcpyAsync(key_host, key_.get(), n_ * 4, cudaMemcpyDeviceToHost, s), "copy");
   check_cuda(cudaStreamSynchronize(s), "copy");
-  // The reference's key, tile * nbuckets + plane, without the sub-tile.
+  // The reference's key, tile * max(nplanes, 1) + plane, without the sub-tile.
+  const uint32_t nplanes = (uint32_t)std::max(g_.nplanes, 1);
   for (size_t i = 0; i < n_; i++)
-    if (key_host[i] != INACTIVE) key_host[i] /= (uint32_t)g_.nsub;
+    if (key_host[i] != INACTIVE) {
+      const uint32_t k = key_host[i] / (uint32_t)g_.nsub;
+      key_host[i] = k / (uint32_t)g_.nbuckets * nplanes + k % (uint32_t)g_.nbuckets;
+    }
   // The reference's layout order (tile, first plane, row, channel): the
   // device's keys ordered by a stable counting sort. The device's own sorted
   // order leaves the order inside a bin free; gridding sums exact terms, so
   // the results do not depend on it.
-  const size_t nref = (size_t)g_.ntu * g_.ntv * (size_t)g_.nbuckets;
+  const size_t nref = (size_t)g_.ntu * g_.ntv * (size_t)nplanes;
   std::vector<uint32_t> start(nref + 1, 0);
   for (size_t i = 0; i < n_; i++)
     if (key_host[i] != INACTIVE) start[key_host[i] + 1]++;
@@ -3393,6 +3488,7 @@ void bin_noalloc(const WgridderOptions& o, size_t nrow, size_t nchan, const doub
   g.sube = 1 << g.log2tile;
   g.nsub_side = 1;
   g.nsub = 1;
+  g.nbuckets = std::max(g.nplanes, 1);
   const uint64_t nbins = (uint64_t)g.ntu * g.ntv * g.nbuckets * g.nsub;
   const uint64_t need_words = 2 * (nbins + 1) + scan_tmp_words(nbins + 1);
   const uint64_t have_words = (NOALLOC_SCRATCH_BYTES - words_off) / sizeof(uint32_t);

@@ -324,7 +324,10 @@ void make_geom(const WgridderOptions& o, size_t nrow, size_t nchan, size_t nvis,
   g.nv = (int32_t)nv;
   g.supp = (int32_t)supp;
   g.nplanes = (int32_t)nplanes;
-  g.nbuckets = (int32_t)std::max<size_t>(nplanes, 1);
+  // First planes: (w + wshift) / dw runs over [0, nplanes - supp + 1) from the
+  // smallest to the largest |w| (plane_count), one more for its rounding.
+  // Bins for the planes that no footprint starts on would only be scanned.
+  g.nbuckets = nplanes ? (int32_t)std::min(nplanes, nplanes + 2 - std::min(supp, nplanes + 1)) : 1;
   g.log2tile = single ? 5 : 4;  // ducc0's tile sizes: 32 cells in f32, 16 in f64
   int tile = 1 << g.log2tile;
   g.ntu = (int32_t)((nu + tile - 1) / tile);

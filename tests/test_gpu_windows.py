@@ -56,3 +56,17 @@ def test_windows_match_the_oracle(single, supp, n):
     got = gridder.dirty2vis(dirty=img, **kw)
     ref = oracle.dirty2vis(dirty=img, **kw)
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+
+
+def test_bin_offsets_past_one_level_of_tile_sums():
+    """Supports of 8 on a 4096^2 grid: 33 M bins, whose offsets are scanned in
+    two levels."""
+    n, nx, nu, cell = 5000, 64, 4096, 2e-4
+    uvw = _uv(n, nu, nu, cell, 5)
+    rng = np.random.default_rng(6)
+    vis = (rng.standard_normal((n, 1)) + 1j * rng.standard_normal((n, 1))).astype(np.complex64)
+    kw = dict(uvw=uvw, freq=np.array([1e9]), pixsize_x=cell, pixsize_y=cell, epsilon=1e-3,
+              kernel=(_kernel(8, True), nu, nu))
+    got = gridder.vis2dirty(vis=vis, npix_x=nx, npix_y=nx, **kw)
+    ref = oracle.vis2dirty(vis=vis, npix_x=nx, npix_y=nx, **kw)
+    assert np.abs(got - ref).max() <= 2e-5 * np.abs(ref).max()
