@@ -16,8 +16,8 @@ struct TcConvArgs {
   int H, W, ld_in, ld_out, ld_mask, Cin, Cout, relu, accumulate;
 };
 
-// Whether the shapes and alignments fit the kernel: W a multiple of 16, H of
-// 8, channels of 32, pixel strides of 8, 16-byte aligned tensors.
+// Whether the shapes and alignments fit the kernel: channels multiples of 32,
+// pixel strides of 8, 16-byte aligned tensors (any height and width).
 bool conv3_tc_supported(const TcConvArgs& a);
 // Launches on s; 0, 1 (the tensor maps were refused) or 2 (launch error).
 int conv3_tc(const TcConvArgs& a, cudaStream_t s);
@@ -36,9 +36,9 @@ struct TcDwArgs {
   int H, W, ld_in, ld_dz, Cin, Cout;
 };
 
-// Whether the weight gradient's shapes fit the tcgen05 kernel: W a multiple
-// of 16, H of 8, input channels of 32, output channels of 64, pixel strides
-// of 8, 16-byte aligned tensors.
+// Whether the weight gradient's shapes fit the tcgen05 kernel: channels
+// multiples of 32, pixel strides of 8, 16-byte aligned tensors (any height and
+// width).
 bool conv3_dw_tc_supported(const TcDwArgs& a);
 // dw += the weight gradient on s; 0, 1 (the tensor maps were refused) or 2.
 int conv3_dw_tc(const TcDwArgs& a, cudaStream_t s);

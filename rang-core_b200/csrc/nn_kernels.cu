@@ -338,34 +338,46 @@ __global__ void __launch_bounds__(128) k_conv3_dw(const DwArgs a) {
   }
 }
 
-// dbias[c] += sum_p dz[p, c]: threads take channel pairs, blocks take pixel ranges.
-__global__ void k_bias_grad(const bf16* __restrict__ dz, int ld, int64_t P, int C, float* __restrict__ db,
-                            int64_t rows_per_block) {
-  __shared__ float red[256][2];
-  const int pairs = C / 2, lanes = 256 / pairs;
-  const int t = threadIdx.x, c2 = t % pairs, r = t / pairs;
-  float s0 = 0.0f, s1 = 0.0f;
+// dbias[c] += sum_p dz[p, c]: threads take eight channels (a 16-byte load) of
+// every `lanes`-th pixel, blocks take pixel ranges.
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16* __restrict__ dz, int ld, int64_t P, int C,
+                                                   float* __restrict__ db, int64_t rows_per_block) {
+  __shared__ float red[256][9];
+  const int c8 = C / 8, lanes = 256 / c8;
+  const int t = threadIdx.x, c = t % c8, r = t / c8;
+  float s[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) s[i] = 0.0f;
   if (r < lanes) {
     const int64_t p0 = (int64_t)blockIdx.x * rows_per_block;
     int64_t p1 = p0 + rows_per_block;
     if (p1 > P) p1 = P;
+#pragma unroll 4
     for (int64_t p = p0 + r; p < p1; p += lanes) {
-      const float2 v = __bfloat1622float2(*reinterpret_cast<const bf162*>(dz + p * ld + 2 * c2));
-      s0 += v.x;
-      s1 += v.y;
+      const uint4 u = *reinterpret_cast<const uint4*>(dz + p * ld + 8 * c);
+      const bf162* h = reinterpret_cast<const bf162*>(&u);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const float2 v = __bfloat1622float2(h[i]);
+        s[2 * i] += v.x;
+        s[2 * i + 1] += v.y;
+      }
     }
   }
-  red[t][0] = s0;
-  red[t][1] = s1;
+#pragma unroll
+  for (int i = 0; i < 8; i++) red[t][i] = s[i];
   __syncthreads();
-  if (r == 0) {
-    for (int k = 1; k < lanes; k++) {
-      s0 += red[k * pairs + c2][0];
-      s1 += red[k * pairs + c2][1];
-    }
-    atomicAdd(&db[2 * c2], s0);
-    atomicAdd(&db[2 * c2 + 1], s1);
+  for (int i = t; i < C; i += 256) {
+    float sum = 0.0f;
+    for (int k = 0; k < lanes; k++) sum += red[k * c8 + i / 8][i % 8];
+    atomicAdd(&db[i], sum);
   }
+}
+
+// 63 us a layer at 67 MB with 4096 pixels a block and 4-byte loads.
+void launch_bias_grad(const bf16* dz, int ld, int64_t P, int C, float* db, cudaStream_t s) {
+  const int64_t rows = (P + 4 * kSMs - 1) / (4 * kSMs) > 64 ? (P + 4 * kSMs - 1) / (4 * kSMs) : 64;
+  k_bias_grad<<<(unsigned)((P + rows - 1) / rows), 256, 0, s>>>(dz, ld, P, C, db, rows);
 }
 
 // wt[ci][tap][co] = w[co][8 - tap][ci]: the weights of the input-gradient convolution.
@@ -669,12 +681,8 @@ int32_t rang_b200_nn_conv3_weight_grad(const void* in, int64_t ld_in, const void
     if (conv3_dw_tc_supported(t)) {
       const int st = conv3_dw_tc(t, (cudaStream_t)stream);
       if (st != 0) return st;
-      if (dbias) {
-        const int64_t rows = 4096, P = batch * height * width;
-        k_bias_grad<<<(unsigned)((P + rows - 1) / rows), 256, 0, (cudaStream_t)stream>>>((const bf16*)dz,
-                                                                                        (int)ld_dz, P, cout, dbias,
-                                                                                        rows);
-      }
+      if (dbias)
+        launch_bias_grad((const bf16*)dz, (int)ld_dz, batch * height * width, cout, dbias, (cudaStream_t)stream);
       return launched();
     }
   }
@@ -696,11 +704,7 @@ int32_t rang_b200_nn_conv3_weight_grad(const void* in, int64_t ld_in, const void
     k_conv3_dw<64><<<grid, 128, dw_smem_bytes<64>(), (cudaStream_t)stream>>>(a);
   else
     k_conv3_dw<32><<<grid, 128, dw_smem_bytes<32>(), (cudaStream_t)stream>>>(a);
-  if (dbias) {
-    const int64_t rows = 4096;
-    k_bias_grad<<<(unsigned)((a.P + rows - 1) / rows), 256, 0, (cudaStream_t)stream>>>((const bf16*)dz, (int)ld_dz,
-                                                                                       a.P, cout, dbias, rows);
-  }
+  if (dbias) launch_bias_grad((const bf16*)dz, (int)ld_dz, a.P, cout, dbias, (cudaStream_t)stream);
   return launched();
 }
 
