@@ -196,8 +196,10 @@ void rang_b200_wgridder_plan_release_work(RangWgridPlan* plan);
  * stream-ordered pool keeps) is not available to other allocators in the
  * process, such as PyTorch's. rang_b200_wgridder_cached_bytes reports the
  * bytes held on the current device; rang_b200_wgridder_release_cached
- * returns them, and the pool's unused memory, to the device (status 0, 2 on
- * a CUDA error), after the work already queued that uses them. */
+ * returns them, and the pool's unused memory, to the device, and the pinned
+ * host buffers that copies of pageable arrays go through (32 MB at most) to
+ * the host (status 0, 2 on a CUDA error), after the work already queued that
+ * uses them. */
 size_t rang_b200_wgridder_cached_bytes(void);
 int32_t rang_b200_wgridder_release_cached(void);
 /* `plan` and `gridding_footprint` (wgridder.rs:3527-3588) on HOST arrays:

@@ -16,6 +16,7 @@
 #include <string>
 
 #include "rang_weights.h"
+#include "host_copy.h"
 #include "wgrid_plan.h"
 
 // The imaging-weight pipeline (wgrid_weights.cu).
@@ -151,7 +152,7 @@ DevBuf upload(const void* host, size_t bytes, cudaStream_t s) {
   DevBuf b;
   if (host && bytes) {
     b.alloc(bytes, s);
-    check_cuda(cudaMemcpyAsync(b.get(), host, bytes, cudaMemcpyHostToDevice, s), "copy to device");
+    copy_to_device(b.get(), host, bytes, s);
   }
   return b;
 }
@@ -209,9 +210,8 @@ void host_vis2dirty_pipelined(const WgridderOptions* o, size_t nrow, size_t ncha
   DevBuf visd(nrow * rowb, sc);
   for (int c = 0; c < nchunk; c++) {
     const size_t r0 = (size_t)c * rpc, r1 = std::min(nrow, r0 + rpc);
-    check_cuda(cudaMemcpyAsync(visd.as<unsigned char>() + r0 * rowb, static_cast<const unsigned char*>(vis) + r0 * rowb,
-                               (r1 - r0) * rowb, cudaMemcpyHostToDevice, sc),
-               "copy to device");
+    copy_to_device(visd.as<unsigned char>() + r0 * rowb, static_cast<const unsigned char*>(vis) + r0 * rowb,
+                   (r1 - r0) * rowb, sc);
     check_cuda(cudaEventRecord(ready.e[c], sc), "record");
   }
   Plan<T> plan(*o, nrow, nchan, u.uvw.as<double>(), freq, u.in, false, s, chunks);
@@ -233,7 +233,7 @@ void host_vis2dirty_pipelined(const WgridderOptions* o, size_t nrow, size_t ncha
   }
   if (plan.same_scan(data, true, s)) {
     std::memcpy(info, plan.info().v, sizeof(plan.info().v));
-    check_cuda(cudaMemcpyAsync(dirty, img.get(), npix * sizeof(T), cudaMemcpyDeviceToHost, s), "copy to host");
+    copy_to_host(dirty, img.get(), npix * sizeof(T), s);
     finish(plan, s);
     return;
   }
@@ -241,7 +241,7 @@ void host_vis2dirty_pipelined(const WgridderOptions* o, size_t nrow, size_t ncha
   std::memcpy(info, exact.info().v, sizeof(exact.info().v));
   if (exact.empty()) return;
   exact.grid(data, VALUE_DATA, img.as<T>(), s, nullptr, true);
-  check_cuda(cudaMemcpyAsync(dirty, img.get(), npix * sizeof(T), cudaMemcpyDeviceToHost, s), "copy to host");
+  copy_to_host(dirty, img.get(), npix * sizeof(T), s);
   finish(exact, s);
 }
 
@@ -274,11 +274,11 @@ void host_vis2dirty(const WgridderOptions* o, size_t nrow, size_t nchan, const d
   DevBuf img(npix * sizeof(T), s);
   if (dirty) {
     plan.grid(u.in, VALUE_DATA, img.as<T>(), s, nullptr, true);
-    check_cuda(cudaMemcpyAsync(dirty, img.get(), npix * sizeof(T), cudaMemcpyDeviceToHost, s), "copy to host");
+    copy_to_host(dirty, img.get(), npix * sizeof(T), s);
   }
   if (psf) {
     plan.grid(u.in, VALUE_UNIT, img.as<T>(), s, nullptr, true);
-    check_cuda(cudaMemcpyAsync(psf, img.get(), npix * sizeof(T), cudaMemcpyDeviceToHost, s), "copy to host");
+    copy_to_host(psf, img.get(), npix * sizeof(T), s);
   }
   finish(plan, s);
 }
@@ -308,7 +308,7 @@ void host_dirty2vis(const WgridderOptions* o, size_t nrow, size_t nchan, const d
   DevBuf out(n * 2 * sizeof(T), s);
   if (plan.chunks() == 1) {
     plan.degrid(img.as<T>(), u.in, out.as<T>(), s);
-    check_cuda(cudaMemcpyAsync(vis, out.get(), n * 2 * sizeof(T), cudaMemcpyDeviceToHost, s), "copy to host");
+    copy_to_host(vis, out.get(), n * 2 * sizeof(T), s);
     finish(plan, s);
     return;
   }
@@ -320,9 +320,8 @@ void host_dirty2vis(const WgridderOptions* o, size_t nrow, size_t nchan, const d
   for (int c = 0; c < plan.chunks(); c++) {
     const size_t r0 = plan.row_begin(c), r1 = plan.row_begin(c + 1);
     check_cuda(cudaStreamWaitEvent(sc, done.e[c], 0), "wait");
-    check_cuda(cudaMemcpyAsync(reinterpret_cast<unsigned char*>(vis) + r0 * rowb, out.as<unsigned char>() + r0 * rowb,
-                               (r1 - r0) * rowb, cudaMemcpyDeviceToHost, sc),
-               "copy to host");
+    copy_to_host(reinterpret_cast<unsigned char*>(vis) + r0 * rowb, out.as<unsigned char>() + r0 * rowb,
+                 (r1 - r0) * rowb, sc);
   }
   check_cuda(cudaStreamSynchronize(sc), "copy to host");
   finish(plan, s);
@@ -638,6 +637,7 @@ int32_t rang_b200_wgridder_release_cached(void) {
     int dev = 0;
     check_cuda(cudaGetDevice(&dev), "no CUDA device");
     flush_cache(dev);  // frees in stream order and waits for those frees
+    release_host_buffers();
     cudaMemPool_t pool;
     check_cuda(cudaDeviceGetDefaultMemPool(&pool, dev), "memory pool");
     check_cuda(cudaMemPoolTrimTo(pool, 0), "memory pool");

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "rang_weights.h"
+#include "host_copy.h"
 #include "wgrid_plan.h"
 #include "wgrid_setup.h"
 
@@ -214,7 +215,7 @@ DevBuf upload_bytes(const void* host, size_t bytes, cudaStream_t s) {
   DevBuf b;
   if (bytes) {
     b.alloc(bytes, s);
-    check_cuda(cudaMemcpyAsync(b.get(), host, bytes, cudaMemcpyHostToDevice, s), "copy to device");
+    copy_to_device(b.get(), host, bytes, s);
   }
   return b;
 }
@@ -246,8 +247,8 @@ void stokes_i(const StokesIInputs& in, StokesIOutputs& out, cudaStream_t s) {
   k_stokes_i<<<grid_blocks(n), 256, 0, s>>>(n, d.as<float>(), w.as<float>(), f.as<uint8_t>(), v.as<float>(),
                                             o.as<float>());
   check_cuda(cudaGetLastError(), "stokes i");
-  check_cuda(cudaMemcpyAsync(out.vis, v.get(), n * 2 * sizeof(float), cudaMemcpyDeviceToHost, s), "copy to host");
-  check_cuda(cudaMemcpyAsync(out.weight, o.get(), n * sizeof(float), cudaMemcpyDeviceToHost, s), "copy to host");
+  copy_to_host(out.vis, v.get(), n * 2 * sizeof(float), s);
+  copy_to_host(out.weight, o.get(), n * sizeof(float), s);
   check_cuda(cudaStreamSynchronize(s), "stokes i");
 }
 
@@ -281,7 +282,7 @@ void imaging_weights(const ImagingWeightInputs& in, ImagingWeightOutputs& out, c
   // finish (weights.rs:190-227), sequentially on the host.
   std::vector<double> host(ncell);
   double tot = 0.0;
-  if (ncell) check_cuda(cudaMemcpyAsync(host.data(), cells.get(), ncell * sizeof(double), cudaMemcpyDeviceToHost, s), "copy");
+  copy_to_host(host.data(), cells.get(), ncell * sizeof(double), s);
   check_cuda(cudaMemcpyAsync(&tot, total.get(), sizeof(double), cudaMemcpyDeviceToHost, s), "copy");
   check_cuda(cudaStreamSynchronize(s), "weight grid");
   if (in.class_ == 2) {
@@ -299,7 +300,7 @@ void imaging_weights(const ImagingWeightInputs& in, ImagingWeightOutputs& out, c
     for (double& v : host)
       if (v != 0.0) v = 1.0;
   }
-  if (ncell) check_cuda(cudaMemcpyAsync(cells.get(), host.data(), ncell * sizeof(double), cudaMemcpyHostToDevice, s), "copy");
+  copy_to_device(cells.get(), host.data(), ncell * sizeof(double), s);
   if (in.rank_filter_level >= 1.0 && ncell) {
     DevBuf filtered(ncell * sizeof(double), s);
     k_weight_rank<<<grid_blocks(ncell), 256, 0, s>>>(cells.as<double>(), filtered.as<double>(), (int64_t)gw,
@@ -313,10 +314,10 @@ void imaging_weights(const ImagingWeightInputs& in, ImagingWeightOutputs& out, c
     k_weight_lookup<<<grid_blocks(n), 256, 0, s>>>(in.nrow, (uint32_t)in.nchan, uvw.as<double>(), wl.as<double>(),
                                                    sel.as<uint8_t>(), g, cells.as<double>(), img.as<float>());
     check_cuda(cudaGetLastError(), "weight lookup");
-    check_cuda(cudaMemcpyAsync(out.weights, img.get(), n * sizeof(float), cudaMemcpyDeviceToHost, s), "copy to host");
+    copy_to_host(out.weights, img.get(), n * sizeof(float), s);
   }
   if (out.grid && ncell)
-    check_cuda(cudaMemcpyAsync(out.grid, cells.get(), ncell * sizeof(double), cudaMemcpyDeviceToHost, s), "copy to host");
+    copy_to_host(out.grid, cells.get(), ncell * sizeof(double), s);
   if (out.sums) {
     DevBuf ws(sizeof(WeightSumsDev), s);
     check_cuda(cudaMemsetAsync(ws.get(), 0, sizeof(WeightSumsDev), s), "memset");
