@@ -397,6 +397,55 @@ __device__ __forceinline__ void eval_taps1(const T* __restrict__ c, T x, T* r) {
   for (int i = 0; i < S - H; i++) r[S - 1 - i] = fma_t(o[i], -x, e[i]);
 }
 
+// The kernel's polynomials for evaluation two coefficients at a time: even and
+// odd coefficient k of tap i (of the first ceil(S / 2)) side by side, for the
+// packed FP32 multiply-add (fma.rn.f32x2, each half rounded as fmaf rounds):
+// a tap costs half the instructions, and the kernels below are bound by them.
+template <int S>
+struct TapPairs {
+  static constexpr int NE = coeff_rows(S), H = (S + 1) / 2;
+  float2 c[NE * H];
+  explicit TapPairs(const float* coeff) {
+    for (int k = 0; k < NE; k++)
+      for (int i = 0; i < H; i++) c[k * H + i] = make_float2(coeff[k * S + i], coeff[(NE + k) * S + i]);
+  }
+};
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// The taps of one axis at x (eval_taps1 in pairs, the same roundings).
+template <int S>
+__device__ __forceinline__ void eval_taps_pairs(const TapPairs<S>& tp, float x, float* r) {
+  constexpr int ne = TapPairs<S>::NE, H = TapPairs<S>::H;
+  const float x2 = x * x;
+  const unsigned long long xx = pack2(x2, x2);
+  unsigned long long eo[H];
+#pragma unroll
+  for (int i = 0; i < H; i++) eo[i] = pack2(tp.c[i].x, tp.c[i].y);
+#pragma unroll
+  for (int k = 1; k < ne; k++)
+#pragma unroll
+    for (int i = 0; i < H; i++) eo[i] = fma2(eo[i], xx, pack2(tp.c[k * H + i].x, tp.c[k * H + i].y));
+#pragma unroll
+  for (int i = 0; i < H; i++) {
+    const float2 v = unpack2(eo[i]);
+    r[i] = fmaf(v.y, x, v.x);
+    if (i < S - H) r[S - 1 - i] = fmaf(v.y, -x, v.x);
+  }
+}
+
 // The stored value of a record's visibility (unit_value, data_value,
 // wgridder.rs:1414-1435): value = vis * phase * wgt with the imaginary part
 // negated where w was flipped; the phase alone times wgt for unit values.
@@ -584,30 +633,21 @@ constexpr float I8_ASCALE = 4194304.0f;  // 2^22
 // balanced limbs need. The taps of every kernel of the table are positive on
 // [-1, 1] and at most 1 + eps, so x lies far inside [-0x8080, 2^23 - 0x8080).
 constexpr float I8_AOFF = 8421504.0f;  // 2^23 + 0x8080
-// Row strides (words) of the staging rows: with them the reads of the eight
+// One staged record, in words: value * v taps placed on the window's 8 columns
+// (rint(value kv 2^sb) + 0x8080, re and im; the offset elsewhere), the w taps
+// times 2^22 (8, read as pairs of planes), the u taps placed on the window's 8
+// rows (zero elsewhere). With a stride that is 2 mod 8 the reads of the eight
 // records of a lane quad (slots 4 tq + j) fall in distinct banks.
-constexpr int I8_KU = 10;   // u taps placed on the window's 8 rows
-constexpr int I8_B = 9;     // uint2: rint(value * placed v taps * 2^sb) + 0x8080 on the 8 columns
-constexpr int I8_KW = 10;   // w taps * 2^22 (8), as float2 pairs of planes
-
-// Staging of one round: per slot (record) the u taps and value * v taps
-// placed on the window's rows and columns (zero, or the offset, elsewhere),
-// the w taps times 2^22 and the key. Slot N, past the N records, stays zero.
+constexpr int I8_SLOT = 42, I8_KW = 18, I8_KU = 28;  // stride; where the w and u taps start
+// Staging of one round: N records and their bin keys. Slot N stays zero.
 template <int N>
 struct I8Slots {
-  float* ku;      // [N + 1][I8_KU]
-  uint2* bv;      // [N + 1][I8_B]
-  float* kw;      // [N + 1][I8_KW]
-  uint32_t* key;  // [N + 1]
-  __host__ __device__ static constexpr size_t bytes() {
-    return ((size_t)(N + 1) * (I8_B * 8 + I8_KU * 4 + I8_KW * 4 + 4) + 15) / 16 * 16;
-  }
-  // bv and kw are read as float2: both start on 8-byte boundaries.
+  uint32_t* slot;  // [N + 1][I8_SLOT]
+  uint32_t* key;   // [N + 1]
+  __host__ __device__ static constexpr size_t bytes() { return ((size_t)(N + 1) * (I8_SLOT + 1) * 4 + 15) / 16 * 16; }
   __device__ void carve(unsigned char* base) {
-    bv = reinterpret_cast<uint2*>(base);
-    kw = reinterpret_cast<float*>(bv + (N + 1) * I8_B);
-    ku = kw + (N + 1) * I8_KW;
-    key = reinterpret_cast<uint32_t*>(ku + (N + 1) * I8_KU);
+    slot = reinterpret_cast<uint32_t*>(base);
+    key = slot + (N + 1) * I8_SLOT;
   }
 };
 
@@ -688,17 +728,18 @@ __device__ __forceinline__ void i8_flush(const Geom<float>& g, FixCell* __restri
   }
 }
 
-// The limb products of a run's first 16 HF records (slots q .. q + len - 1 of
-// bin run; the zero slot past them) added to the window's fragments.
-template <int NP, int HF, int N>
+// The limb products of a run's first 16 HF records (slots q .. q + len - 1, the
+// zero slot past them; FULL: all 16 HF of them) added to the window's fragments.
+template <int NP, int HF, bool FULL, int N>
 __device__ __forceinline__ void i8_contract(const I8Slots<N>& st, int q, int len, int h0, int (&acc)[NP][2][3][4]) {
   const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
   // This lane's records: k = 4tq + j and 16 + 4tq + j, j < 4.
-  int slot[4 * HF];
+  int rec[4 * HF];  // where their slots start
+  const int first = (q + 4 * tq) * I8_SLOT;
 #pragma unroll
   for (int j = 0; j < 4 * HF; j++) {
-    const int k = (j < 4 ? 4 * tq : 16 + 4 * tq) + (j & 3);
-    slot[j] = k < len ? q + k : N;
+    const int k = j < 4 ? j : 12 + j;  // past 4tq
+    rec[j] = FULL || 4 * tq + k < len ? first + k * I8_SLOT : N * I8_SLOT;
   }
   float kuv[4 * HF];
   uint32_t b[2][3][HF];  // B limbs per component: registers for k 4tq.. and 16 + 4tq..
@@ -707,8 +748,8 @@ __device__ __forceinline__ void i8_contract(const I8Slots<N>& st, int q, int len
     uint2 bvv[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      kuv[4 * hf + j] = st.ku[slot[4 * hf + j] * I8_KU + gq];
-      bvv[j] = st.bv[slot[4 * hf + j] * I8_B + gq];
+      kuv[4 * hf + j] = __uint_as_float(st.slot[rec[4 * hf + j] + I8_KU + gq]);
+      bvv[j] = *reinterpret_cast<const uint2*>(st.slot + rec[4 * hf + j] + 2 * gq);
     }
     limbs4(bvv[0].x, bvv[1].x, bvv[2].x, bvv[3].x, b[0][0][hf], b[0][1][hf], b[0][2][hf]);
     limbs4(bvv[0].y, bvv[1].y, bvv[2].y, bvv[3].y, b[1][0][hf], b[1][1][hf], b[1][2][hf]);
@@ -718,15 +759,12 @@ __device__ __forceinline__ void i8_contract(const I8Slots<N>& st, int q, int len
     uint32_t a[3][2 * HF];  // per limb: rows gq (plane 2h), gq + 8 (plane 2h + 1) x k halves
 #pragma unroll
     for (int hf = 0; hf < HF; hf++) {
-      float2 w[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        w[j] = *reinterpret_cast<const float2*>(st.kw + slot[4 * hf + j] * I8_KW + 2 * (h0 + h));
       uint32_t x[4], y[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        x[j] = __float_as_uint(fmaf(w[j].x, kuv[4 * hf + j], I8_AOFF));
-        y[j] = __float_as_uint(fmaf(w[j].y, kuv[4 * hf + j], I8_AOFF));
+        const float2 w = *reinterpret_cast<const float2*>(st.slot + rec[4 * hf + j] + I8_KW + 2 * (h0 + h));
+        x[j] = __float_as_uint(fmaf(w.x, kuv[4 * hf + j], I8_AOFF));
+        y[j] = __float_as_uint(fmaf(w.y, kuv[4 * hf + j], I8_AOFF));
       }
       limbs4(x[0], x[1], x[2], x[3], a[0][2 * hf], a[1][2 * hf], a[2][2 * hf]);
       limbs4(y[0], y[1], y[2], y[3], a[0][2 * hf + 1], a[1][2 * hf + 1], a[2][2 * hf + 1]);
@@ -773,7 +811,7 @@ __global__ void __launch_bounds__(32 * i8_warps(S), i8_blocks(S))
     k_grid_i8(const __grid_constant__ Geom<float> g, Inputs in, int mode, const VisRecord* __restrict__ rec,
               const uint32_t* __restrict__ sorted, uint64_t kbase, uint64_t kend, uint32_t chunk, uint32_t nbins,
               FixCell* __restrict__ grids, int pg0, int npg, FixScale* __restrict__ fs,
-              const int* __restrict__ run) {
+              const int* __restrict__ run, const __grid_constant__ TapPairs<S> taps) {
   static_assert(S >= 1 && S <= 8, "8 x 8 windows");
   if (run && *run == 0) return;  // a speculative pass's regridding, not needed
   constexpr int W = i8_warps(S), N = 32 * W;
@@ -783,19 +821,14 @@ __global__ void __launch_bounds__(32 * i8_warps(S), i8_blocks(S))
   unsigned long long* flush_buf = reinterpret_cast<unsigned long long*>(smem + (tid >> 5) * I8_FLUSH_BYTES);
   I8Slots<N> st;
   st.carve(smem + W * I8_FLUSH_BYTES);
-  {  // the zero slot: u and w taps 0, B rows at the offset (value 0)
-    float* zk = st.ku + N * I8_KU;
-    uint2* zb = st.bv + N * I8_B;
-    float* zw = st.kw + N * I8_KW;
-    if (tid < I8_KU) zk[tid] = 0.0f;
-    if (tid < I8_B) zb[tid] = make_uint2(0x8080u, 0x8080u);
-    if (tid < I8_KW) zw[tid] = 0.0f;
-    if (tid == 0) st.key[N] = INACTIVE;
-  }
+  // the zero slot: u and w taps 0, B columns at the offset (value 0)
+  if (tid < I8_SLOT) st.slot[N * I8_SLOT + tid] = tid < 16 ? 0x8080u : 0u;
+  if (I8_SLOT > 32 * W && tid + 32 * W < I8_SLOT) st.slot[N * I8_SLOT + tid + 32 * W] = 0u;
+  if (tid == 0) st.key[N] = INACTIVE;
   const uint64_t k0 = kbase + (uint64_t)blockIdx.x * chunk;
   const uint64_t k1 = min(kend, k0 + chunk);
   const float bscale = ldexpf(1.0f, fs->sb);
-  bool bad = false;
+  float bad = 0.0f;  // NaN once a value or a tap's argument was not finite
 
   int acc[NP][2][3][4];
 #pragma unroll
@@ -825,44 +858,43 @@ __global__ void __launch_bounds__(32 * i8_warps(S), i8_blocks(S))
       const float wt = prefetched_wgt(*pre, in);
       const cplx<float> vv = with_vis ? prefetched_vis(*pre, in) : cplx<float>{1.0f, 0.0f};
       float ku[S], kv[S], kw[S];
-      eval_taps2<float, S>(g.coeff, g.ne, r.x0, r.y0, ku, kv);
-      if (g.do_wgridding) eval_taps1<S>(g.coeff, r.xw, kw);
+      eval_taps_pairs<S>(taps, r.x0, ku);
+      eval_taps_pairs<S>(taps, r.y0, kv);
+      if (g.do_wgridding) eval_taps_pairs<S>(taps, r.xw, kw);
       // record_value: value = vis * phase * wgt, imaginary part negated where w was flipped.
       const float flip = (r.meta & 256u) ? -1.0f : 1.0f;
       const float pr = r.ph_re * wt, pi = r.ph_im * wt;
       const float vr = vv.re * pr - vv.im * pi, vi = (vv.re * pi + vv.im * pr) * flip;
-      bad |= !isfinite(vr) || !isfinite(vi) || !isfinite(r.x0) || !isfinite(r.y0) || !isfinite(r.xw);
-      const int mp = (int)(r.meta >> 16), ur = (int)((r.meta >> 9) & 7u), dv = (int)((r.meta >> 4) & 15u);
+      // Zero times anything that is not finite is NaN, and stays.
+      bad = fmaf(vr, 0.0f, fmaf(vi, 0.0f, fmaf(r.x0, 0.0f, fmaf(r.y0, 0.0f, fmaf(r.xw, 0.0f, bad)))));
+      const uint32_t ur = (r.meta >> 9) & 7u, dv = (r.meta >> 4) & 15u;
       const float br = vr * bscale, bi = vi * bscale;
-      uint2 bt[S];
+      uint32_t* rec = st.slot + tid * I8_SLOT;
+      // The value's columns dv .. dv + S - 1, the offset in the others. Planes
+      // outside this pass's are left to the flush, which drops them.
+      uint2* cb = reinterpret_cast<uint2*>(rec);
+#pragma unroll
+      for (int i = S; i < 8; i++) cb[(dv + i) & 7u] = make_uint2(0x8080u, 0x8080u);
+      cb += dv;
 #pragma unroll
       for (int i = 0; i < S; i++)
-        bt[i] = make_uint2((uint32_t)(__float2int_rn(br * kv[i]) + 0x8080), (uint32_t)(__float2int_rn(bi * kv[i]) + 0x8080));
+        cb[i] = make_uint2((uint32_t)(__float2int_rn(br * kv[i]) + 0x8080), (uint32_t)(__float2int_rn(bi * kv[i]) + 0x8080));
       float urow[8];
-      uint2 brow[8];
-      rotate8<S>(ku, ur, urow);
-      place8<S>(bt, dv, make_uint2(0x8080u, 0x8080u), brow);
-      float wrow[8];
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        float w = 0.0f;
-        if (g.do_wgridding) {
-          if (j < S && mp + j >= pg0 && mp + j < pg0 + npg) w = kw[j < S ? j : 0] * I8_ASCALE;
-        } else if (j == 0) {
-          w = I8_ASCALE;
-        }
-        wrow[j] = w;
-      }
-      float2* cu = reinterpret_cast<float2*>(st.ku + tid * I8_KU);
-      uint2* cb = st.bv + tid * I8_B;
-      float2* cw = reinterpret_cast<float2*>(st.kw + tid * I8_KW);
+      rotate8<S>(ku, (int)ur, urow);
+      float2* cu = reinterpret_cast<float2*>(rec + I8_KU);
+      float2* cw = reinterpret_cast<float2*>(rec + I8_KW);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         cu[j] = make_float2(urow[2 * j], urow[2 * j + 1]);
-        cw[j] = make_float2(wrow[2 * j], wrow[2 * j + 1]);
+        float2 w = make_float2(0.0f, 0.0f);
+        if (g.do_wgridding) {
+          if (2 * j < S) w.x = kw[2 * j < S ? 2 * j : 0] * I8_ASCALE;
+          if (2 * j + 1 < S) w.y = kw[2 * j + 1 < S ? 2 * j + 1 : 0] * I8_ASCALE;
+        } else if (j == 0) {
+          w.x = I8_ASCALE;
+        }
+        cw[j] = w;
       }
-#pragma unroll
-      for (int j = 0; j < 8; j++) cb[j] = brow[j];
       st.key[tid] = r.bin;
     }
     // The next round's record and value, in flight while this one is contracted.
@@ -882,15 +914,17 @@ __global__ void __launch_bounds__(32 * i8_warps(S), i8_blocks(S))
       // The run: slots [q, q + len) of bin gk, at most 32.
       const unsigned m = __ballot_sync(0xffffffffu, q + lane < nb && st.key[q + lane] == gk);
       const int len = __popc(m);
-      if (len > 16)
-        i8_contract<NP, 2>(st, q, len, h0, acc);
+      if (len == 32)
+        i8_contract<NP, 2, true>(st, q, len, h0, acc);
+      else if (len > 16)
+        i8_contract<NP, 2, false>(st, q, len, h0, acc);
       else
-        i8_contract<NP, 1>(st, q, len, h0, acc);
+        i8_contract<NP, 1, false>(st, q, len, h0, acc);
       q += len;
     }
   }
   if (win.key != INACTIVE) i8_flush<NP>(g, grids, pg0, npg, win, 8, h0, acc, flush_buf);
-  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&fs->nonfinite, 1);
+  if (__any_sync(0xffffffffu, bad != 0.0f) && lane == 0) atomicOr(&fs->nonfinite, 1);
 }
 
 // ------------------------------------------------------------------ tensor-core degridder
@@ -987,7 +1021,8 @@ __global__ void __launch_bounds__(H16_BATCH, h16_blocks(S))
     k_degrid_h(const __grid_constant__ Geom<float> g, Inputs wts, const VisRecord* __restrict__ rec,
                const uint32_t* __restrict__ sorted, uint64_t kbase, uint64_t kend, uint32_t chunk, uint32_t nbins,
                const cplx<float>* __restrict__ grids, int pg0, int npg, const __grid_constant__ DegridOut out,
-               int first, int last, const uint32_t* __restrict__ kb_ptr, const uint32_t* __restrict__ ke_ptr) {
+               int first, int last, const uint32_t* __restrict__ kb_ptr, const uint32_t* __restrict__ ke_ptr,
+               const __grid_constant__ TapPairs<S> taps) {
   static_assert(S >= 1 && S <= 8, "8 x 8 windows");
   if (kb_ptr) {  // a range the device computed: the grid covers its largest size
     kbase = *kb_ptr;
@@ -1031,9 +1066,10 @@ __global__ void __launch_bounds__(H16_BATCH, h16_blocks(S))
       const VisRecord r = prefetched_record(*pre);
       const float tw = prefetched_wgt(*pre, wts);
       float ku[S], kv[S], kw[S];
-      eval_taps2<float, S>(g.coeff, g.ne, r.x0, r.y0, ku, kv);
-      if (g.do_wgridding) eval_taps1<S>(g.coeff, r.xw, kw);
-      const int mp = (int)(r.meta >> 16), ur = (int)((r.meta >> 9) & 7u), dv = (int)((r.meta >> 4) & 15u);
+      eval_taps_pairs<S>(taps, r.x0, ku);
+      eval_taps_pairs<S>(taps, r.y0, kv);
+      if (g.do_wgridding) eval_taps_pairs<S>(taps, r.xw, kw);
+      const int ur = (int)((r.meta >> 9) & 7u), dv = (int)((r.meta >> 4) & 15u);
 #pragma unroll
       for (int i = 0; i < S; i++) kv[i] *= H16_BSCALE;
       float urow[8], vrow[8], wrow[8];
@@ -1041,10 +1077,11 @@ __global__ void __launch_bounds__(H16_BATCH, h16_blocks(S))
       place8<S>(kv, dv, 0.0f, vrow);
 #pragma unroll
       for (int j = 0; j < 8; j++) {
+        // Planes outside this pass's are zero in the window.
         float w = 0.0f;
         if (g.do_wgridding) {
-          if (j < S && mp + j >= pg0 && mp + j < pg0 + npg) w = kw[j < S ? j : 0];
-        } else if (j == 0 && pg0 == 0) {
+          if (j < S) w = kw[j < S ? j : 0];
+        } else if (j == 0) {
           w = 1.0f;
         }
         wrow[j] = w;
@@ -1162,22 +1199,22 @@ __global__ void __launch_bounds__(H16_BATCH, h16_blocks(S))
           tr[h] = fmaf(kup[h].x, wr[h][0] * invp.x, kup[h].y * (wr[h][1] * invp.y));
           ti[h] = fmaf(kup[h].x, wi[h][0] * invp.x, kup[h].y * (wi[h][1] * invp.y));
         }
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-          for (int o = 1; o < 4; o <<= 1) {
-            tr[h] += __shfl_xor_sync(0xffffffffu, tr[h], o);
-            ti[h] += __shfl_xor_sync(0xffffffffu, ti[h], o);
-          }
-        // Every lane of a quad holds both records' sums: lane tq = h writes record h.
-        const int slot = tq ? sr[1] : sr[0];
+        // Odd lanes of a quad take record gq + 8, even ones record gq: each
+        // gives the other's half away, then the two halves of its own are added.
+        const bool odd = tq & 1;
+        float sr_ = odd ? tr[1] : tr[0], si_ = odd ? ti[1] : ti[0];
+        sr_ += __shfl_xor_sync(0xffffffffu, odd ? tr[0] : tr[1], 1);
+        si_ += __shfl_xor_sync(0xffffffffu, odd ? ti[0] : ti[1], 1);
+        sr_ += __shfl_xor_sync(0xffffffffu, sr_, 2);
+        si_ += __shfl_xor_sync(0xffffffffu, si_, 2);
+        const int slot = odd ? sr[1] : sr[0];
         if (tq < 2 && slot != H16_BATCH) {
           {
             const float4 fo = st.out[slot];
             const uint32_t idx = __float_as_uint(fo.w);
             const uint64_t k = kb + (uint64_t)slot;
             cplx<float>* dst = out.mode == DEGRID_TO_VIS ? out.vis + idx : out.stored + k;
-            cplx<float> accv{tq ? tr[1] : tr[0], (tq ? ti[1] : ti[0]) * fo.z};
+            cplx<float> accv{sr_, si_ * fo.z};
             if (!first) {
               const cplx<float> prev = *dst;
               accv = {accv.re + prev.re, accv.im + prev.im};

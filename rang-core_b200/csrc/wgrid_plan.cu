@@ -2089,7 +2089,7 @@ void launch_grid_i8(cudaStream_t s, const Geom<float>& g, const Inputs& in, int 
   {
     StageTimer timer_(ST_GRID, s);
     fast::k_grid_i8<S><<<nblocks, 32 * W, smem, s>>>(g, in, mode, rec, sorted, kbase, kend, chunk, nbins,
-                                                             grids, pg0, npg, fs, run);
+                                                         grids, pg0, npg, fs, run, fast::TapPairs<S>(g.coeff));
   }
   check_cuda(cudaGetLastError(), "grid kernel (integer tensor cores)");
 }
@@ -2126,7 +2126,8 @@ void launch_degrid_h(cudaStream_t s, const Geom<float>& g, const Inputs& wts, co
   {
     StageTimer timer_(ST_DEGRID, s);
     fast::k_degrid_h<S><<<nblocks, fast::H16_BATCH, smem, s>>>(g, wts, rec, sorted, kbase, kend, chunk, nbins, grids,
-                                                               pg0, npg, out, first, last, kb_ptr, ke_ptr);
+                                                               pg0, npg, out, first, last, kb_ptr, ke_ptr,
+                                                               fast::TapPairs<S>(g.coeff));
   }
   check_cuda(cudaGetLastError(), "degrid kernel (tensor cores)");
 }
