@@ -2112,6 +2112,22 @@ void launch_grid_f64(cudaStream_t s, const Geom<double>& g, const Inputs& in, in
 }
 
 template <int S>
+void launch_degrid_f64(cudaStream_t s, const Geom<double>& g, const Inputs& wts, const double* uvw, const double* foc,
+                       const uint32_t* key, const uint32_t* sorted, uint64_t kbase, uint64_t kend, uint32_t nbins,
+                       const cplx<double>* grids, int pg0, int npg, cplx<double>* vis, int first, int last) {
+  if (kend <= kbase) return;
+  const int smem = (int)(fast::F64DegridSlots::bytes() + fast::F64_BATCH * sizeof(fast::Prefetched64));
+  const uint32_t chunk = warp_chunk(kend - kbase, fast::F64_BLOCKS);
+  const unsigned nblocks = (unsigned)((kend - kbase + chunk - 1) / chunk);
+  {
+    StageTimer timer_(ST_DEGRID, s);
+    fast::k_degrid_f64<S><<<nblocks, fast::F64_BATCH, smem, s>>>(g, wts, uvw, foc, key, sorted, kbase, kend, chunk,
+                                                                 nbins, grids, pg0, npg, vis, first, last);
+  }
+  check_cuda(cudaGetLastError(), "degrid kernel (FP64 tensor cores)");
+}
+
+template <int S>
 void launch_degrid_h(cudaStream_t s, const Geom<float>& g, const Inputs& wts, const fast::VisRecord* rec,
                      const uint32_t* sorted, uint64_t kbase, uint64_t kend, uint32_t nbins,
                      const cplx<float>* grids, int pg0, int npg, const fast::DegridOut& out, int first, int last,
@@ -3128,6 +3144,13 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
                                 last);
           }
           fast_path = true;
+        } else if constexpr (sizeof(T) == 8 && SV <= 8) {
+          if (!fused) {
+            launch_degrid_f64<SV>(s, g_, wts, uvw_.as<double>(), foc_.as<double>(), key_.as<uint32_t>(),
+                                  sorted_.as<uint32_t>(), chunk_sorted_[c], chunk_sorted_[c + 1], (uint32_t)nbins_,
+                                  grids.as<cplx<T>>(), (int)pg0, n, reinterpret_cast<cplx<T>*>(vis), first, last);
+            fast_path = true;
+          }
         }
         if (!fast_path && fused) throw DeviceError("stored values need the tensor-core degridder");
         if (!fast_path)
