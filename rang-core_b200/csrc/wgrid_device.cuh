@@ -30,8 +30,6 @@ struct Inputs {
 
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ void sincos_t(float a, float* s, float* c) { sincosf(a, s, c); }
-__device__ __forceinline__ void sincos_t(double a, double* s, double* c) { sincos(a, s, c); }
 
 // VisData::get (wgridder.rs:950-957): the value in working precision.
 template <class T>
@@ -229,6 +227,21 @@ __device__ __forceinline__ T w_factor(const Geom<T>& g, int nth, int p, double w
   return eval_tap<T, S>(g.coeff, g.ne, nth, locz);
 }
 
+// exp(2 pi i t) for t in turns: the nearest whole number of turns taken off
+// exactly, then sincospi, which needs no reduction by pi. (An angle 2 pi t
+// rounded first, as the reference forms it, is off by its own rounding: the
+// result here is at least as close.)
+__device__ __forceinline__ cplx<float> cis_turns(double t, float) {
+  float s, c;
+  sincospif((float)(2.0 * (t - rint(t))), &s, &c);
+  return {c, s};
+}
+__device__ __forceinline__ cplx<double> cis_turns(double t, double) {
+  double s, c;
+  sincospi(2.0 * (t - rint(t)), &s, &c);
+  return {c, s};
+}
+
 template <class T>
 __device__ __forceinline__ cplx<T> cmul(cplx<T> a, cplx<T> b) {
   return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
@@ -239,15 +252,7 @@ template <class T>
 __device__ __forceinline__ cplx<T> shift_phase(const Geom<T>& g, const double b[3], double imflip,
                                                double f_over_c, double sign) {
   double fct = sign * imflip * (b[0] * g.lshift + b[1] * g.mshift + b[2] * g.nshift);
-  double tmp = fct * f_over_c;
-  T ang;
-  if (sizeof(T) == 4)
-    ang = (T)(2.0 * PI * (tmp - floor(tmp)));
-  else
-    ang = (T)(2.0 * PI * tmp);
-  T s, c;
-  sincos_t(ang, &s, &c);
-  return {c, s};
+  return cis_turns(fct * f_over_c, (T)0);
 }
 
 // unit_value (wgridder.rs:1414-1424).

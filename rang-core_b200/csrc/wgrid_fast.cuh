@@ -265,7 +265,7 @@ static_assert(sizeof(VisRecord) == 32, "records are one 32-byte sector");
 // iteration ahead of their use (the pass otherwise waited on them).
 struct CountIn {
   uint32_t word = 0;
-  double4 b = {0.0, 0.0, 0.0, 1.0};  // the row's coordinates and sign (k_row_coords)
+  double4 b = {0.0, 0.0, 0.0, 0.0};  // the row's coordinates and phase (k_row_coords)
   double f = 0.0;
 };
 __device__ __forceinline__ CountIn count_in(const uint32_t* __restrict__ bits, const double4* __restrict__ rowc,
@@ -278,16 +278,19 @@ __device__ __forceinline__ CountIn count_in(const uint32_t* __restrict__ bits, c
 }
 
 // Each row's coordinates as the binning uses them (row_coord: flips,
-// recentring, w made non-negative) and the sign of that flip, once per row:
+// recentring, w made non-negative; w negated here where that flipped it) and
+// its shift phase in turns per f / c (shift_phase with sign +1), once per row:
 // the count pass then reads them instead of forming them for every channel
 // (the same doubles, so the same keys and records).
 __global__ void k_row_coords(uint64_t nrow, const double* __restrict__ uvw, double fu, double fv, double fw,
-                             double r_l, double r_m, double4* __restrict__ out) {
+                             double r_l, double r_m, double lshift, double mshift, double nshift,
+                             double4* __restrict__ out) {
   for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < nrow;
        r += (uint64_t)gridDim.x * blockDim.x) {
     double b[3];
     const double sgn = row_coord(uvw, r, fu, fv, fw, r_l, r_m, b);
-    out[r] = make_double4(b[0], b[1], b[2], sgn);
+    const double turns = sgn * (b[0] * lshift + b[1] * mshift + b[2] * nshift);
+    out[r] = make_double4(b[0], b[1], copysign(b[2], sgn), turns);
   }
 }
 
@@ -325,10 +328,8 @@ __global__ void __launch_bounds__(256, COUNT_BLOCKS)
     if (i < n) {
       act = ((cur.word >> (i & 31)) & 1u) != 0;
       if (act) {
-        const double b[3] = {cur.b.x, cur.b.y, cur.b.z};
-        const double imflip = cur.b.w;
         const double f = cur.f;
-        const double u = b[0] * f, v = b[1] * f, w = b[2] * f;
+        const double u = cur.b.x * f, v = cur.b.y * f, w = fabs(cur.b.z) * f;
         double uf, vf;
         int iu0, iv0;
         getpix(g, u, v, uf, vf, iu0, iv0);
@@ -353,12 +354,12 @@ __global__ void __launch_bounds__(256, COUNT_BLOCKS)
         }
         float ph_re = 1.0f, ph_im = 0.0f;
         if (SHIFT) {
-          const cplx<float> ph = shift_phase<float>(g, b, imflip, f, 1.0);
+          const cplx<float> ph = cis_turns(cur.b.w * f, 0.0f);
           ph_re = ph.re;
           ph_im = ph.im;
         }
         const uint32_t meta = (((sv & tmask) - sb * se) << 4) |
-                              (imflip < 0.0 ? 256u : 0u) | ((su & 7u) << 9) | ((uint32_t)mp << 16);
+                              (signbit(cur.b.z) ? 256u : 0u) | ((su & 7u) << 9) | ((uint32_t)mp << 16);
         reinterpret_cast<uint4*>(rec + i)[0] =
             make_uint4(__float_as_uint(x0), __float_as_uint(y0), __float_as_uint(xw), (uint32_t)i);
         reinterpret_cast<uint4*>(rec + i)[1] = make_uint4(__float_as_uint(ph_re), __float_as_uint(ph_im), meta, k);

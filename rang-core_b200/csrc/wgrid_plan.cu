@@ -1641,16 +1641,8 @@ __device__ __forceinline__ double screen_arg(const Geom<T>& g, int i, int j) {
 template <class T>
 __device__ __forceinline__ cplx<T> screen(const Geom<T>& g, double s, int p, bool adjoint) {
   double w0 = g.wmin + (double)p * g.dw;
-  double phs = w0 * s;
-  if (adjoint) phs *= -1.0;
-  T ang;
-  if (sizeof(T) == 4)
-    ang = (T)(2.0 * PI * (phs - floor(phs)));
-  else
-    ang = (T)(2.0 * PI * phs);
-  T sn, cs;
-  sincos_t(ang, &sn, &cs);
-  return {cs, sn};
+  const double phs = w0 * s;
+  return cis_turns(adjoint ? -phs : phs, (T)0);
 }
 
 // global_corrections (wgridder.rs:822-861) per pixel, full image.
@@ -2527,7 +2519,8 @@ template <class T>
 void Plan<T>::row_coords(DevBuf& out, cudaStream_t s) const {
   if (nrow_ == 0) return;
   fast::k_row_coords<<<blocks_for(nrow_, 256, 148u * 8u), 256, 0, s>>>(nrow_, uvw_.as<double>(), g_.fu, g_.fv, g_.fw,
-                                                                       g_.r_l, g_.r_m, out.as<double4>());
+                                                                       g_.r_l, g_.r_m, g_.lshift, g_.mshift, g_.nshift,
+                                                                       out.as<double4>());
   check_cuda(cudaGetLastError(), "row coordinates");
 }
 
