@@ -226,11 +226,14 @@ struct FixTraits<double> {
   }
 };
 
-// One plane of the fixed-point grid to floating point: rows [0, rows) and
-// [nu - rows, nu) (every row when rows is 0), each cell rounded once.
+// Planes (one per blockIdx.y) of the fixed-point grid to floating point: rows
+// [0, rows) and [nu - rows, nu) (every row when rows is 0), each cell rounded
+// once.
 template <class T>
 __global__ void k_fix_to_plane(const typename FixTraits<T>::Cell* __restrict__ fix, int nu, int nv, int rows,
                                const FixScale* fs, cplx<T>* __restrict__ out) {
+  fix += (size_t)blockIdx.y * nu * nv;
+  out += (size_t)blockIdx.y * nu * nv;
   const int q = fs->q;
   const bool nan = fs->nonfinite != 0;
   const int nr = rows == 0 ? nu : 2 * rows;

@@ -1786,11 +1786,14 @@ __global__ void k_place(const __grid_constant__ Geom<T> g, const T* __restrict__
 // jx(j) = (nv - ny/2 + j) mod nv of a plane, so that each is one contiguous
 // length-nu transform (a single cuFFT pass, where the strided columns took
 // four). `rows` is the touched-row count of fft_touched_rows (0: all rows):
-// the other rows are zero after gridding and are written as zeros unread.
+// the other rows are zero after gridding and are written as zeros unread. One
+// plane per blockIdx.z.
 template <class T>
 __global__ void k_cols_to_t(const __grid_constant__ Geom<T> g, const cplx<T>* __restrict__ plane, int rows,
                             cplx<T>* __restrict__ t) {
   __shared__ cplx<T> tile[32][33];
+  plane += (size_t)blockIdx.z * g.nu * g.nv;
+  t += (size_t)blockIdx.z * g.ny * g.nu;
   const int u0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {  // plane rows: consecutive j
     const int u = u0 + k, j = j0 + threadIdx.x;
@@ -1812,6 +1815,8 @@ template <class T>
 __global__ void k_t_to_cols(const __grid_constant__ Geom<T> g, const cplx<T>* __restrict__ t, int rows,
                             cplx<T>* __restrict__ plane) {
   __shared__ cplx<T> tile[32][33];
+  t += (size_t)blockIdx.z * g.ny * g.nu;
+  plane += (size_t)blockIdx.z * g.nu * g.nv;
   const int u0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {  // t rows: consecutive u
     const int j = j0 + k, u = u0 + threadIdx.x;
@@ -1826,10 +1831,13 @@ __global__ void k_t_to_cols(const __grid_constant__ Geom<T> g, const cplx<T>* __
 }
 
 // k_place into the transposed columns: t[j][ix] (t zeroed first). Consecutive
-// threads take consecutive image rows i, so that the writes are contiguous.
+// threads take consecutive image rows i, so that the writes are contiguous. Plane
+// p + blockIdx.y into its columns.
 template <class T>
 __global__ void k_place_t(const __grid_constant__ Geom<T> g, const T* __restrict__ img, int p,
                           cplx<T>* __restrict__ t) {
+  p += (int)blockIdx.y;
+  t += (size_t)blockIdx.y * g.ny * g.nu;
   uint64_t npix = (uint64_t)g.nx * g.ny;
   for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < npix; q += (uint64_t)gridDim.x * blockDim.x) {
     int j = (int)(q / g.nx), i = (int)(q - (uint64_t)j * g.nx);
@@ -1880,8 +1888,8 @@ struct FftTraits<double> {
   }
 };
 
-struct FftPair {
-  cufftHandle rows = 0, cols = 0;
+struct FftPlan {
+  cufftHandle h = 0;
   std::mutex mu;
 };
 
@@ -1889,65 +1897,30 @@ void check_fft(cufftResult r, const char* what) {
   if (r != CUFFT_SUCCESS) throw DeviceError(std::string("cuFFT ") + what + " failed (" + std::to_string((int)r) + ")");
 }
 
-// Row transforms (length nv, nu rows) and image-column transforms (length nu,
-// ny/2 columns of stride nv) of one grid size, per device, kept for the life
-// of the process.
+// `batch` consecutive transforms of length `n`, per device, kept for the life
+// of the process (touched-row batches are rounded up to 64 so that few exist).
 template <class T>
-FftPair& fft_plans(int nu, int nv, int ny) {
+FftPlan& fft_plan(int n, int batch) {
   static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int>, std::unique_ptr<FftPair>> cache;
+  static std::map<std::tuple<int, int, int>, std::unique_ptr<FftPlan>> cache;
   int dev = 0;
   check_cuda(cudaGetDevice(&dev), "device");
   std::lock_guard<std::mutex> lock(mu);
-  auto key = std::make_tuple(dev, nu, nv, ny);
-  auto& slot = cache[key];
+  auto& slot = cache[std::make_tuple(dev, n, batch)];
   if (!slot) {
-    auto p = std::make_unique<FftPair>();
-    int n_row[1] = {nv};
-    check_fft(cufftPlanMany(&p->rows, 1, n_row, nullptr, 1, nv, nullptr, 1, nv, FftTraits<T>::type, nu), "row plan");
-    int n_col[1] = {nu};
-    int emb[1] = {nu};
-    check_fft(cufftPlanMany(&p->cols, 1, n_col, emb, nv, 1, emb, nv, 1, FftTraits<T>::type, ny / 2), "column plan");
+    auto p = std::make_unique<FftPlan>();
+    int len[1] = {n};
+    check_fft(cufftPlanMany(&p->h, 1, len, nullptr, 1, n, nullptr, 1, n, FftTraits<T>::type, batch), "plan");
     slot = std::move(p);
   }
   return *slot;
 }
 
-// The image-column transforms of one plane: columns [nv - ny/2, nv) and [0, ny/2).
 template <class T>
-void fft_cols(FftPair& f, cplx<T>* plane, int nv, int ny, int dir, cudaStream_t s) {
+void fft_exec(FftPlan& f, cplx<T>* p, int dir, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(f.mu);
-  check_fft(cufftSetStream(f.cols, s), "stream");
-  check_fft(FftTraits<T>::exec(f.cols, plane + (nv - ny / 2), dir), "columns");
-  check_fft(FftTraits<T>::exec(f.cols, plane, dir), "columns");
-}
-
-template <class T>
-void fft_rows(FftPair& f, cplx<T>* plane, int dir, cudaStream_t s) {
-  std::lock_guard<std::mutex> lock(f.mu);
-  check_fft(cufftSetStream(f.rows, s), "stream");
-  check_fft(FftTraits<T>::exec(f.rows, plane, dir), "rows");
-}
-
-// Row transforms (length nv) of `batch` consecutive rows, per device, kept
-// for the life of the process; batches are rounded up to 64 rows so that few
-// plans exist.
-template <class T>
-FftPair& fft_row_plan(int nv, int batch) {
-  static std::mutex mu;
-  static std::map<std::tuple<int, int, int>, std::unique_ptr<FftPair>> cache;
-  int dev = 0;
-  check_cuda(cudaGetDevice(&dev), "device");
-  std::lock_guard<std::mutex> lock(mu);
-  auto& slot = cache[std::make_tuple(dev, nv, batch)];
-  if (!slot) {
-    auto p = std::make_unique<FftPair>();
-    int n_row[1] = {nv};
-    check_fft(cufftPlanMany(&p->rows, 1, n_row, nullptr, 1, nv, nullptr, 1, nv, FftTraits<T>::type, batch),
-              "row plan");
-    slot = std::move(p);
-  }
-  return *slot;
+  check_fft(cufftSetStream(f.h, s), "stream");
+  check_fft(FftTraits<T>::exec(f.h, p, dir), "transform");
 }
 
 // The touched rows as transformed: urows rounded up to 64, or 0 (every row)
@@ -1960,16 +1933,20 @@ int touched_row_count(int urows, int nu) {
 // The v transforms of the rows footprints can touch: storage rows [0, b)
 // and [nu - b, nu), b = touched_row_count (every row when b is 0).
 template <class T>
-void fft_touched_rows(FftPair& all, cplx<T>* plane, int nu, int nv, int b, int dir, cudaStream_t s) {
-  if (b == 0) {
-    fft_rows<T>(all, plane, dir, s);
-    return;
-  }
-  FftPair& f = fft_row_plan<T>(nv, b);
-  std::lock_guard<std::mutex> lock(f.mu);
-  check_fft(cufftSetStream(f.rows, s), "stream");
-  check_fft(FftTraits<T>::exec(f.rows, plane, dir), "rows");
-  check_fft(FftTraits<T>::exec(f.rows, plane + (size_t)(nu - b) * nv, dir), "rows");
+void fft_touched_rows(cplx<T>* plane, int nu, int nv, int b, int dir, cudaStream_t s) {
+  FftPlan& f = fft_plan<T>(nv, b == 0 ? nu : b);
+  fft_exec<T>(f, plane, dir, s);
+  if (b) fft_exec<T>(f, plane + (size_t)(nu - b) * nv, dir, s);
+}
+
+// Whether the transforms of n planes (their cells and image columns) run as
+// one launch per step over all of them instead of plane by plane: where a
+// plane's launches are shorter than it takes to issue them. At 7 planes of
+// 462^2 28 launches of 2 to 5 us each became 4; from about 64 MB a plane's
+// steps fill the chip and meet the plane in L2.
+constexpr size_t BATCH_BYTES = (size_t)64 << 20;
+bool batch_planes(int n, size_t plane, size_t tplane, size_t cell) {
+  return (size_t)n * (plane + tplane) * cell <= BATCH_BYTES && (size_t)n * std::max(plane, tplane) < (1u << 30);
 }
 
 template <class T, int S>
@@ -2743,9 +2720,13 @@ void Plan<T>::corrections(cudaStream_t s) {
 
 // Planes that fit at once: each takes `plane_bytes` (its grid and its image
 // columns, transposed); `fixed` bytes more are needed whatever the group.
+// Without `ask`, work spaces of at most 64 MB are taken to fit (the question
+// takes the driver 0.1 ms, a tenth of a small call); a caller whose allocation
+// then fails asks.
 template <class T>
-size_t Plan<T>::plane_group(size_t plane_bytes, size_t fixed) const {
+size_t Plan<T>::plane_group(size_t plane_bytes, size_t fixed, bool ask) const {
   size_t nplanes = (size_t)std::max(g_.nplanes, 1);
+  if (!ask && nplanes * plane_bytes + fixed <= ((size_t)64 << 20)) return nplanes;
   size_t freeb = 0, total = 0;
   check_cuda(cudaMemGetInfo(&freeb, &total), "memory info");
   auto group_of = [&](size_t avail) {
@@ -2792,21 +2773,21 @@ void zero_touched(void* grids, size_t cell_bytes, int n, int nu, int nv, int row
 // its image columns (transposed), and whatever the group the floating-point
 // plane being transformed and the image accumulator.
 template <class T>
-void Plan<T>::grid_sizes(size_t& plane_bytes, size_t& fixed, size_t& group) const {
+void Plan<T>::grid_sizes(size_t& plane_bytes, size_t& fixed, size_t& group, bool ask) const {
   using FixCell = typename fast::FixTraits<T>::Cell;
   const size_t npix = (size_t)o_.nx * o_.ny;
   const size_t plane = (size_t)g_.nu * g_.nv;
   const size_t tplane = (size_t)g_.ny * g_.nu;
   plane_bytes = plane * sizeof(FixCell) + tplane * sizeof(cplx<T>);
   fixed = plane * sizeof(cplx<T>) + npix * sizeof(T);
-  group = plane_group(plane_bytes, fixed);
+  group = plane_group(plane_bytes, fixed, ask);
 }
 
 template <class T>
 size_t Plan<T>::footprint(int nout) const {
   if (nvis_ == 0) return 0;
   size_t plane_bytes, fixed, group;
-  grid_sizes(plane_bytes, fixed, group);
+  grid_sizes(plane_bytes, fixed, group, true);
   return (size_t)std::max(nout, 1) * (group * plane_bytes + fixed);
 }
 
@@ -2825,12 +2806,22 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
   const size_t plane = (size_t)g_.nu * g_.nv;
   const size_t tplane = (size_t)g_.ny * g_.nu;  // a plane's image columns, transposed
   size_t plane_bytes, fixed, group;
-  grid_sizes(plane_bytes, fixed, group);
-  DevBuf grids(group * plane * sizeof(FixCell), s);
-  DevBuf fpl(plane * cell, s);  // the plane being transformed, in floating point
-  DevBuf cols(group * tplane * cell, s);
+  DevBuf grids, fpl, cols;  // the fixed-point planes; planes being transformed; their image columns
+  bool batched = false;
+  auto take = [&](bool ask) {
+    grid_sizes(plane_bytes, fixed, group, ask);
+    batched = batch_planes((int)group, plane, tplane, cell);
+    grids.alloc(group * plane * sizeof(FixCell), s);
+    fpl.alloc((batched ? group : 1) * plane * cell, s);
+    cols.alloc(group * tplane * cell, s);
+  };
+  try {
+    take(false);
+  } catch (const DeviceError&) {
+    cudaGetLastError();
+    take(true);
+  }
   DevBuf acc(group < nplanes ? npix * sizeof(T) : 0, s);
-  FftPair& fft = fft_plans<T>(g_.nu, g_.nv, g_.ny);
   const int gmax =
       std::min<int>(max_window_planes(g_.L, sizeof(FixCell)), (int)std::min<size_t>(nplanes, 64));
   const int smem = gmax * g_.L * g_.L * (int)sizeof(FixCell);
@@ -2941,24 +2932,29 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
     else
       with_supp_double(g_.supp, run);
     const dim3 tgrid((unsigned)((g_.nu + 31) / 32), (unsigned)((g_.ny + 31) / 32)), tblock(32, 8);
-    FftPair& tf = fft_row_plan<T>(g_.nu, g_.ny);  // the image columns, transposed: ny transforms of length nu
-    for (int p = 0; p < n; p++) {
+    // One plane a step, or (batched) all n: rows along v, the image columns
+    // transposed, ny transforms of length nu each. Batched, untouched rows are
+    // transformed as they are: nothing reads them.
+    const int step = batched ? n : 1;
+    for (int p = 0; p < n; p += step) {
       const FixCell* fpg = fg + (size_t)p * plane;
       cplx<T>* pl = fpl.as<cplx<T>>();
       cplx<T>* tp = cols.as<cplx<T>>() + (size_t)p * tplane;
       {
         StageTimer timer_(ST_FIXED, s);
         const uint64_t ncell = (uint64_t)(rows == 0 ? g_.nu : 2 * rows) * g_.nv;
-        fast::k_fix_to_plane<T><<<blocks_for(ncell, 256), 256, 0, s>>>(fpg, g_.nu, g_.nv, rows, fs, pl);
+        fast::k_fix_to_plane<T>
+            <<<dim3(blocks_for(ncell, 256), (unsigned)step), 256, 0, s>>>(fpg, g_.nu, g_.nv, rows, fs, pl);
       }
       check_cuda(cudaGetLastError(), "fixed point");
       StageTimer timer_(ST_FFT, s, 3);
-      fft_touched_rows<T>(fft, pl, g_.nu, g_.nv, rows, CUFFT_INVERSE, s);
-      k_cols_to_t<T><<<tgrid, tblock, 0, s>>>(g_, pl, rows, tp);
+      if (batched)
+        fft_exec<T>(fft_plan<T>(g_.nv, n * g_.nu), pl, CUFFT_INVERSE, s);
+      else
+        fft_touched_rows<T>(pl, g_.nu, g_.nv, rows, CUFFT_INVERSE, s);
+      k_cols_to_t<T><<<dim3(tgrid.x, tgrid.y, (unsigned)step), tblock, 0, s>>>(g_, pl, rows, tp);
       check_cuda(cudaGetLastError(), "transpose");
-      std::lock_guard<std::mutex> lock(tf.mu);
-      check_fft(cufftSetStream(tf.rows, s), "stream");
-      check_fft(FftTraits<T>::exec(tf.rows, tp, CUFFT_INVERSE), "columns");
+      fft_exec<T>(fft_plan<T>(g_.nu, step * g_.ny), tp, CUFFT_INVERSE, s);
     }
     bool first = pg0 == 0, last = pg0 + n >= nplanes;
     {
@@ -3064,10 +3060,22 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
   const size_t nplanes = (size_t)std::max(g_.nplanes, 1);
   const size_t plane = (size_t)g_.nu * g_.nv;
   const size_t tplane = (size_t)g_.ny * g_.nu;  // a plane's image columns, transposed
-  const size_t group = plane_group(plane * cell, tplane * cell + npix * sizeof(T));
-  DevBuf grids(group * plane * cell, s);
-  DevBuf img(npix * sizeof(T), s);
-  FftPair& fft = fft_plans<T>(g_.nu, g_.nv, g_.ny);
+  size_t group = 0;
+  DevBuf grids, img, cols;
+  bool batched = false;
+  auto take = [&](bool ask) {
+    group = plane_group(plane * cell, tplane * cell + npix * sizeof(T), ask);
+    batched = batch_planes((int)group, plane, tplane, cell);
+    grids.alloc(group * plane * cell, s);
+    img.alloc(npix * sizeof(T), s);
+    cols.alloc((batched ? group : 1) * tplane * cell, s);
+  };
+  try {
+    take(false);
+  } catch (const DeviceError&) {
+    cudaGetLastError();
+    take(true);
+  }
   const double* corr = corr_.as<double>();
   const size_t nu2 = (size_t)g_.nx / 2 + 1, nv2 = (size_t)g_.ny / 2 + 1;
   {
@@ -3082,31 +3090,28 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
       (int)std::min<size_t>(nplanes, 64));
   const int smem = gmax * g_.L * Lp * (int)sizeof(cplx<T>);
   const int rows = touched_row_count(urows_, g_.nu);
-  DevBuf cols(tplane * cell, s);
   const dim3 tgrid((unsigned)((g_.nu + 31) / 32), (unsigned)((g_.ny + 31) / 32)), tblock(32, 8);
-  FftPair& tf = fft_row_plan<T>(g_.nu, g_.ny);
   for (size_t pg0 = 0; pg0 < nplanes; pg0 += group) {
     int n = (int)std::min(group, nplanes - pg0);
     zero_touched(grids.get(), cell, n, g_.nu, g_.nv, rows, s);
-    for (int p = 0; p < n; p++) {
+    const int step = batched ? n : 1;  // planes a step, as in grid
+    for (int p = 0; p < n; p += step) {
       cplx<T>* pl = grids.as<cplx<T>>() + (size_t)p * plane;
-      check_cuda(cudaMemsetAsync(cols.get(), 0, tplane * cell, s), "memset");
+      check_cuda(cudaMemsetAsync(cols.get(), 0, (size_t)step * tplane * cell, s), "memset");
       {
         StageTimer timer_(ST_PLACE, s);
-        k_place_t<T><<<blocks_for(npix, 256), 256, 0, s>>>(g_, img.as<T>(), (int)pg0 + p, cols.as<cplx<T>>());
+        k_place_t<T><<<dim3(blocks_for(npix, 256), (unsigned)step), 256, 0, s>>>(g_, img.as<T>(), (int)pg0 + p,
+                                                                                 cols.as<cplx<T>>());
       }
       check_cuda(cudaGetLastError(), "place");
-      {
-        StageTimer timer_(ST_FFT, s, 3);
-        {
-          std::lock_guard<std::mutex> lock(tf.mu);
-          check_fft(cufftSetStream(tf.rows, s), "stream");
-          check_fft(FftTraits<T>::exec(tf.rows, cols.as<cplx<T>>(), CUFFT_FORWARD), "columns");
-        }
-        k_t_to_cols<T><<<tgrid, tblock, 0, s>>>(g_, cols.as<cplx<T>>(), rows, pl);
-        check_cuda(cudaGetLastError(), "transpose");
-        fft_touched_rows<T>(fft, pl, g_.nu, g_.nv, rows, CUFFT_FORWARD, s);
-      }
+      StageTimer timer_(ST_FFT, s, 3);
+      fft_exec<T>(fft_plan<T>(g_.nu, step * g_.ny), cols.as<cplx<T>>(), CUFFT_FORWARD, s);
+      k_t_to_cols<T><<<dim3(tgrid.x, tgrid.y, (unsigned)step), tblock, 0, s>>>(g_, cols.as<cplx<T>>(), rows, pl);
+      check_cuda(cudaGetLastError(), "transpose");
+      if (batched)
+        fft_exec<T>(fft_plan<T>(g_.nv, n * g_.nu), pl, CUFFT_FORWARD, s);
+      else
+        fft_touched_rows<T>(pl, g_.nu, g_.nv, rows, CUFFT_FORWARD, s);
     }
     bool first = pg0 == 0, last = pg0 + n >= nplanes;
     auto run = [&](auto S) {

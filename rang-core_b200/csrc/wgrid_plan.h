@@ -183,10 +183,10 @@ class Plan {
   // writes the stored values in sorted order, the integer gridder reads them).
   bool fused_values() const;
   // Bytes of one gridding plane group and of the fixed part, and the group.
-  void grid_sizes(size_t& plane_bytes, size_t& fixed, size_t& group) const;
+  void grid_sizes(size_t& plane_bytes, size_t& fixed, size_t& group, bool ask = false) const;
   void corrections(cudaStream_t s);
   int touched_rows(double umax, double wmax) const;
-  size_t plane_group(size_t plane_bytes, size_t fixed) const;
+  size_t plane_group(size_t plane_bytes, size_t fixed, bool ask = false) const;
 
   WgridderOptions o_;
   size_t nrow_, nchan_, n_;
