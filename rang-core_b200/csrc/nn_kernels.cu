@@ -25,6 +25,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 
@@ -398,98 +399,122 @@ union V8 {
   bf162 h[4];
 };
 
-// out[b, y, x, c] = mean of in[b, 2y + i, 2x + j, c] (H, W the input size).
-__global__ void k_pool(const bf16* __restrict__ in, int ld_in, bf16* __restrict__ out, int ld_out, int64_t B, int H,
-                       int W, int C) {
-  const int h = H / 2, w = W / 2, c8 = C / 8;
-  const int64_t n = B * h * w * c8;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % c8) * 8;
-    const int64_t q = i / c8;
-    const int x = (int)(q % w), y = (int)((q / w) % h);
-    const int64_t b = q / ((int64_t)w * h);
-    const int64_t p = (b * H + 2 * y) * W + 2 * x;
+// The kernels below move tensors once and are bound by HBM; a thread takes
+// eight channels (16 bytes) of one low-resolution pixel and its 2 x 2 group, so
+// that the index arithmetic (in I: 32 bits unless the tensor needs more; 64-bit
+// divisions per element held them to half the bandwidth) is done once for
+// five accesses.
+template <class I>
+struct Group {
+  I q, p;  // the low-resolution pixel; the first of its 2 x 2 group
+  int c;   // the first of its channels
+};
+// Element i of (B, h, w, c8): h x w the low resolution.
+template <class I>
+__device__ __forceinline__ Group<I> group_of(I i, int h, int w, int c8) {
+  const I q = i / (I)c8, row = q / (I)w, b = row / (I)h;
+  Group<I> g;
+  g.q = q;
+  g.c = (int)(i - q * (I)c8) * 8;
+  const I y = row - b * (I)h, x = q - row * (I)w;
+  g.p = ((b * (I)h + y) * 2 * (I)w + x) * 2;  // (b * 2h + 2y) * 2w + 2x
+  return g;
+}
+
+// out[b, y, x, c] = mean of in[b, 2y + i, 2x + j, c] (h, w the output size).
+template <class I>
+__global__ void __launch_bounds__(256) k_pool(const bf16* __restrict__ in, int ld_in, bf16* __restrict__ out,
+                                              int ld_out, I n, int h, int w, int c8) {
+  const I W = 2 * (I)w;
+  for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < n; i += (I)gridDim.x * blockDim.x) {
+    const Group<I> g = group_of<I>(i, h, w, c8);
+    const bf16* s = in + (int64_t)g.p * ld_in + g.c;
     V8 v[4], o;
-    v[0].u = *reinterpret_cast<const uint4*>(in + p * ld_in + c);
-    v[1].u = *reinterpret_cast<const uint4*>(in + (p + 1) * ld_in + c);
-    v[2].u = *reinterpret_cast<const uint4*>(in + (p + W) * ld_in + c);
-    v[3].u = *reinterpret_cast<const uint4*>(in + (p + W + 1) * ld_in + c);
+    v[0].u = *reinterpret_cast<const uint4*>(s);
+    v[1].u = *reinterpret_cast<const uint4*>(s + ld_in);
+    v[2].u = *reinterpret_cast<const uint4*>(s + (int64_t)W * ld_in);
+    v[3].u = *reinterpret_cast<const uint4*>(s + ((int64_t)W + 1) * ld_in);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const float2 s0 = __bfloat1622float2(v[0].h[k]), s1 = __bfloat1622float2(v[1].h[k]);
       const float2 s2 = __bfloat1622float2(v[2].h[k]), s3 = __bfloat1622float2(v[3].h[k]);
       o.h[k] = __floats2bfloat162_rn(0.25f * (((s0.x + s1.x) + s2.x) + s3.x), 0.25f * (((s0.y + s1.y) + s2.y) + s3.y));
     }
-    *reinterpret_cast<uint4*>(out + q * ld_out + c) = o.u;
+    *reinterpret_cast<uint4*>(out + (int64_t)g.q * ld_out + g.c) = o.u;
   }
 }
 
 // g[p, c] = (g[p, c] + dpool[p / 2, c] / 4) * (act[p, c] > 0), in place: the
 // gradient of an encoder output that feeds both the skip connection (g holds
-// that part) and the pooling.
-__global__ void k_pool_backward(bf16* __restrict__ g, int ld_g, const bf16* __restrict__ dpool, int ld_dp,
-                                const bf16* __restrict__ act, int ld_act, int64_t B, int H, int W, int C) {
-  const int c8 = C / 8, h = H / 2, w = W / 2;
-  const int64_t n = B * H * W * c8;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % c8) * 8;
-    const int64_t p = i / c8;
-    const int x = (int)(p % W), y = (int)((p / W) % H);
-    const int64_t b = p / ((int64_t)W * H);
-    const int64_t q = (b * h + y / 2) * w + x / 2;
-    V8 gv, dv, av;
-    gv.u = *reinterpret_cast<const uint4*>(g + p * ld_g + c);
-    dv.u = *reinterpret_cast<const uint4*>(dpool + q * ld_dp + c);
-    av.u = *reinterpret_cast<const uint4*>(act + p * ld_act + c);
+// that part) and the pooling (h, w the pooled size).
+template <class I>
+__global__ void __launch_bounds__(256)
+    k_pool_backward(bf16* __restrict__ grad, int ld_g, const bf16* __restrict__ dpool, int ld_dp,
+                    const bf16* __restrict__ act, int ld_act, I n, int h, int w, int c8) {
+  const I W = 2 * (I)w;
+  for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < n; i += (I)gridDim.x * blockDim.x) {
+    const Group<I> g = group_of<I>(i, h, w, c8);
+    V8 dv, gv[4], av[4];
+    dv.u = *reinterpret_cast<const uint4*>(dpool + (int64_t)g.q * ld_dp + g.c);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const float2 s = __bfloat1622float2(gv.h[k]), d = __bfloat1622float2(dv.h[k]), m = __bfloat1622float2(av.h[k]);
-      const float v0 = m.x > 0.0f ? s.x + 0.25f * d.x : 0.0f;
-      const float v1 = m.y > 0.0f ? s.y + 0.25f * d.y : 0.0f;
-      gv.h[k] = __floats2bfloat162_rn(v0, v1);
+    for (int j = 0; j < 4; j++) {
+      const int64_t p = (int64_t)g.p + (j & 1) + (j >> 1) * (int64_t)W;
+      gv[j].u = *reinterpret_cast<const uint4*>(grad + p * ld_g + g.c);
+      av[j].u = *reinterpret_cast<const uint4*>(act + p * ld_act + g.c);
     }
-    *reinterpret_cast<uint4*>(g + p * ld_g + c) = gv.u;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int64_t p = (int64_t)g.p + (j & 1) + (j >> 1) * (int64_t)W;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const float2 s = __bfloat1622float2(gv[j].h[k]), d = __bfloat1622float2(dv.h[k]);
+        const float2 m = __bfloat1622float2(av[j].h[k]);
+        const float v0 = m.x > 0.0f ? s.x + 0.25f * d.x : 0.0f;
+        const float v1 = m.y > 0.0f ? s.y + 0.25f * d.y : 0.0f;
+        gv[j].h[k] = __floats2bfloat162_rn(v0, v1);
+      }
+      *reinterpret_cast<uint4*>(grad + p * ld_g + g.c) = gv[j].u;
+    }
   }
 }
 
-// out[b, y, x, c] = in[b, y / 2, x / 2, c] (H, W the output size).
-__global__ void k_upsample(const bf16* __restrict__ in, int ld_in, bf16* __restrict__ out, int ld_out, int64_t B,
-                           int H, int W, int C) {
-  const int c8 = C / 8, h = H / 2, w = W / 2;
-  const int64_t n = B * H * W * c8;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % c8) * 8;
-    const int64_t p = i / c8;
-    const int x = (int)(p % W), y = (int)((p / W) % H);
-    const int64_t b = p / ((int64_t)W * H);
-    const int64_t q = (b * h + y / 2) * w + x / 2;
-    *reinterpret_cast<uint4*>(out + p * ld_out + c) = *reinterpret_cast<const uint4*>(in + q * ld_in + c);
+// out[b, y, x, c] = in[b, y / 2, x / 2, c] (h, w the input size).
+template <class I>
+__global__ void __launch_bounds__(256) k_upsample(const bf16* __restrict__ in, int ld_in, bf16* __restrict__ out,
+                                                  int ld_out, I n, int h, int w, int c8) {
+  const I W = 2 * (I)w;
+  for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < n; i += (I)gridDim.x * blockDim.x) {
+    const Group<I> g = group_of<I>(i, h, w, c8);
+    const uint4 v = *reinterpret_cast<const uint4*>(in + (int64_t)g.q * ld_in + g.c);
+    bf16* d = out + (int64_t)g.p * ld_out + g.c;
+    *reinterpret_cast<uint4*>(d) = v;
+    *reinterpret_cast<uint4*>(d + ld_out) = v;
+    *reinterpret_cast<uint4*>(d + (int64_t)W * ld_out) = v;
+    *reinterpret_cast<uint4*>(d + ((int64_t)W + 1) * ld_out) = v;
   }
 }
 
-// out[b, y, x, c] = sum of g[b, 2y + i, 2x + j, c] (H, W the output size).
-__global__ void k_upsample_backward(const bf16* __restrict__ g, int ld_g, bf16* __restrict__ out, int ld_out,
-                                    int64_t B, int H, int W, int C) {
-  const int c8 = C / 8, W2 = 2 * W;
-  const int64_t n = B * H * W * c8;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % c8) * 8;
-    const int64_t q = i / c8;
-    const int x = (int)(q % W), y = (int)((q / W) % H);
-    const int64_t b = q / ((int64_t)W * H);
-    const int64_t p = (b * 2 * H + 2 * y) * W2 + 2 * x;
+// out[b, y, x, c] = sum of g[b, 2y + i, 2x + j, c] (h, w the output size).
+template <class I>
+__global__ void __launch_bounds__(256) k_upsample_backward(const bf16* __restrict__ grad, int ld_g,
+                                                           bf16* __restrict__ out, int ld_out, I n, int h, int w,
+                                                           int c8) {
+  const I W = 2 * (I)w;
+  for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < n; i += (I)gridDim.x * blockDim.x) {
+    const Group<I> g = group_of<I>(i, h, w, c8);
+    const bf16* s = grad + (int64_t)g.p * ld_g + g.c;
     V8 v[4], o;
-    v[0].u = *reinterpret_cast<const uint4*>(g + p * ld_g + c);
-    v[1].u = *reinterpret_cast<const uint4*>(g + (p + 1) * ld_g + c);
-    v[2].u = *reinterpret_cast<const uint4*>(g + (p + W2) * ld_g + c);
-    v[3].u = *reinterpret_cast<const uint4*>(g + (p + W2 + 1) * ld_g + c);
+    v[0].u = *reinterpret_cast<const uint4*>(s);
+    v[1].u = *reinterpret_cast<const uint4*>(s + ld_g);
+    v[2].u = *reinterpret_cast<const uint4*>(s + (int64_t)W * ld_g);
+    v[3].u = *reinterpret_cast<const uint4*>(s + ((int64_t)W + 1) * ld_g);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const float2 s0 = __bfloat1622float2(v[0].h[k]), s1 = __bfloat1622float2(v[1].h[k]);
       const float2 s2 = __bfloat1622float2(v[2].h[k]), s3 = __bfloat1622float2(v[3].h[k]);
       o.h[k] = __floats2bfloat162_rn(((s0.x + s1.x) + s2.x) + s3.x, ((s0.y + s1.y) + s2.y) + s3.y);
     }
-    *reinterpret_cast<uint4*>(out + q * ld_out + c) = o.u;
+    *reinterpret_cast<uint4*>(out + (int64_t)g.q * ld_out + g.c) = o.u;
   }
 }
 
@@ -497,22 +522,20 @@ __global__ void k_upsample_backward(const bf16* __restrict__ g, int ld_g, bf16* 
 
 // x[b, y, x, :] = (resid[offs[b] + y * ld_r + x] * s_r, psf[y * ld_p + x] * s_p, 0, ..., 0)
 // as 32 channels (the network input, padded to the convolution's channel step).
-__global__ void k_pack(const float* __restrict__ resid, const int64_t* __restrict__ offs, int64_t ld_r,
-                       const float* __restrict__ psf, int64_t ld_p, float s_r, float s_p, bf16* __restrict__ x,
-                       int64_t B, int H, int W) {
-  const int64_t n = B * H * W;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int xx = (int)(i % W), yy = (int)((i / W) % H);
-    const int64_t b = i / ((int64_t)W * H);
+// Four threads a pixel, one for each 16 bytes of it.
+template <class I>
+__global__ void __launch_bounds__(256)
+    k_pack(const float* __restrict__ resid, const int64_t* __restrict__ offs, int64_t ld_r,
+           const float* __restrict__ psf, int64_t ld_p, float s_r, float s_p, bf16* __restrict__ x, I n4, int H, int W) {
+  for (I k = blockIdx.x * (I)blockDim.x + threadIdx.x; k < n4; k += (I)gridDim.x * blockDim.x) {
     V8 v;
     v.u = make_uint4(0, 0, 0, 0);
-    v.h[0] = __floats2bfloat162_rn(resid[offs[b] + yy * ld_r + xx] * s_r, psf[yy * ld_p + xx] * s_p);
-    uint4* dst = reinterpret_cast<uint4*>(x + i * 32);
-    dst[0] = v.u;
-    const uint4 z = make_uint4(0, 0, 0, 0);
-    dst[1] = z;
-    dst[2] = z;
-    dst[3] = z;
+    if ((k & 3) == 0) {
+      const I i = k >> 2, row = i / (I)W, b = row / (I)H;
+      const int64_t yy = (int64_t)(row - b * (I)H), xx = (int64_t)(i - row * (I)W);
+      v.h[0] = __floats2bfloat162_rn(resid[offs[b] + yy * ld_r + xx] * s_r, psf[yy * ld_p + xx] * s_p);
+    }
+    reinterpret_cast<uint4*>(x)[k] = v.u;
   }
 }
 
@@ -594,9 +617,15 @@ __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ 
     grad[i] = 2.0f * d * inv;
     part += d * d * inv;
   }
+  __shared__ float red[32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, part);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
+  __syncthreads();
+  if (threadIdx.x == 0) {  // one atomic per block: one per warp of the whole grid took 40 of 53 us
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) part += red[w];
+    atomicAdd(loss, part);
+  }
 }
 
 // dst[offs[b] + y * ld + x] = out[b, y, x] * scale for rows [win[4b], win[4b+1])
@@ -633,6 +662,18 @@ __global__ void k_to_bf16(const float* __restrict__ src, bf16* __restrict__ dst,
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     dst[i] = __float2bfloat16_rn(src[i]);
 }
+
+// f with n in 32 bits where every index of its kernel fits (a grid stride past
+// n, and four times n for the pixels of a 2 x 2 group), else in 64.
+template <class F>
+void with_index(int64_t n, F&& f) {
+  if (n < (1ll << 28))
+    f((uint32_t)n);
+  else
+    f((uint64_t)n);
+}
+// Blocks of a kernel that ends in atomics on a few addresses.
+unsigned few_blocks(int64_t n) { return (unsigned)std::min<int64_t>((n + 255) / 256, 4 * kSMs); }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 bool aligned4(const void* p) { return ((uintptr_t)p & 3u) == 0; }
@@ -727,8 +768,11 @@ int32_t rang_b200_nn_pool(const void* in, int64_t ld_in, void* out, int64_t ld_o
                           int32_t width, int32_t channels, void* stream) {
   if (!in || !out || batch <= 0 || height <= 0 || width <= 0 || height % 2 || width % 2 || channels % 8) return 1;
   if (ld_in % 8 || ld_out % 8 || !aligned16(in) || !aligned16(out)) return 1;
-  k_pool<<<grid_for(batch * (height / 2) * (width / 2) * (channels / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const bf16*)in, (int)ld_in, (bf16*)out, (int)ld_out, batch, height, width, channels);
+  const int64_t n = batch * (height / 2) * (width / 2) * (channels / 8);
+  with_index(n, [&](auto i) {
+    k_pool<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const bf16*)in, (int)ld_in, (bf16*)out, (int)ld_out, i,
+                                                          height / 2, width / 2, channels / 8);
+  });
   return launched();
 }
 
@@ -738,9 +782,12 @@ int32_t rang_b200_nn_pool_backward(void* grad, int64_t ld_grad, const void* dpoo
   if (!grad || !dpool || !act || batch <= 0 || height <= 0 || width <= 0 || height % 2 || width % 2 || channels % 8)
     return 1;
   if (ld_grad % 8 || ld_dpool % 8 || ld_act % 8 || !aligned16(grad) || !aligned16(dpool) || !aligned16(act)) return 1;
-  k_pool_backward<<<grid_for(batch * height * width * (channels / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (bf16*)grad, (int)ld_grad, (const bf16*)dpool, (int)ld_dpool, (const bf16*)act, (int)ld_act, batch, height, width,
-      channels);
+  const int64_t n = batch * (height / 2) * (width / 2) * (channels / 8);
+  with_index(n, [&](auto i) {
+    k_pool_backward<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((bf16*)grad, (int)ld_grad, (const bf16*)dpool,
+                                                                   (int)ld_dpool, (const bf16*)act, (int)ld_act, i,
+                                                                   height / 2, width / 2, channels / 8);
+  });
   return launched();
 }
 
@@ -748,8 +795,11 @@ int32_t rang_b200_nn_upsample(const void* in, int64_t ld_in, void* out, int64_t 
                               int32_t width, int32_t channels, void* stream) {
   if (!in || !out || batch <= 0 || height <= 0 || width <= 0 || height % 2 || width % 2 || channels % 8) return 1;
   if (ld_in % 8 || ld_out % 8 || !aligned16(in) || !aligned16(out)) return 1;
-  k_upsample<<<grid_for(batch * height * width * (channels / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const bf16*)in, (int)ld_in, (bf16*)out, (int)ld_out, batch, height, width, channels);
+  const int64_t n = batch * (height / 2) * (width / 2) * (channels / 8);
+  with_index(n, [&](auto i) {
+    k_upsample<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const bf16*)in, (int)ld_in, (bf16*)out, (int)ld_out, i,
+                                                              height / 2, width / 2, channels / 8);
+  });
   return launched();
 }
 
@@ -757,8 +807,11 @@ int32_t rang_b200_nn_upsample_backward(const void* grad, int64_t ld_grad, void* 
                                        int32_t height, int32_t width, int32_t channels, void* stream) {
   if (!grad || !out || batch <= 0 || height <= 0 || width <= 0 || channels % 8) return 1;
   if (ld_grad % 8 || ld_out % 8 || !aligned16(grad) || !aligned16(out)) return 1;
-  k_upsample_backward<<<grid_for(batch * height * width * (channels / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const bf16*)grad, (int)ld_grad, (bf16*)out, (int)ld_out, batch, height, width, channels);
+  const int64_t n = batch * height * width * (channels / 8);
+  with_index(n, [&](auto i) {
+    k_upsample_backward<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const bf16*)grad, (int)ld_grad, (bf16*)out,
+                                                                       (int)ld_out, i, height, width, channels / 8);
+  });
   return launched();
 }
 
@@ -766,8 +819,11 @@ int32_t rang_b200_nn_pack(const float* resid, const int64_t* offsets, int64_t ld
                           int64_t ld_psf, float scale_resid, float scale_psf, void* x, int64_t batch, int32_t height,
                           int32_t width, void* stream) {
   if (!resid || !offsets || !psf || !x || batch <= 0 || height <= 0 || width <= 0 || !aligned16(x)) return 1;
-  k_pack<<<grid_for(batch * height * width), 256, 0, (cudaStream_t)stream>>>(
-      resid, offsets, ld_resid, psf, ld_psf, scale_resid, scale_psf, (bf16*)x, batch, height, width);
+  const int64_t n = batch * height * width * 4;
+  with_index(n, [&](auto i) {
+    k_pack<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(resid, offsets, ld_resid, psf, ld_psf, scale_resid, scale_psf,
+                                                          (bf16*)x, i, height, width);
+  });
   return launched();
 }
 
@@ -782,7 +838,7 @@ int32_t rang_b200_nn_head_backward(const void* act, int64_t ld, const float* w, 
                                    int64_t ld_dact, float* dw, float* dbias, int64_t pixels, void* stream) {
   if (!act || !w || !dout || !dact || !dw || !dbias || pixels <= 0 || ld % 8 || ld_dact % 8) return 1;
   if (!aligned16(act) || !aligned16(dact)) return 1;
-  k_head_backward<<<grid_for(pixels), 256, 0, (cudaStream_t)stream>>>((const bf16*)act, (int)ld, w, dout, (bf16*)dact,
+  k_head_backward<<<few_blocks(pixels), 256, 0, (cudaStream_t)stream>>>((const bf16*)act, (int)ld, w, dout, (bf16*)dact,
                                                                       (int)ld_dact, dw, dbias, pixels);
   return launched();
 }
@@ -790,7 +846,7 @@ int32_t rang_b200_nn_head_backward(const void* act, int64_t ld, const float* w, 
 int32_t rang_b200_nn_mse(const float* pred, const float* target, const int64_t* offsets, int64_t ld_target,
                          float* grad, float* loss, int64_t batch, int32_t height, int32_t width, void* stream) {
   if (!pred || !target || !offsets || !grad || !loss || batch <= 0 || height <= 0 || width <= 0) return 1;
-  k_mse<<<grid_for(batch * height * width), 256, 0, (cudaStream_t)stream>>>(pred, target, offsets, ld_target, grad,
+  k_mse<<<few_blocks(batch * height * width), 256, 0, (cudaStream_t)stream>>>(pred, target, offsets, ld_target, grad,
                                                                             loss, batch, height, width);
   return launched();
 }
