@@ -628,7 +628,7 @@ __device__ __forceinline__ cplx<float> prefetched_vis(const Prefetched& p, const
 // stages its records once, one per thread.
 __host__ __device__ constexpr int i8_warps(int S) { return S >= 7 ? 2 : 1; }
 __host__ __device__ constexpr int i8_pairs(int S) { return ((S + 1) / 2 + i8_warps(S) - 1) / i8_warps(S); }
-__host__ __device__ constexpr int i8_blocks(int S) { return S <= 4 ? 16 : S <= 6 ? 12 : 9; }  // per SM
+__host__ __device__ constexpr int i8_blocks(int S) { return S <= 4 ? 16 : S <= 6 ? 12 : 8; }  // per SM
 constexpr float I8_ASCALE = 4194304.0f;  // 2^22
 // A's integers (w tap x u tap x 2^22) are formed without a conversion
 // instruction: y = x + 2^23 + 0x8080 lies in [2^23, 2^24), where FP32 spacing is
@@ -935,7 +935,7 @@ __global__ void __launch_bounds__(32 * i8_warps(S), i8_blocks(S))
 
 constexpr int H16_BATCH = 32;
 constexpr float H16_BSCALE = 16384.0f;  // 2^14: v taps stay clear of FP16 subnormals
-constexpr int h16_blocks(int S) { return S <= 6 ? 24 : 12; }  // one-warp blocks per SM
+constexpr int h16_blocks(int S) { return S <= 6 ? 24 : 16; }  // one-warp blocks per SM
 constexpr int H16_KU = 10;  // u taps placed on the window's 8 rows (read as float2)
 constexpr int H16_KV = 10;  // v taps * 2^14 placed on the 8 columns (read as float2)
 constexpr int H16_KW = 12;  // w taps (8, read as float4)
