@@ -5,8 +5,8 @@
 //   grid      every selected (row, channel) sample's float weight added, in
 //             double, to its half-plane cell (atomics; warps whose samples
 //             share a cell add once), and to the total
-//   finish    Briggs / uniform / natural on the host, in the reference's
-//             sequential order (the Briggs sum of squares is order-sensitive)
+//   finish    Briggs / uniform / natural per cell; the Briggs sum of squares,
+//             which is order-sensitive, on the host in the reference's order
 //   rank      the rank filter, one thread per cell, same window loop order
 //   lookup    each sample's cell value as a float
 //   sums      the header sums (visibility weight sum, total, max, count)
@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "rang_weights.h"
@@ -54,6 +55,11 @@ __device__ __forceinline__ int64_t weight_cell(const WGeom& g, double u, double 
   return -1;
 }
 
+// i / nchan, by a 32-bit division where i fits (a 64-bit one takes four times as long).
+__device__ __forceinline__ uint64_t row_of(uint64_t i, uint32_t nchan) {
+  return (i >> 32) == 0 ? (uint64_t)((uint32_t)i / nchan) : i / nchan;
+}
+
 __device__ __forceinline__ double warp_sum_d(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -72,7 +78,7 @@ __global__ void k_weight_grid(uint64_t nrow, uint32_t nchan, const double* __res
     int64_t cell = -1;
     double w = 0.0;
     if (i < n) {
-      const uint64_t row = i / nchan, ch = i - row * nchan;
+      const uint64_t row = row_of(i, nchan), ch = i - row * nchan;
       if (selected[row]) {
         double um = uvw[3 * row], vm = uvw[3 * row + 1];
         if (vm < 0.0) {
@@ -100,6 +106,14 @@ __global__ void k_weight_grid(uint64_t nrow, uint32_t nchan, const double* __res
   }
   part = warp_sum_d(part);
   if ((threadIdx.x & 31) == 0 && part != 0.0) atomicAdd(total, part);
+}
+
+// finish (weights.rs:190-227) of each cell, s_sq from the host's sum.
+__global__ void k_weight_finish(double* __restrict__ cells, int64_t ncell, int class_, double s_sq) {
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncell; c += (int64_t)gridDim.x * blockDim.x) {
+    const double v = cells[c];
+    if (v != 0.0) cells[c] = class_ == 2 ? 1.0 / (1.0 + v * s_sq) : class_ == 1 ? 1.0 / v : 1.0;
+  }
 }
 
 // rank_filter (weights.rs:229-269): each non-zero cell above `limit` times
@@ -139,7 +153,7 @@ __global__ void k_weight_lookup(uint64_t nrow, uint32_t nchan, const double* __r
                                 const double* __restrict__ cells, float* __restrict__ out) {
   const uint64_t n = nrow * nchan;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t row = i / nchan, ch = i - row * nchan;
+    const uint64_t row = row_of(i, nchan), ch = i - row * nchan;
     float v = 0.0f;
     if (selected[row]) {
       const double lambda = wavelength[ch];
@@ -176,12 +190,25 @@ __global__ void k_weight_sums(uint64_t n, const float* __restrict__ weights, con
     largest = fmax(largest, __shfl_xor_sync(0xffffffffu, largest, o));
     count += __shfl_xor_sync(0xffffffffu, count, o);
   }
-  if ((threadIdx.x & 31) == 0) {
-    if (vsum != 0.0) atomicAdd(&out->vsum, vsum);
-    if (total != 0.0) atomicAdd(&out->total, total);
-    if (count) atomicAdd(&out->count, count);
-    // largest >= 0: its bits order as the values do.
-    atomicMax(&out->max_bits, (unsigned long long)__double_as_longlong(largest));
+  // One set of atomics per block: one per warp of the grid, all on four
+  // addresses, took most of the kernel.
+  __shared__ WeightSumsDev part[32];
+  if ((threadIdx.x & 31) == 0)
+    part[threadIdx.x >> 5] = WeightSumsDev{vsum, total, (unsigned long long)__double_as_longlong(largest), count};
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    WeightSumsDev r = part[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
+      r.vsum += part[w].vsum;
+      r.total += part[w].total;
+      // largest >= 0: its bits order as the values do.
+      r.max_bits = r.max_bits > part[w].max_bits ? r.max_bits : part[w].max_bits;
+      r.count += part[w].count;
+    }
+    if (r.vsum != 0.0) atomicAdd(&out->vsum, r.vsum);
+    if (r.total != 0.0) atomicAdd(&out->total, r.total);
+    if (r.count) atomicAdd(&out->count, r.count);
+    atomicMax(&out->max_bits, r.max_bits);
   }
 }
 
@@ -279,28 +306,25 @@ void imaging_weights(const ImagingWeightInputs& in, ImagingWeightOutputs& out, c
                                                  total.as<double>());
     check_cuda(cudaGetLastError(), "weight grid");
   }
-  // finish (weights.rs:190-227), sequentially on the host.
-  std::vector<double> host(ncell);
-  double tot = 0.0;
-  copy_to_host(host.data(), cells.get(), ncell * sizeof(double), s);
-  check_cuda(cudaMemcpyAsync(&tot, total.get(), sizeof(double), cudaMemcpyDeviceToHost, s), "copy");
-  check_cuda(cudaStreamSynchronize(s), "weight grid");
+  // finish (weights.rs:190-227): the cells come to the host only for the
+  // Briggs sum of squares, whose order matters.
+  double s_sq = 0.0;
   if (in.class_ == 2) {
+    const std::unique_ptr<double[]> host(new double[std::max<size_t>(ncell, 1)]);
+    double tot = 0.0;
+    copy_to_host(host.get(), cells.get(), ncell * sizeof(double), s);
+    check_cuda(cudaMemcpyAsync(&tot, total.get(), sizeof(double), cudaMemcpyDeviceToHost, s), "copy");
+    check_cuda(cudaStreamSynchronize(s), "weight grid");
     double avg_w = 0.0;
-    for (double v : host) avg_w += v * v;
+    for (size_t c = 0; c < ncell; c++) avg_w += host[c] * host[c];
     avg_w /= tot;
     const double numerator_sqrt = 5.0 * std::exp(-2.302585092994046 * in.robust);  // -LN_10 * robust
-    const double s_sq = numerator_sqrt * numerator_sqrt / avg_w;
-    for (double& v : host)
-      if (v != 0.0) v = 1.0 / (1.0 + v * s_sq);
-  } else if (in.class_ == 1) {
-    for (double& v : host)
-      if (v != 0.0) v = 1.0 / v;
-  } else {
-    for (double& v : host)
-      if (v != 0.0) v = 1.0;
+    s_sq = numerator_sqrt * numerator_sqrt / avg_w;
   }
-  copy_to_device(cells.get(), host.data(), ncell * sizeof(double), s);
+  if (ncell) {
+    k_weight_finish<<<grid_blocks(ncell), 256, 0, s>>>(cells.as<double>(), (int64_t)ncell, (int)in.class_, s_sq);
+    check_cuda(cudaGetLastError(), "weight finish");
+  }
   if (in.rank_filter_level >= 1.0 && ncell) {
     DevBuf filtered(ncell * sizeof(double), s);
     k_weight_rank<<<grid_blocks(ncell), 256, 0, s>>>(cells.as<double>(), filtered.as<double>(), (int64_t)gw,
@@ -322,7 +346,7 @@ void imaging_weights(const ImagingWeightInputs& in, ImagingWeightOutputs& out, c
     DevBuf ws(sizeof(WeightSumsDev), s);
     check_cuda(cudaMemsetAsync(ws.get(), 0, sizeof(WeightSumsDev), s), "memset");
     if (n) {
-      k_weight_sums<<<grid_blocks(n), 256, 0, s>>>(n, wts.as<float>(), img.as<float>(), ws.as<WeightSumsDev>());
+      k_weight_sums<<<std::min(grid_blocks(n), 148u * 8u), 256, 0, s>>>(n, wts.as<float>(), img.as<float>(), ws.as<WeightSumsDev>());
       check_cuda(cudaGetLastError(), "weight sums");
     }
     WeightSumsDev r{};
