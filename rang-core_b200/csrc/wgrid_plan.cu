@@ -2287,6 +2287,20 @@ size_t cached_free_bytes(int dev) {
   return t;
 }
 
+// Whether the cache of the current device holds a buffer of each of these
+// sizes (those too small to be cached aside).
+static bool cache_holds(std::initializer_list<size_t> sizes) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lock(g_cache_mu);
+  for (size_t n : sizes) {
+    if (n < CACHED_MIN) continue;
+    if (std::none_of(g_cache.begin(), g_cache.end(), [&](const CachedBuf& b) { return b.dev == dev && b.bytes == n; }))
+      return false;
+  }
+  return true;
+}
+
 void flush_cache(int dev) {
   std::vector<CachedBuf> out;
   {
@@ -2720,13 +2734,19 @@ void Plan<T>::corrections(cudaStream_t s) {
 
 // Planes that fit at once: each takes `plane_bytes` (its grid and its image
 // columns, transposed); `fixed` bytes more are needed whatever the group.
-// Without `ask`, work spaces of at most 64 MB are taken to fit (the question
-// takes the driver 0.1 ms, a tenth of a small call); a caller whose allocation
-// then fails asks.
+// Without `ask`, all planes are taken to fit where their work space is at
+// most 64 MB, or within the budget's cap and its large buffers (`whole`, the
+// sizes for all planes) lie in this library's cache from an earlier pass: the
+// question takes the driver 0.1 ms on a good day and milliseconds while other
+// processes keep it busy. A caller whose allocation then fails asks.
 template <class T>
-size_t Plan<T>::plane_group(size_t plane_bytes, size_t fixed, bool ask) const {
+size_t Plan<T>::plane_group(size_t plane_bytes, size_t fixed, bool ask, std::initializer_list<size_t> whole) const {
   size_t nplanes = (size_t)std::max(g_.nplanes, 1);
-  if (!ask && nplanes * plane_bytes + fixed <= ((size_t)64 << 20)) return nplanes;
+  if (!ask) {
+    const size_t need = nplanes * plane_bytes + fixed;
+    if (need <= ((size_t)64 << 20)) return nplanes;
+    if (need <= ((size_t)64 << 30) && whole.size() && cache_holds(whole)) return nplanes;
+  }
   size_t freeb = 0, total = 0;
   check_cuda(cudaMemGetInfo(&freeb, &total), "memory info");
   auto group_of = [&](size_t avail) {
@@ -2780,7 +2800,8 @@ void Plan<T>::grid_sizes(size_t& plane_bytes, size_t& fixed, size_t& group, bool
   const size_t tplane = (size_t)g_.ny * g_.nu;
   plane_bytes = plane * sizeof(FixCell) + tplane * sizeof(cplx<T>);
   fixed = plane * sizeof(cplx<T>) + npix * sizeof(T);
-  group = plane_group(plane_bytes, fixed, ask);
+  const size_t n = (size_t)std::max(g_.nplanes, 1);
+  group = plane_group(plane_bytes, fixed, ask, {n * plane * sizeof(FixCell), n * tplane * sizeof(cplx<T>)});
 }
 
 template <class T>
@@ -3064,7 +3085,7 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
   DevBuf grids, img, cols;
   bool batched = false;
   auto take = [&](bool ask) {
-    group = plane_group(plane * cell, tplane * cell + npix * sizeof(T), ask);
+    group = plane_group(plane * cell, tplane * cell + npix * sizeof(T), ask, {nplanes * plane * cell});
     batched = batch_planes((int)group, plane, tplane, cell);
     grids.alloc(group * plane * cell, s);
     img.alloc(npix * sizeof(T), s);

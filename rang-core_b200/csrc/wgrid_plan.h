@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <string>
 #include <utility>
 #include <vector>
@@ -186,7 +187,8 @@ class Plan {
   void grid_sizes(size_t& plane_bytes, size_t& fixed, size_t& group, bool ask = false) const;
   void corrections(cudaStream_t s);
   int touched_rows(double umax, double wmax) const;
-  size_t plane_group(size_t plane_bytes, size_t fixed, bool ask = false) const;
+  size_t plane_group(size_t plane_bytes, size_t fixed, bool ask = false,
+                     std::initializer_list<size_t> whole = {}) const;
 
   WgridderOptions o_;
   size_t nrow_, nchan_, n_;
