@@ -219,11 +219,12 @@ bool scan_vectors(const Inputs& in, bool with_vis) {
          (in.wgt_kind == WGT_NONE || (al(in.wgt, 16) && al(in.wgt2, 16))) && al(in.mask, 4);
 }
 
-// Groups of four visibilities each lane has in flight (half as many in
-// double precision, whose values take twice the registers): at four blocks
-// per SM that is 72 bytes per lane, 73 KB per SM, of complex64 values and
-// mask in flight; more groups spill.
-constexpr int SCAN_GROUPS = 2;
+// Groups of four visibilities each lane has in flight: two of complex64 values
+// (at four blocks per SM 72 bytes per lane, 73 KB per SM, with the mask; more
+// spill), four of weights alone, eight of the mask alone, whose groups are four
+// bytes a lane; half as many in double precision, whose values take twice the
+// registers.
+__host__ __device__ constexpr int scan_groups(int vis, bool wgt, bool single) { return (vis ? 2 : wgt ? 4 : 8) / (single ? 1 : 2); }
 
 // scan (wgridder.rs:1051-1077): the count is exact and min/max are order
 // independent, so the result is the reference's bit for bit. A warp takes
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(256, 4) k_scan(uint32_t nrow, uint32_t nchan, 
                        const double* __restrict__ foc, double fw, Inputs in, int vec, int clean,
                        ScanOut* out, uint32_t* __restrict__ bits) {
   const uint64_t n = (uint64_t)nrow * nchan;
-  constexpr int G = sizeof(T) == 4 ? SCAN_GROUPS : SCAN_GROUPS / 2;
+  constexpr int G = scan_groups(VIS, WGT, sizeof(T) == 4);
   constexpr uint64_t BLOCK = 128ull * G;
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t wid = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
