@@ -18,6 +18,13 @@
 // weights, and keeps all nine taps' weights in shared memory for its whole
 // life where they fit, else streams three taps a step.
 //
+// With resident weights the patches also share boxes: `s` patches (2 or 4) take
+// every s-th column of 8 s columns, so that patch c's shift dx is the box of the
+// columns c + dx - 1, c + dx - 1 + s, ..., which patch c + 1 reads at shift
+// dx - 1. s + 2 boxes of a step serve the 3 s shifts (a 5-D map splits the
+// columns by their remainder): a layer of 32 channels over 81 images of 256^2
+// took 335 us with a box per patch and shift, 222 so.
+//
 // Blocks are persistent, one per SM: warp 0 issues the TMA loads into a ring
 // of stages, warp 1 issues tcgen05.mma (kind::f16, bf16 inputs, f32
 // accumulation) and commits each stage back to the loader, and sixteen more
@@ -104,6 +111,14 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
       "[%2];" ::"r"(saddr(dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(saddr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,
+                                            int c3, int c4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], "
+      "[%2];" ::"r"(saddr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(saddr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
       : "memory");
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
@@ -202,7 +217,8 @@ struct TcConv {
 // the weights stay in shared memory, patch groups, output-channel tiles.
 struct TcConvRun {
   int mt, stages, resident, groups, nt, tiles_x, tiles_y;
-  int wide;  // the output takes 32-byte stores
+  int wide;   // the output takes 32-byte stores
+  int share;  // the patches share boxes (a group is mt patches of interleaved columns)
 };
 // Past the stages and the resident weights: full, empty, weights, accumulator
 // full and empty, done, the TMEM address, the failure flag, the bias.
@@ -227,7 +243,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int nc = a.Cin / KC;
-  const int stage_bytes = run.mt * L::A_PATCH + (run.resident ? 0 : 3 * L::B_TAP);
+  const int stage_bytes = (run.share ? run.mt + 2 : run.mt) * L::A_PATCH + (run.resident ? 0 : 3 * L::B_TAP);
+  const int nj = run.share ? nc : 3 * nc;  // steps of a patch group
   unsigned char* weights = smem + run.stages * stage_bytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(weights + (run.resident ? 9 * nc * L::B_TAP : 0));
   uint64_t* empty = full + TC_MAX_STAGES;
@@ -276,15 +293,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
     int it = 0;
     for (int g = g0; g < run.groups && !*bad; g += gstep) {
-      for (int j = 0; j < 3 * nc; j++, it++) {  // channel block cb, horizontal tap dx
-        const int s = it % run.stages, cb = j / 3, dx = j - 3 * cb;
+      for (int j = 0; j < nj; j++, it++) {  // channel block cb, horizontal tap dx
+        const int s = it % run.stages, cb = run.share ? j : j / 3, dx = run.share ? 0 : j - 3 * cb;
         if (it >= run.stages && !mbar_wait(&empty[s], ((it / run.stages) - 1) & 1)) {
           *bad = 1;
           break;
         }
         unsigned char* st = smem + s * stage_bytes;
         mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
-        for (int m = 0; m < run.mt; m++) {
+        if (run.share) {  // box b: columns x0 + b - 1 and every mt-th after it
+          const PatchAt q = patch_at(g, run.tiles_x, run.tiles_y);  // x0 in columns over mt
+          for (int b = 0; b < run.mt + 2; b++) {
+            const int i = b == 0 ? q.x0 - 1 : b <= run.mt ? q.x0 : q.x0 + 1, r = b == 0 ? run.mt - 1 : (b - 1) % run.mt;
+            tma_load_5d(st + b * L::A_PATCH, &tin, &full[s], cb * KC, i, r, q.y0 - 1, q.img);
+          }
+        }
+        for (int m = 0; m < run.mt && !run.share; m++) {
           const PatchAt q = patch_at(g * run.mt + m, run.tiles_x, run.tiles_y);
           tma_load_4d(st + m * L::A_PATCH, &tin, &full[s], cb * KC, q.x0 + dx - 1, q.y0 - 1, q.img);
         }
@@ -315,15 +339,31 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       }
       tc_fence_after();
       const uint32_t acc = tmem + (uint32_t)(ab * run.mt * BN);
-      for (int j = 0; j < 3 * nc; j++) {
-        const int cb = j / 3, dx = j - 3 * cb;
+      for (int j = 0; j < nj; j++) {
+        const int cb = run.share ? j : j / 3, dx = run.share ? 0 : j - 3 * cb;
         if (!mbar_wait(&full[s], phase)) {
           *bad = 1;
           break;
         }
         tc_fence_after();
         const uint32_t alo = desc_lo(saddr(smem + s * stage_bytes));
-        if (leader) {
+        if (leader && run.share) {
+#pragma unroll
+          for (int m = 0; m < L::MT; m++)
+            if (m < run.mt) {
+#pragma unroll
+              for (int i = 0; i < 9; i++) {  // dx, then dy: the order of the other form's sums
+                const int dx3 = i / 3, dy = i % 3;
+                const uint32_t blo = wlo + (uint32_t)((3 * dy + dx3) * nc + cb) * (L::B_TAP / 16);
+#pragma unroll
+                for (int k = 0; k < KC / 16; k++)
+                  umma(acc + (uint32_t)(m * BN),
+                       alo + (uint32_t)(((m + dx3) * L::A_PATCH + dy * TC_TW * L::ROW + 32 * k) / 16), hi,
+                       blo + (uint32_t)(2 * k), hi, idesc, (j | i | k) != 0);
+              }
+            }
+          umma_commit(&empty[s]);
+        } else if (leader) {
 #pragma unroll
           for (int dy = 0; dy < 3; dy++) {
             const uint32_t blo = run.resident ? wlo + (uint32_t)((3 * dy + dx) * nc + cb) * (L::B_TAP / 16)
@@ -362,8 +402,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       tc_fence_after();
       for (int i = set; i < run.mt * (BN / 32); i += TC_EPI_WARPS / 4) {
         const int m = i / (BN / 32), c = (i - m * (BN / 32)) * 32;
-        const PatchAt q = patch_at(g * run.mt + m, run.tiles_x, run.tiles_y);
-        const int x = q.x0 + r % TC_TW, y = q.y0 + r / TC_TW;
+        const PatchAt q = patch_at(run.share ? g : g * run.mt + m, run.tiles_x, run.tiles_y);
+        const int x = run.share ? (q.x0 + r % TC_TW) * run.mt + m : q.x0 + r % TC_TW, y = q.y0 + r / TC_TW;
         const bool in = q.img < a.batch && x < a.W && y < a.H;
         const int64_t p = in ? ((int64_t)q.img * a.H + y) * a.W + x : 0;
         float v[32];
@@ -611,6 +651,21 @@ bool nhwc_map(CUtensorMap* m, const bf16* base, int channels, int ld, int W, int
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same with the columns split by their remainder mod s (W a multiple of
+// s): dimensions (channel, column / s, column mod s, row, image), box (C, 8, 1,
+// rows, 1).
+bool nhwc_map_split(CUtensorMap* m, const bf16* base, int channels, int ld, int W, int H, int64_t batch, int C, int rows,
+                    int s) {
+  const cuuint64_t px = (cuuint64_t)ld * 2;
+  cuuint64_t dims[5] = {(cuuint64_t)channels, (cuuint64_t)(W / s), (cuuint64_t)s, (cuuint64_t)H, (cuuint64_t)batch};
+  cuuint64_t strides[4] = {px * (cuuint64_t)s, px, px * (cuuint64_t)W, px * (cuuint64_t)W * (cuuint64_t)H};
+  cuuint32_t box[5] = {(cuuint32_t)C, (cuuint32_t)TC_TW, 1, (cuuint32_t)rows, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  return encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, C == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int sm_count() {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -622,7 +677,6 @@ int launch(const TcConvArgs& a, cudaStream_t s) {
   using L = TcConv<KC, BN>;
   if (!encoder()) return 2;
   CUtensorMap tin, tw;
-  if (!nhwc_map(&tin, a.in, a.Cin, a.ld_in, a.W, a.H, a.batch, KC, TC_ROWS)) return 1;
   cuuint64_t wdims[2] = {(cuuint64_t)9 * a.Cin, (cuuint64_t)a.Cout};
   cuuint64_t wstrides[1] = {(cuuint64_t)9 * a.Cin * 2};
   cuuint32_t wbox[2] = {(cuuint32_t)KC, (cuuint32_t)BN};
@@ -646,7 +700,24 @@ int launch(const TcConvArgs& a, cudaStream_t s) {
   const int budget = TC_SMEM - TC_CONTROL - 1024;
   const int64_t wbytes = (int64_t)9 * a.Cin * BN * 2;
   run.resident = wbytes + 2 * run.mt * L::A_PATCH <= budget;
-  const int stage = run.mt * L::A_PATCH + (run.resident ? 0 : 3 * L::B_TAP);
+  // Shared boxes: s columns apart, where the weights are resident beside two
+  // stages, s divides the width, the groups (8 s columns wide) overhang it by an
+  // eighth at most and every SM has one.
+  for (int s = L::MT; s >= 2 && !run.share; s /= 2) {
+    const int tx = (a.W + TC_TW * s - 1) / (TC_TW * s);
+    const int64_t groups = a.batch * tx * run.tiles_y;
+    if (wbytes + 2 * (s + 2) * L::A_PATCH > budget || a.W % s || 8 * tx * TC_TW * s > 9 * a.W || groups * run.nt < sms)
+      continue;
+    run.share = 1;
+    run.resident = 1;
+    run.mt = s;
+    run.tiles_x = tx;
+    run.groups = (int)groups;
+  }
+  if (run.share ? !nhwc_map_split(&tin, a.in, a.Cin, a.ld_in, a.W, a.H, a.batch, KC, TC_ROWS, run.mt)
+                : !nhwc_map(&tin, a.in, a.Cin, a.ld_in, a.W, a.H, a.batch, KC, TC_ROWS))
+    return 1;
+  const int stage = (run.share ? run.mt + 2 : run.mt) * L::A_PATCH + (run.resident ? 0 : 3 * L::B_TAP);
   run.stages = (int)((budget - (run.resident ? wbytes : 0)) / stage);
   if (run.stages > TC_MAX_STAGES) run.stages = TC_MAX_STAGES;
   const int bytes = run.stages * stage + (run.resident ? (int)wbytes : 0) + TC_CONTROL + 1024;

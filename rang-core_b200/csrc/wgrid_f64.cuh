@@ -189,7 +189,11 @@ __device__ __forceinline__ void f64_flush(const Geom<double>& g, FixCell2* __res
 // reference's grid_task_body, wgridder.rs:2102-2156, on windows): each warp
 // takes `chunk` consecutive sorted visibilities, stages F64_BATCH at a time
 // (coordinates, taps and value from uvw and the data, as k_grid does) and
-// contracts each run of one bin eight records at a time.
+// contracts each run of one bin eight records at a time. It is bound by
+// latency at 12 warps per SM, which its registers allow (DMMA 25 % busy): 16.5 M
+// visibilities of support 8 took 5.7 ms while every bin flushed its whole
+// window, 3.5 with windows that move, 3.3 with the flush in a loop (unrolled it
+// outgrew the instruction cache). 8, 10 and 16 warps measured no faster.
 template <int S>
 __global__ void __launch_bounds__(F64_BATCH, F64_BLOCKS)
     k_grid_f64(const __grid_constant__ Geom<double> g, Inputs in, int mode, const double* __restrict__ uvw,
@@ -376,7 +380,8 @@ struct F64DegridSlots {
 // and along u with FMAs. Blocks of at most eight records take the 8-row MMA.
 // One thread per visibility over a tile's window in shared memory, which
 // this replaces for supports up to 8, read every cell of every footprint from
-// shared memory: 2.91 ms for 16.5 M visibilities of support 8.
+// shared memory: 2.91 ms for 16.5 M visibilities of support 8, 2.36 now (the
+// FP64 tensor pipe is busy 44 % of the time, 11 warps per SM by registers).
 template <int S>
 __global__ void __launch_bounds__(F64_BATCH, F64_BLOCKS)
     k_degrid_f64(const __grid_constant__ Geom<double> g, Inputs wts, const double* __restrict__ uvw,

@@ -306,7 +306,9 @@ __global__ void k_row_coords(uint64_t nrow, const double* __restrict__ uvw, doub
 // plan's uniform choices (w-planes, phase shift, row chunks) are template
 // arguments: tested in the loop they cost branches and reloads of the plan's
 // constants on every visibility. Three blocks per SM (at most 85 registers)
-// measured 9.20 ms per call at 1.06 G visibilities, four 9.32, five 9.61.
+// measured 9.20 ms per call at 1.06 G visibilities, four 9.32, five 9.61. It is
+// bound by issue (80 % of the slots; the conversion unit 60 %, FP64 20 %):
+// 17.5 ms for two calls became 16.1 with the phase formed once per row in turns.
 constexpr int COUNT_BLOCKS = 3;
 template <bool WPL, bool SHIFT, bool CHUNKED>
 __global__ void __launch_bounds__(256, COUNT_BLOCKS)
@@ -628,6 +630,8 @@ __device__ __forceinline__ cplx<float> prefetched_vis(const Prefetched& p, const
 // stages its records once, one per thread.
 __host__ __device__ constexpr int i8_warps(int S) { return S >= 7 ? 2 : 1; }
 __host__ __device__ constexpr int i8_pairs(int S) { return ((S + 1) / 2 + i8_warps(S) - 1) / i8_warps(S); }
+// Blocks per SM: 12 blocks (168 registers) up to support 6; 54 M visibilities at
+// support 8 took 6.18 ms at 9 blocks of two warps (registers spilt) and 6.12 at 8.
 __host__ __device__ constexpr int i8_blocks(int S) { return S <= 4 ? 16 : S <= 6 ? 12 : 8; }  // per SM
 constexpr float I8_ASCALE = 4194304.0f;  // 2^22
 // A's integers (w tap x u tap x 2^22) are formed without a conversion
@@ -810,6 +814,12 @@ __device__ __forceinline__ void block_sync() {
 // outside the run read the zero slot; runs of at most 16 take the MMAs of
 // half the depth. The next round's records and values are loaded while the
 // current round is contracted.
+//
+// It is bound by issue and by latency at 11 warps per SM (59 % of the issue
+// slots, the integer tensor pipe 21 %). 1.06 G visibilities of support 6 took
+// 31.3 ms while every bin flushed its whole window and staging ran on scalar
+// multiply-adds in blocks of 8192 records, 26.2 now; 54 M of support 8, where
+// bins are sparse and the flush's atomics were the bound, 19.6 and 6.1.
 template <int S>
 __global__ void __launch_bounds__(32 * i8_warps(S), i8_blocks(S))
     k_grid_i8(const __grid_constant__ Geom<float> g, Inputs in, int mode, const VisRecord* __restrict__ rec,
@@ -1019,7 +1029,11 @@ struct DegridOut {
 // to support 6, 24 warps per SM (80 registers) measured 4 % faster than 16 (122
 // registers) and 20 (96), and as fast as 28. The w contraction before the u
 // taps and one output lane per record (two lanes of each quad) measured 10 %
-// faster than u first and one lane writing both records.
+// faster than u first and one lane writing both records. From support 7, 16
+// (128 registers) against 12 took 5.5 ms against 6.1 at 54 M visibilities.
+// It is bound by issue (69 % of the slots, the FP16 tensor pipe 45 %). That
+// call took 12.5 ms while a warp read the whole window of every bin; 1.06 G
+// visibilities of support 6, 27.6 then and 26.3 now.
 template <int S>
 __global__ void __launch_bounds__(H16_BATCH, h16_blocks(S))
     k_degrid_h(const __grid_constant__ Geom<float> g, Inputs wts, const VisRecord* __restrict__ rec,

@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 SHAPES = [(32, 32, 1, 8, 8), (32, 32, 3, 20, 12), (96, 32, 1, 33, 17), (32, 96, 2, 18, 23), (64, 192, 1, 40, 24),
           (192, 64, 2, 17, 9), (128, 64, 5, 16, 8), (128, 384, 1, 24, 40), (384, 128, 1, 22, 16), (32, 128, 1, 15, 31),
-          (64, 32, 9, 48, 56)]
+          (64, 32, 9, 48, 56),
+          # boxes shared between interleaved patches, the last with overhang
+          (32, 32, 16, 96, 64), (64, 64, 12, 80, 48), (32, 96, 20, 64, 32), (96, 32, 10, 128, 60)]
 
 
 def _bf16(a, dev):
