@@ -58,13 +58,13 @@ WORKLOAD = "ms2dirty+dirty2ms 1.06G vis 4096^2"
 CONFIG1 = "ms2dirty 16.5M vis 1024^2"
 PROFILE_CASE = "ms2dirty+dirty2ms 132M vis 2048^2"
 # DRAM bytes (read + written) per launch of the dominant kernels, from one ncu
-# capture (dram__bytes_read.sum + dram__bytes_write.sum) of each on the
+# capture (dram__bytes_read.sum + dram__bytes_write.sum, as rate x duration) of each on the
 # 132 M-visibility profiling case, as (bytes, active visibilities of that
 # launch): a launch of another workload is scaled by its active visibilities.
 # A profiler figure, not something this script can time.
 DRAM_CAPTURE = {
-    "k_grid_i8": (7.865198e9 + 0.640229e9, 105697663),
-    "k_degrid_h": (6.992914e9 + 1.269871e9, 105697663),
+    "k_grid_i8": (6.611e9, 105697663),
+    "k_degrid_h": (7.362e9, 105697663),
 }
 METRIC = "Mvis/s ms2dirty+dirty2ms @eps=1e-5 vs FP64"
 UNIT = "Mvis/s"
