@@ -58,6 +58,31 @@ def test_windows_match_the_oracle(single, supp, n):
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("single", [True, False])
+@pytest.mark.parametrize("supp,nu,nv,nx,ny", [(4, 4, 4, 2, 2), (4, 4, 14, 2, 6), (4, 6, 4, 2, 2), (5, 6, 6, 2, 2),
+                                              (5, 8, 6, 4, 2), (6, 6, 8, 2, 4), (7, 8, 8, 4, 2), (8, 8, 10, 4, 4)])
+def test_grids_smaller_than_two_windows(single, supp, nu, nv, nx, ny):
+    """The smallest grids an explicit kernel may have: a window of 8 cells wraps
+    around them twice."""
+    n, cell = 300, 2e-3
+    rng = np.random.default_rng(supp + nu)
+    uvw = np.stack([rng.uniform(-0.5, 0.5, n) / cell, rng.uniform(-0.5, 0.5, n) / cell,
+                    rng.uniform(-40.0, 40.0, n)], axis=1) * (synth.C_LIGHT / 1e9)
+    vis = rng.standard_normal((n, 1)) + 1j * rng.standard_normal((n, 1))
+    img = rng.standard_normal((nx, ny))
+    if single:
+        vis, img = vis.astype(np.complex64), img.astype(np.float32)
+    kw = dict(uvw=uvw, freq=np.array([1e9]), pixsize_x=cell, pixsize_y=cell, epsilon=1e-3,
+              kernel=(_kernel(supp, single), nu, nv))
+    tol = 2e-5 if single else 1e-12
+    got = gridder.vis2dirty(vis=vis, npix_x=nx, npix_y=ny, **kw)
+    ref = oracle.vis2dirty(vis=vis, npix_x=nx, npix_y=ny, **kw)
+    assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+    got = gridder.dirty2vis(dirty=img, **kw)
+    ref = oracle.dirty2vis(dirty=img, **kw)
+    assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+
+
 def test_bin_offsets_past_one_level_of_tile_sums():
     """Supports of 8 on a 4096^2 grid: 33 M bins, whose offsets are scanned in
     two levels."""
