@@ -19,6 +19,8 @@ struct TcConvArgs {
 // Whether the shapes and alignments fit the kernel: channels multiples of 32,
 // pixel strides of 8, 16-byte aligned tensors (any height and width).
 bool conv3_tc_supported(const TcConvArgs& a);
+// Whether it is the faster kernel for them (patches mostly filled, or few).
+bool conv3_tc_preferred(const TcConvArgs& a);
 // Launches on s; 0, 1 (the tensor maps were refused) or 2 (launch error).
 int conv3_tc(const TcConvArgs& a, cudaStream_t s);
 // Waits for s and reads (and clears) the device flag that a block sets when
@@ -40,5 +42,6 @@ struct TcDwArgs {
 // multiples of 32, pixel strides of 8, 16-byte aligned tensors (any height and
 // width).
 bool conv3_dw_tc_supported(const TcDwArgs& a);
+bool conv3_dw_tc_preferred(const TcDwArgs& a);  // as conv3_tc_preferred
 // dw += the weight gradient on s; 0, 1 (the tensor maps were refused) or 2.
 int conv3_dw_tc(const TcDwArgs& a, cudaStream_t s);

@@ -681,7 +681,8 @@ bool aligned4(const void* p) { return ((uintptr_t)p & 3u) == 0; }
 int32_t launched() { return cudaGetLastError() == cudaSuccess ? 0 : 2; }
 
 // Which kernel rang_b200_nn_conv3 runs: 0 the tcgen05 / TMA kernel where the
-// shapes allow it, else the mma.sync kernel; 1 always the mma.sync kernel.
+// shapes allow it and it is the faster one, else the mma.sync kernel; 1 always
+// the mma.sync kernel.
 std::atomic<int> g_conv_path{0};
 
 }  // namespace
@@ -698,7 +699,7 @@ int32_t rang_b200_nn_conv3(const void* in, int64_t ld_in, const void* w, const f
   if (g_conv_path.load() == 0) {
     const TcConvArgs t{(const bf16*)in, (const bf16*)w, bias, (bf16*)out, (const bf16*)mask, batch, height, width,
                        (int)ld_in, (int)ld_out, (int)ld_mask, cin, cout, relu, accumulate};
-    if (conv3_tc_supported(t)) return conv3_tc(t, (cudaStream_t)stream);
+    if (conv3_tc_supported(t) && conv3_tc_preferred(t)) return conv3_tc(t, (cudaStream_t)stream);
   }
   ConvArgs a{(const bf16*)in, (const bf16*)w, bias, (bf16*)out, (const bf16*)mask,
              batch * height * width, height, width, (int)ld_in, (int)ld_out, (int)ld_mask, cin, cout, relu, accumulate};
@@ -719,7 +720,7 @@ int32_t rang_b200_nn_conv3_weight_grad(const void* in, int64_t ld_in, const void
   if (g_conv_path.load() == 0) {
     const TcDwArgs t{(const bf16*)in, (const bf16*)dz, dw, batch, 0, 0, height, width, (int)ld_in, (int)ld_dz,
                      cin, cout};
-    if (conv3_dw_tc_supported(t)) {
+    if (conv3_dw_tc_supported(t) && conv3_dw_tc_preferred(t)) {
       const int st = conv3_dw_tc(t, (cudaStream_t)stream);
       if (st != 0) return st;
       if (dbias)

@@ -12,6 +12,13 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(32, 32, 1, 8, 8), (32, 32, 3, 20, 12), (96, 32, 1, 33, 17), (32, 96, 2, 18, 23), (64, 192, 1, 40, 24),
           (192, 64, 2, 17, 9), (128, 64, 5, 16, 8), (128, 384, 1, 24, 40), (384, 128, 1, 22, 16), (32, 128, 1, 15, 31),
           (64, 32, 9, 48, 56),
+          # images smaller than a patch, down to one pixel, with more and fewer
+          # pixels than one block's
+          (32, 32, 1, 1, 1), (128, 64, 80, 1, 1), (64, 128, 3, 2, 2), (128, 128, 5, 4, 4), (32, 64, 2, 7, 5),
+          (96, 32, 40, 3, 8), (384, 128, 20, 2, 3),
+          # where the mma.sync kernels take over: patches counted and their filling
+          (32, 32, 511, 1, 3), (32, 32, 512, 1, 3), (128, 128, 1024, 2, 4), (64, 64, 1023, 4, 4), (64, 64, 1024, 4, 4),
+          (32, 128, 1100, 1, 2),
           # boxes shared between interleaved patches, the last with overhang
           (32, 32, 16, 96, 64), (64, 64, 12, 80, 48), (32, 96, 20, 64, 32), (96, 32, 10, 128, 60)]
 
@@ -55,3 +62,50 @@ def test_convolution_and_weight_gradient_on_any_image_size(cin, cout, B, H, W):
     assert np.abs(dw.cpu().numpy().reshape(ref.shape) - ref).max() <= 1e-5 * np.abs(ref).max()
     ref = dz.reshape(-1, cout).sum(0)
     assert np.abs(db.cpu().numpy() - ref).max() <= 1e-5 * np.abs(dz).reshape(-1, cout).sum(0).max()
+
+
+def _us(f, reps=20):
+    import torch
+
+    for _ in range(3):
+        f()
+    best = float("inf")
+    for _ in range(5):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        for _ in range(reps):
+            f()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b) / reps * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("cin,cout,B,H,W", [(128, 128, 4096, 1, 1), (384, 128, 4096, 1, 1), (128, 64, 4096, 2, 2)])
+def test_many_small_images_cost_their_pixels(cin, cout, B, H, W):
+    """Patches of 8 x 16 pixels that hold one to four: the default takes no
+    longer than the mma.sync kernels (half as long again is the noise's room;
+    all patches took 2.5 to 5 times as long)."""
+    import torch
+
+    from rang import learned
+
+    dev = torch.device("cuda", 0)
+    s = torch.cuda.current_stream().cuda_stream
+    x = torch.randn(B * H * W, cin, device=dev).bfloat16()
+    w = torch.randn(cout, 9, cin, device=dev).bfloat16()
+    b = torch.zeros(cout, device=dev)
+    out = torch.empty(B * H * W, cout, device=dev, dtype=torch.bfloat16)
+
+    def conv():
+        learned._call("conv3", x.data_ptr(), cin, w.data_ptr(), b.data_ptr(), out.data_ptr(), cout, None, 0, B, H, W,
+                      cin, cout, 1, 0, s)
+
+    lib = learned._library()
+    took = _us(conv)
+    lib.rang_b200_nn_set_conv_path(1)
+    try:
+        bare = _us(conv)
+    finally:
+        lib.rang_b200_nn_set_conv_path(0)
+    assert took <= 1.5 * bare, (took, bare)
