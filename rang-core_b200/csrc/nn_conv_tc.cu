@@ -762,6 +762,9 @@ int launch_dw(TcDwArgs a, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
+// Input channels per block: the widest tile that divides them.
+int dw_tile(int cin) { return cin % 128 == 0 ? 128 : cin % 96 == 0 ? 96 : cin % 64 == 0 ? 64 : 32; }
+
 template <int CO>
 int launch_dw_co(const TcDwArgs& a, cudaStream_t s) {
   if (a.Cin % 128 == 0) return launch_dw<CO, 64, 128>(a, s);
@@ -803,8 +806,15 @@ bool conv3_dw_tc_preferred(const TcDwArgs& a) {
 }
 
 int conv3_dw_tc(const TcDwArgs& a, cudaStream_t s) {
-  if (a.Cout % 128 == 0) return launch_dw_co<128>(a, s);
-  if (a.Cout % 64 == 0) return launch_dw_co<64>(a, s);
+  // Output channels per block: the most with which there are blocks enough (at
+  // least 4 patches each) for every SM a few times. A block ends by adding
+  // 3 x CO x BN sums to dw, most of a small call: 128 to 128 channels over 32
+  // patches 13.4 us at 128, 6.4 at 32; over 128 patches 17.3, 13.9 and 10.3 at 128,
+  // 64 and 32; over 512 28.6 and 23.4 at 128 and 64; 32 to 64 channels over 512
+  // patches 9.7 at 64, 11.1 at 32.
+  const int64_t blocks = (patch_count(a.batch, a.W, a.H) + 3) / 4 * 3 * (a.Cin / dw_tile(a.Cin)), sms = sm_count();
+  if (a.Cout % 128 == 0 && blocks * (a.Cout / 128) >= 3 * sms) return launch_dw_co<128>(a, s);
+  if (a.Cout % 64 == 0 && blocks * (a.Cout / 64) >= 2 * sms) return launch_dw_co<64>(a, s);
   return launch_dw_co<32>(a, s);
 }
 

@@ -19,6 +19,8 @@ SHAPES = [(32, 32, 1, 8, 8), (32, 32, 3, 20, 12), (96, 32, 1, 33, 17), (32, 96, 
           # where the mma.sync kernels take over: patches counted and their filling
           (32, 32, 511, 1, 3), (32, 32, 512, 1, 3), (128, 128, 1024, 2, 4), (64, 64, 1023, 4, 4), (64, 64, 1024, 4, 4),
           (32, 128, 1100, 1, 2),
+          # the weight gradient's blocks of 32, 64 and 128 output channels
+          (128, 128, 32, 16, 8), (128, 128, 130, 16, 8), (128, 128, 600, 8, 8), (32, 64, 390, 9, 8), (32, 64, 400, 9, 8),
           # boxes shared between interleaved patches, the last with overhang
           (32, 32, 16, 96, 64), (64, 64, 12, 80, 48), (32, 96, 20, 64, 32), (96, 32, 10, 128, 60)]
 
