@@ -49,8 +49,9 @@ int32_t rang_b200_nn_conv3_weight_grad(const void* in, int64_t ld_in, const void
 /* Which kernels conv3 and conv3_weight_grad run: 0 (the default) the tcgen05
  * kernels (TMA operands, TMEM accumulator) wherever the shapes and alignments
  * allow them, except for many images much smaller than their 8 x 16 patches, else
- * the mma.sync kernels; 1 always the mma.sync kernels.
- * Process-wide; returns the previous value. */
+ * the mma.sync kernels; 1 always the mma.sync kernels; 2 as 0, but
+ * no two patches of a convolution share TMA boxes (the same results bit for
+ * bit; for tests). Process-wide; returns the previous value. */
 int32_t rang_b200_nn_set_conv_path(int32_t path);
 
 /* Waits for the stream and reports whether a tcgen05 convolution gave up on

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           const PatchAt q = patch_at(g, run.tiles_x, run.tiles_y);  // x0 in columns over mt
           for (int b = 0; b < run.mt + 2; b++) {
             const int i = b == 0 ? q.x0 - 1 : b <= run.mt ? q.x0 : q.x0 + 1, r = b == 0 ? run.mt - 1 : (b - 1) % run.mt;
-            tma_load_5d(st + b * L::A_PATCH, &tin, &full[s], cb * KC, i, r, q.y0 - 1, q.img);
+            tma_load_5d(st + b * L::A_PATCH, &tin, &full[s], cb * KC, r, i, q.y0 - 1, q.img);
           }
         }
         for (int m = 0; m < run.mt && !run.share; m++) {
@@ -652,14 +652,14 @@ bool nhwc_map(CUtensorMap* m, const bf16* base, int channels, int ld, int W, int
 }
 
 // The same with the columns split by their remainder mod s (W a multiple of
-// s): dimensions (channel, column / s, column mod s, row, image), box (C, 8, 1,
-// rows, 1).
+// s): dimensions (channel, column mod s, column / s, row, image), whose strides
+// ascend, each a multiple of the one before; box (C, 1, 8, rows, 1).
 bool nhwc_map_split(CUtensorMap* m, const bf16* base, int channels, int ld, int W, int H, int64_t batch, int C, int rows,
                     int s) {
   const cuuint64_t px = (cuuint64_t)ld * 2;
-  cuuint64_t dims[5] = {(cuuint64_t)channels, (cuuint64_t)(W / s), (cuuint64_t)s, (cuuint64_t)H, (cuuint64_t)batch};
-  cuuint64_t strides[4] = {px * (cuuint64_t)s, px, px * (cuuint64_t)W, px * (cuuint64_t)W * (cuuint64_t)H};
-  cuuint32_t box[5] = {(cuuint32_t)C, (cuuint32_t)TC_TW, 1, (cuuint32_t)rows, 1};
+  cuuint64_t dims[5] = {(cuuint64_t)channels, (cuuint64_t)s, (cuuint64_t)(W / s), (cuuint64_t)H, (cuuint64_t)batch};
+  cuuint64_t strides[4] = {px, px * (cuuint64_t)s, px * (cuuint64_t)W, px * (cuuint64_t)W * (cuuint64_t)H};
+  cuuint32_t box[5] = {(cuuint32_t)C, 1, (cuuint32_t)TC_TW, (cuuint32_t)rows, 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   return encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, C == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
@@ -705,21 +705,21 @@ int launch(const TcConvArgs& a, cudaStream_t s) {
   run.resident = wbytes + 2 * run.mt * L::A_PATCH <= budget;
   // Shared boxes: s columns apart, where the weights are resident beside two
   // stages, s divides the width, the groups (8 s columns wide) overhang it by an
-  // eighth at most and every SM has one.
-  for (int s = L::MT; s >= 2 && !run.share; s /= 2) {
+  // eighth at most and every SM has one. Where the driver refuses the 5-D map each
+  // patch has its own (the same sums in the same order).
+  for (int s = L::MT; s >= 2 && a.share && !run.share; s /= 2) {
     const int tx = (a.W + TC_TW * s - 1) / (TC_TW * s);
     const int64_t groups = a.batch * tx * run.tiles_y;
     if (wbytes + 2 * (s + 2) * L::A_PATCH > budget || a.W % s || 8 * tx * TC_TW * s > 9 * a.W || groups * run.nt < sms)
       continue;
+    if (!nhwc_map_split(&tin, a.in, a.Cin, a.ld_in, a.W, a.H, a.batch, KC, TC_ROWS, s)) break;
     run.share = 1;
     run.resident = 1;
     run.mt = s;
     run.tiles_x = tx;
     run.groups = (int)groups;
   }
-  if (run.share ? !nhwc_map_split(&tin, a.in, a.Cin, a.ld_in, a.W, a.H, a.batch, KC, TC_ROWS, run.mt)
-                : !nhwc_map(&tin, a.in, a.Cin, a.ld_in, a.W, a.H, a.batch, KC, TC_ROWS))
-    return 1;
+  if (!run.share && !nhwc_map(&tin, a.in, a.Cin, a.ld_in, a.W, a.H, a.batch, KC, TC_ROWS)) return 1;
   const int stage = (run.share ? run.mt + 2 : run.mt) * L::A_PATCH + (run.resident ? 0 : 3 * L::B_TAP);
   run.stages = (int)((budget - (run.resident ? wbytes : 0)) / stage);
   if (run.stages > TC_MAX_STAGES) run.stages = TC_MAX_STAGES;

@@ -14,6 +14,7 @@ struct TcConvArgs {
   const __nv_bfloat16* mask;
   int64_t batch;
   int H, W, ld_in, ld_out, ld_mask, Cin, Cout, relu, accumulate;
+  int share;  // whether patches may share boxes
 };
 
 // Whether the shapes and alignments fit the kernel: channels multiples of 32,

@@ -682,7 +682,7 @@ int32_t launched() { return cudaGetLastError() == cudaSuccess ? 0 : 2; }
 
 // Which kernel rang_b200_nn_conv3 runs: 0 the tcgen05 / TMA kernel where the
 // shapes allow it and it is the faster one, else the mma.sync kernel; 1 always
-// the mma.sync kernel.
+// the mma.sync kernel; 2 as 0 without boxes shared between patches.
 std::atomic<int> g_conv_path{0};
 
 }  // namespace
@@ -696,9 +696,9 @@ int32_t rang_b200_nn_conv3(const void* in, int64_t ld_in, const void* w, const f
   if (cin % 32 || cout % 32 || ld_in < cin || ld_out < cout || ld_in % 8 || ld_out % 8) return 1;
   if (!aligned16(in) || !aligned16(w) || !aligned4(out) || (mask && (ld_mask % 8 || !aligned4(mask)))) return 1;
   if (ld_in > INT32_MAX || ld_out > INT32_MAX || ld_mask > INT32_MAX) return 1;
-  if (g_conv_path.load() == 0) {
+  if (const int path = g_conv_path.load(); path != 1) {
     const TcConvArgs t{(const bf16*)in, (const bf16*)w, bias, (bf16*)out, (const bf16*)mask, batch, height, width,
-                       (int)ld_in, (int)ld_out, (int)ld_mask, cin, cout, relu, accumulate};
+                       (int)ld_in, (int)ld_out, (int)ld_mask, cin, cout, relu, accumulate, path == 0};
     if (conv3_tc_supported(t) && conv3_tc_preferred(t)) return conv3_tc(t, (cudaStream_t)stream);
   }
   ConvArgs a{(const bf16*)in, (const bf16*)w, bias, (bf16*)out, (const bf16*)mask,
@@ -717,7 +717,7 @@ int32_t rang_b200_nn_conv3_weight_grad(const void* in, int64_t ld_in, const void
   if (!in || !dz || !dw || batch <= 0 || height <= 0 || width <= 0 || cin <= 0 || cout <= 0) return 1;
   if (cin % 32 || cout % 32 || ld_in < cin || ld_dz < cout || ld_in % 8 || ld_dz % 8 || cout > 512) return 1;
   if (!aligned16(in) || !aligned16(dz) || ld_in > INT32_MAX || ld_dz > INT32_MAX) return 1;
-  if (g_conv_path.load() == 0) {
+  if (g_conv_path.load() != 1) {
     const TcDwArgs t{(const bf16*)in, (const bf16*)dz, dw, batch, 0, 0, height, width, (int)ld_in, (int)ld_dz,
                      cin, cout};
     if (conv3_dw_tc_supported(t) && conv3_dw_tc_preferred(t)) {
@@ -750,7 +750,7 @@ int32_t rang_b200_nn_conv3_weight_grad(const void* in, int64_t ld_in, const void
   return launched();
 }
 
-int32_t rang_b200_nn_set_conv_path(int32_t path) { return g_conv_path.exchange(path == 1 ? 1 : 0); }
+int32_t rang_b200_nn_set_conv_path(int32_t path) { return g_conv_path.exchange(path == 1 || path == 2 ? path : 0); }
 
 int32_t rang_b200_nn_wait_probe(int64_t limit_ns, void* stream) {
   if (limit_ns < 0 || limit_ns > 10000000000ll) return 1;

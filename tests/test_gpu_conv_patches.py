@@ -22,7 +22,9 @@ SHAPES = [(32, 32, 1, 8, 8), (32, 32, 3, 20, 12), (96, 32, 1, 33, 17), (32, 96, 
           # the weight gradient's blocks of 32, 64 and 128 output channels
           (128, 128, 32, 16, 8), (128, 128, 130, 16, 8), (128, 128, 600, 8, 8), (32, 64, 390, 9, 8), (32, 64, 400, 9, 8),
           # boxes shared between interleaved patches, the last with overhang
-          (32, 32, 16, 96, 64), (64, 64, 12, 80, 48), (32, 96, 20, 64, 32), (96, 32, 10, 128, 60)]
+          (32, 32, 16, 96, 64), (64, 64, 12, 80, 48), (32, 96, 20, 64, 32), (96, 32, 10, 128, 60),
+          # one patch a block too many for one round
+          (32, 32, 162, 16, 8), (128, 128, 81, 16, 16)]
 
 
 def _bf16(a, dev):
@@ -64,6 +66,33 @@ def test_convolution_and_weight_gradient_on_any_image_size(cin, cout, B, H, W):
     assert np.abs(dw.cpu().numpy().reshape(ref.shape) - ref).max() <= 1e-5 * np.abs(ref).max()
     ref = dz.reshape(-1, cout).sum(0)
     assert np.abs(db.cpu().numpy() - ref).max() <= 1e-5 * np.abs(dz).reshape(-1, cout).sum(0).max()
+
+
+@pytest.mark.parametrize("cin,cout,B,H,W", [(32, 32, 16, 96, 64), (64, 64, 12, 80, 48), (32, 96, 20, 64, 32),
+                                            (96, 32, 10, 128, 60), (32, 32, 40, 16, 122)])
+def test_patches_that_share_boxes_give_the_same_bits(cin, cout, B, H, W):
+    import torch
+
+    from rang import learned
+
+    dev = torch.device("cuda", 0)
+    s = torch.cuda.current_stream().cuda_stream
+    x = torch.randn(B * H * W, cin, device=dev).bfloat16()
+    w = torch.randn(cout, 9, cin, device=dev).bfloat16()
+    b = torch.randn(cout, device=dev)
+    lib = learned._library()
+    out = []
+    for path in (0, 2):
+        y = torch.empty(B * H * W, cout, device=dev, dtype=torch.bfloat16)
+        lib.rang_b200_nn_set_conv_path(path)
+        try:
+            learned._call("conv3", x.data_ptr(), cin, w.data_ptr(), b.data_ptr(), y.data_ptr(), cout, None, 0, B, H, W,
+                          cin, cout, 1, 0, s)
+        finally:
+            assert lib.rang_b200_nn_set_conv_path(0) == path
+        out.append(y)
+    assert lib.rang_b200_nn_device_status(s) == 0
+    assert torch.equal(out[0], out[1])
 
 
 def _us(f, reps=20):
