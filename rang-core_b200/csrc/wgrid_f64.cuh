@@ -144,7 +144,8 @@ __device__ __forceinline__ void f64_flush(const Geom<double>& g, FixCell2* __res
                                           double* buf) {
   const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
   const int o = (gq - w.rb) & 7;  // this lane's row of the window
-  const int col = wrapped(w.sv0 + (lane >> 2), g.nv);
+  int col = w.sv0 + (lane >> 2);
+  if (col >= g.nv) col -= g.nv;
   const size_t plane = (size_t)g.nu * g.nv;
   // This lane's word of a cell: the low or high part of re or im.
   unsigned long long* base =
@@ -177,10 +178,7 @@ __device__ __forceinline__ void f64_flush(const Geom<double>& g, FixCell2* __res
         const long long v = __double2ll_rn((lane & 1) ? h : (y - h) * 4294967296.0);
         if (v != 0) atomicAdd(cell, (unsigned long long)v);
         cell += (size_t)g.nv * 4;
-        if (--wrap == 0) {
-          cell -= plane * 4;
-          wrap = g.nu;
-        }
+        if (--wrap == 0) cell -= plane * 4;
       }
     }
     __syncwarp();
@@ -481,8 +479,11 @@ __global__ void __launch_bounds__(F64_BATCH, F64_BLOCKS)
         win = next;
         const int o = (gq - win.rb) & 7;  // this lane's row of the window
         if (o >= 8 - enter) {
-          const int row = wrapped(win.su0 + o, g.nu);
-          const int c0 = wrapped(win.sv0 + tq, g.nv), c1 = wrapped(win.sv0 + tq + 4, g.nv);
+          int row = win.su0 + o;
+          if (row >= g.nu) row -= g.nu;
+          int c0 = win.sv0 + tq, c1 = c0 + 4;
+          if (c0 >= g.nv) c0 -= g.nv;
+          if (c1 >= g.nv) c1 -= g.nv;
 #pragma unroll
           for (int p = 0; p < S; p++) {
             const int pp = win.mp + p;

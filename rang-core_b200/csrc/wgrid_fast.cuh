@@ -491,14 +491,6 @@ __device__ __forceinline__ void window_of(const Geom<T>& g, uint32_t key, uint32
               (uint32_t)g.nv);
 }
 
-// A window's row or column on the grid, i taken from its first one (i < n + 8).
-// The smallest grids (make_geom: twice half the support, from 4) are smaller
-// than a window, which then wraps twice.
-__device__ __forceinline__ int wrapped(int i, int n) {
-  if (i >= n) i -= n;
-  return i >= n ? i - n : i;
-}
-
 // A warp's window as it moves from bin to bin of the sorted order. Its rows
 // sit at u mod 8 (on the shifted indices), so that the next bin of the same
 // strip, a few rows further along u, keeps every row the two windows share in
@@ -714,7 +706,8 @@ __device__ __forceinline__ void i8_flush(const Geom<float>& g, FixCell* __restri
   const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
   const int o = (gq - w.rb) & 7;  // this lane's row of the window
   const int e = lane >> 4, word = lane & 15;
-  const int col = wrapped(w.sv0 + (word >> 1), g.nv);
+  int col = w.sv0 + (word >> 1);
+  if (col >= g.nv) col -= g.nv;
   const size_t plane = (size_t)g.nu * g.nv;
 #pragma unroll
   for (int h = 0; h < NP; h++) {
@@ -735,7 +728,9 @@ __device__ __forceinline__ void i8_flush(const Geom<float>& g, FixCell* __restri
                                (word & 1);
     for (int i = 0; i < leave; i++) {
       const unsigned long long v = buf[i * 32 + lane];
-      if (ok && v) atomicAdd(base + (size_t)wrapped(w.su0 + i, g.nu) * g.nv * 2, v);
+      int row = w.su0 + i;
+      if (row >= g.nu) row -= g.nu;
+      if (ok && v) atomicAdd(base + (size_t)row * g.nv * 2, v);
     }
     __syncwarp();
   }
@@ -1137,8 +1132,11 @@ __global__ void __launch_bounds__(H16_BATCH, h16_blocks(S))
         win = next;
         const int o = (gq - win.rb) & 7;  // this lane's row of the window
         const bool mine = o >= 8 - enter;
-        const int row = wrapped(win.su0 + o, g.nu);
-        const int c0 = wrapped(win.sv0 + 2 * tq, g.nv), c1 = wrapped(win.sv0 + 2 * tq + 1, g.nv);
+        int row = win.su0 + o;
+        if (row >= g.nu) row -= g.nu;
+        int c0 = win.sv0 + 2 * tq, c1 = c0 + 1;
+        if (c0 >= g.nv) c0 -= g.nv;
+        if (c1 >= g.nv) c1 -= g.nv;
         cplx<float> v[S][2];  // [plane][column]
         float m = 0.0f;
 #pragma unroll

@@ -2849,14 +2849,14 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
   const int smem = gmax * g_.L * g_.L * (int)sizeof(FixCell);
   const double* corr = corr_.as<double>();
   const size_t nu2 = (size_t)g_.nx / 2 + 1, nv2 = (size_t)g_.ny / 2 + 1;
-  const bool integer = sizeof(T) == 4 && grid_method() == GRID_INT8;
+  const bool integer = sizeof(T) == 4 && windows() && grid_method() == GRID_INT8;
   if (data.vis_kind == VIS_SORTED && !(integer && bound))
     throw DeviceError("stored values need the integer gridder and their bound");
   const bool own_bound = !bound && !(scanned && bound_of(data, mode));
   // Row chunks arriving (`ready`) are gridded as they come when the integer
   // gridder takes all planes at once (k_spec_scale); otherwise the pass
   // waits for all of them.
-  const bool speculate = ready && integer && own_bound && nchunk_ > 1 && group >= nplanes && g_.supp <= 8;
+  const bool speculate = ready && integer && own_bound && nchunk_ > 1 && group >= nplanes;
   if (ready && !speculate)
     for (int c = 0; c < nchunk_; c++) check_cuda(cudaStreamWaitEvent(s, ready[c], 0), "wait");
   // The fixed-point scales: from the scan's value maxima when `data` is the
@@ -2939,10 +2939,12 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
             continue;
           }
         } else if constexpr (SV <= 8) {
-          launch_grid_f64<SV>(s, g_, data, (int)mode, uvw_.as<double>(), foc_.as<double>(), key_.as<uint32_t>(),
-                              sorted_.as<uint32_t>(), chunk_sorted_[c], chunk_sorted_[c + 1], (uint32_t)nbins_, fg,
-                              (int)pg0, n, fs);
-          continue;
+          if (windows()) {
+            launch_grid_f64<SV>(s, g_, data, (int)mode, uvw_.as<double>(), foc_.as<double>(), key_.as<uint32_t>(),
+                                sorted_.as<uint32_t>(), chunk_sorted_[c], chunk_sorted_[c + 1], (uint32_t)nbins_, fg,
+                                (int)pg0, n, fs);
+            continue;
+          }
         }
         launch_grid<T, SV>(smem, chunk_tasks_[c + 1] - chunk_tasks_[c], s, g_, data, (int)mode, uvw_.as<double>(),
                            foc_.as<double>(), sorted_.as<uint32_t>(), tasks_.as<Task>() + chunk_tasks_[c],
@@ -3018,7 +3020,7 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
     const size_t nb = (size_t)g_.ntu * g_.ntv * (size_t)g_.nbuckets * (size_t)g_.nsub;
     const size_t np = (size_t)std::max(g_.nplanes, 1), pl = (size_t)g_.nu * g_.nv;
     const size_t npx = (size_t)o_.nx * o_.ny, tpl = (size_t)g_.ny * g_.nu;
-    stream_bins = sizeof(T) == 4 && !fused && g_.supp <= 8 && nchunk_ > 1 &&
+    stream_bins = sizeof(T) == 4 && !fused && windows() && nchunk_ > 1 &&
                   (size_t)nchunk_ * nb < 0xffffffffull &&
                   plane_group(pl * sizeof(cplx<T>), tpl * sizeof(cplx<T>) + npx * sizeof(T)) >= np;
     if (stream_bins) {
@@ -3142,30 +3144,32 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
       for (int c = 0; c < nchunk_; c++) {  // row chunk c, final after the last plane group
         bool fast_path = false;
         if constexpr (sizeof(T) == 4 && SV <= 8) {
-          fast::DegridOut out;
-          if (fused) {
-            out = *static_cast<const fast::DegridOut*>(fused);
-            out.block0 = block0;
-            block0 += degrid_parts(g_.supp, chunk_sorted_[c + 1] - chunk_sorted_[c]);
-          } else {
-            out.vis = reinterpret_cast<cplx<float>*>(vis);
+          if (windows()) {
+            fast::DegridOut out;
+            if (fused) {
+              out = *static_cast<const fast::DegridOut*>(fused);
+              out.block0 = block0;
+              block0 += degrid_parts(g_.supp, chunk_sorted_[c + 1] - chunk_sorted_[c]);
+            } else {
+              out.vis = reinterpret_cast<cplx<float>*>(vis);
+            }
+            if (stream_bins) {  // the chunk's sorted range is on the device: at most its rows' visibilities
+              if (pg0 == 0) bin_chunk(c);
+              const uint32_t* st = starts_.as<uint32_t>() + (size_t)c * nbins_;
+              launch_degrid_h<SV>(s, g_, wts, rec_.as<fast::VisRecord>(), sorted_.as<uint32_t>(), 0,
+                                  (uint64_t)(row_begin(c + 1) - row_begin(c)) * nchan_, (uint32_t)nbins_,
+                                  reinterpret_cast<const cplx<float>*>(grids.as<cplx<T>>()), (int)pg0, n, out, first,
+                                  last, st, st + nbins_);
+            } else {
+              launch_degrid_h<SV>(s, g_, wts, rec_.as<fast::VisRecord>(), sorted_.as<uint32_t>(), chunk_sorted_[c],
+                                  chunk_sorted_[c + 1], (uint32_t)nbins_,
+                                  reinterpret_cast<const cplx<float>*>(grids.as<cplx<T>>()), (int)pg0, n, out, first,
+                                  last);
+            }
+            fast_path = true;
           }
-          if (stream_bins) {  // the chunk's sorted range is on the device: at most its rows' visibilities
-            if (pg0 == 0) bin_chunk(c);
-            const uint32_t* st = starts_.as<uint32_t>() + (size_t)c * nbins_;
-            launch_degrid_h<SV>(s, g_, wts, rec_.as<fast::VisRecord>(), sorted_.as<uint32_t>(), 0,
-                                (uint64_t)(row_begin(c + 1) - row_begin(c)) * nchan_, (uint32_t)nbins_,
-                                reinterpret_cast<const cplx<float>*>(grids.as<cplx<T>>()), (int)pg0, n, out, first,
-                                last, st, st + nbins_);
-          } else {
-            launch_degrid_h<SV>(s, g_, wts, rec_.as<fast::VisRecord>(), sorted_.as<uint32_t>(), chunk_sorted_[c],
-                                chunk_sorted_[c + 1], (uint32_t)nbins_,
-                                reinterpret_cast<const cplx<float>*>(grids.as<cplx<T>>()), (int)pg0, n, out, first,
-                                last);
-          }
-          fast_path = true;
         } else if constexpr (sizeof(T) == 8 && SV <= 8) {
-          if (!fused) {
+          if (!fused && windows()) {
             launch_degrid_f64<SV>(s, g_, wts, uvw_.as<double>(), foc_.as<double>(), key_.as<uint32_t>(),
                                   sorted_.as<uint32_t>(), chunk_sorted_[c], chunk_sorted_[c + 1], (uint32_t)nbins_,
                                   grids.as<cplx<T>>(), (int)pg0, n, reinterpret_cast<cplx<T>*>(vis), first, last);
@@ -3230,7 +3234,7 @@ __global__ void k_gather_sorted(uint64_t n, const uint32_t* __restrict__ sorted,
 
 template <class T>
 bool Plan<T>::fused_values() const {
-  return sizeof(T) == 4 && g_.supp <= 8 && grid_method() == GRID_INT8;
+  return sizeof(T) == 4 && windows() && grid_method() == GRID_INT8;
 }
 
 template <class T>

@@ -183,6 +183,12 @@ class Plan {
   // The single-precision tensor-core kernels serve the pass (the degridder
   // writes the stored values in sorted order, the integer gridder reads them).
   bool fused_values() const;
+  // Whether the window kernels take this plan: supports up to 8, on grids of at
+  // least a window's 8 rows and columns, around which a window wraps once (an
+  // explicit kernel may have a grid of 4 or 6; wrapping twice cost the degridder
+  // 5 % and the gridder 4 % everywhere). The tile kernels, which take any size,
+  // run the others.
+  bool windows() const { return g_.supp <= 8 && g_.nu >= 8 && g_.nv >= 8; }
   // Bytes of one gridding plane group and of the fixed part, and the group.
   void grid_sizes(size_t& plane_bytes, size_t& fixed, size_t& group, bool ask = false) const;
   void corrections(cudaStream_t s);

@@ -61,9 +61,9 @@ def test_windows_match_the_oracle(single, supp, n):
 @pytest.mark.parametrize("single", [True, False])
 @pytest.mark.parametrize("supp,nu,nv,nx,ny", [(4, 4, 4, 2, 2), (4, 4, 14, 2, 6), (4, 6, 4, 2, 2), (5, 6, 6, 2, 2),
                                               (5, 8, 6, 4, 2), (6, 6, 8, 2, 4), (7, 8, 8, 4, 2), (8, 8, 10, 4, 4)])
-def test_grids_smaller_than_two_windows(single, supp, nu, nv, nx, ny):
-    """The smallest grids an explicit kernel may have: a window of 8 cells wraps
-    around them twice."""
+def test_grids_smaller_than_a_window(single, supp, nu, nv, nx, ny):
+    """The smallest grids an explicit kernel may have, around which a window of 8
+    cells would wrap twice: the tile kernels' (with the first sizes that are not)."""
     n, cell = 300, 2e-3
     rng = np.random.default_rng(supp + nu)
     uvw = np.stack([rng.uniform(-0.5, 0.5, n) / cell, rng.uniform(-0.5, 0.5, n) / cell,
@@ -81,6 +81,27 @@ def test_grids_smaller_than_two_windows(single, supp, nu, nv, nx, ny):
     got = gridder.dirty2vis(dirty=img, **kw)
     ref = oracle.dirty2vis(dirty=img, **kw)
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("nu,nv", [(4, 6), (8, 8)])
+def test_residual_on_the_smallest_grids(nu, nv):
+    import torch
+
+    from rang import wgrid_torch
+
+    n, cell = 300, 2e-3
+    rng = np.random.default_rng(nu)
+    uvw = np.stack([rng.uniform(-0.5, 0.5, n) / cell, rng.uniform(-0.5, 0.5, n) / cell,
+                    rng.uniform(-40.0, 40.0, n)], axis=1) * (synth.C_LIGHT / 1e9)
+    vis = (rng.standard_normal((n, 1)) + 1j * rng.standard_normal((n, 1))).astype(np.complex64)
+    img = rng.standard_normal((2, 2)).astype(np.float32)
+    kw = dict(uvw=uvw, freq=np.array([1e9]), pixsize_x=cell, pixsize_y=cell, epsilon=1e-3,
+              kernel=(_kernel(4, True), nu, nv))
+    ref = oracle.vis2dirty(vis=vis - oracle.dirty2vis(dirty=img, **kw), npix_x=2, npix_y=2, **kw)
+    plan = wgrid_torch.DevicePlan(torch.from_numpy(uvw).cuda(), kw["freq"], npix_x=2, npix_y=2, pixsize_x=cell,
+                                  pixsize_y=cell, epsilon=1e-3, kernel=kw["kernel"])
+    got, _ = plan.residual(torch.from_numpy(vis).cuda(), model=torch.from_numpy(img).cuda())
+    assert np.abs(got.cpu().numpy() - ref).max() <= 2e-5 * np.abs(ref).max()
 
 
 def test_bin_offsets_past_one_level_of_tile_sums():
