@@ -1889,8 +1889,12 @@ struct FftTraits<double> {
   }
 };
 
+// A plan without a work area of its own: executions of one plan may be in
+// flight on several streams at once, so each caller brings its own (`work`
+// bytes, fft_exec).
 struct FftPlan {
   cufftHandle h = 0;
+  size_t work = 0;
   std::mutex mu;
 };
 
@@ -1911,16 +1915,21 @@ FftPlan& fft_plan(int n, int batch) {
   if (!slot) {
     auto p = std::make_unique<FftPlan>();
     int len[1] = {n};
-    check_fft(cufftPlanMany(&p->h, 1, len, nullptr, 1, n, nullptr, 1, n, FftTraits<T>::type, batch), "plan");
+    check_fft(cufftCreate(&p->h), "plan");
+    check_fft(cufftSetAutoAllocation(p->h, 0), "plan");
+    check_fft(cufftMakePlanMany(p->h, 1, len, nullptr, 1, n, nullptr, 1, n, FftTraits<T>::type, batch, &p->work),
+              "plan");
     slot = std::move(p);
   }
   return *slot;
 }
 
+// The transforms of `p` on `s`; `work` holds f.work bytes of `s` until they are done.
 template <class T>
-void fft_exec(FftPlan& f, cplx<T>* p, int dir, cudaStream_t s) {
+void fft_exec(FftPlan& f, cplx<T>* p, int dir, const DevBuf& work, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(f.mu);
   check_fft(cufftSetStream(f.h, s), "stream");
+  if (f.work) check_fft(cufftSetWorkArea(f.h, work.get()), "work area");
   check_fft(FftTraits<T>::exec(f.h, p, dir), "transform");
 }
 
@@ -1934,10 +1943,9 @@ int touched_row_count(int urows, int nu) {
 // The v transforms of the rows footprints can touch: storage rows [0, b)
 // and [nu - b, nu), b = touched_row_count (every row when b is 0).
 template <class T>
-void fft_touched_rows(cplx<T>* plane, int nu, int nv, int b, int dir, cudaStream_t s) {
-  FftPlan& f = fft_plan<T>(nv, b == 0 ? nu : b);
-  fft_exec<T>(f, plane, dir, s);
-  if (b) fft_exec<T>(f, plane + (size_t)(nu - b) * nv, dir, s);
+void fft_touched_rows(FftPlan& f, cplx<T>* plane, int nu, int nv, int b, int dir, const DevBuf& work, cudaStream_t s) {
+  fft_exec<T>(f, plane, dir, work, s);
+  if (b) fft_exec<T>(f, plane + (size_t)(nu - b) * nv, dir, work, s);
 }
 
 // Whether the transforms of n planes (their cells and image columns) run as
@@ -1948,6 +1956,28 @@ void fft_touched_rows(cplx<T>* plane, int nu, int nv, int b, int dir, cudaStream
 constexpr size_t BATCH_BYTES = (size_t)64 << 20;
 bool batch_planes(int n, size_t plane, size_t tplane, size_t cell) {
   return (size_t)n * (plane + tplane) * cell <= BATCH_BYTES && (size_t)n * std::max(plane, tplane) < (1u << 30);
+}
+
+// A pass's transforms: along v, all rows of `n` planes (batched) or, n 0, of
+// the touched rows of one plane (fft_touched_rows); along u, the image columns
+// of n planes, transposed.
+template <class T>
+FftPlan& fft_rows(const Geom<T>& g, int rows, int n) {
+  return fft_plan<T>(g.nv, n ? n * g.nu : rows ? rows : g.nu);
+}
+template <class T>
+FftPlan& fft_cols(const Geom<T>& g, int n) {
+  return fft_plan<T>(g.nu, n * g.ny);
+}
+// The largest work area of a pass of `nplanes` planes, `group` at a time (the
+// last group may be smaller).
+template <class T>
+size_t fft_work_bytes(const Geom<T>& g, int rows, bool batched, size_t group, size_t nplanes) {
+  if (!batched) return std::max(fft_rows<T>(g, rows, 0).work, fft_cols<T>(g, 1).work);
+  size_t w = 0;
+  for (size_t n : {group, nplanes % group})
+    if (n) w = std::max({w, fft_rows<T>(g, rows, (int)n).work, fft_cols<T>(g, (int)n).work});
+  return w;
 }
 
 template <class T, int S>
@@ -2828,14 +2858,16 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
   const size_t plane = (size_t)g_.nu * g_.nv;
   const size_t tplane = (size_t)g_.ny * g_.nu;  // a plane's image columns, transposed
   size_t plane_bytes, fixed, group;
-  DevBuf grids, fpl, cols;  // the fixed-point planes; planes being transformed; their image columns
+  DevBuf grids, fpl, cols, fft_work;  // the fixed-point planes; planes being transformed; their image columns
   bool batched = false;
+  const int rows = touched_row_count(urows_, g_.nu);
   auto take = [&](bool ask) {
     grid_sizes(plane_bytes, fixed, group, ask);
     batched = batch_planes((int)group, plane, tplane, cell);
     grids.alloc(group * plane * sizeof(FixCell), s);
     fpl.alloc((batched ? group : 1) * plane * cell, s);
     cols.alloc(group * tplane * cell, s);
+    fft_work.alloc(fft_work_bytes<T>(g_, rows, batched, group, nplanes), s);
   };
   try {
     take(false);
@@ -2885,7 +2917,6 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
   }
   check_cuda(cudaGetLastError(), "scale");
   fast::FixScale* fs = scale_.as<fast::FixScale>();
-  const int rows = touched_row_count(urows_, g_.nu);
   for (size_t pg0 = 0; pg0 < nplanes; pg0 += group) {
     int n = (int)std::min(group, nplanes - pg0);
     zero_touched(grids.get(), sizeof(FixCell), n, g_.nu, g_.nv, rows, s);
@@ -2973,12 +3004,12 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
       check_cuda(cudaGetLastError(), "fixed point");
       StageTimer timer_(ST_FFT, s, 3);
       if (batched)
-        fft_exec<T>(fft_plan<T>(g_.nv, n * g_.nu), pl, CUFFT_INVERSE, s);
+        fft_exec<T>(fft_rows<T>(g_, rows, n), pl, CUFFT_INVERSE, fft_work, s);
       else
-        fft_touched_rows<T>(pl, g_.nu, g_.nv, rows, CUFFT_INVERSE, s);
+        fft_touched_rows<T>(fft_rows<T>(g_, rows, 0), pl, g_.nu, g_.nv, rows, CUFFT_INVERSE, fft_work, s);
       k_cols_to_t<T><<<dim3(tgrid.x, tgrid.y, (unsigned)step), tblock, 0, s>>>(g_, pl, rows, tp);
       check_cuda(cudaGetLastError(), "transpose");
-      fft_exec<T>(fft_plan<T>(g_.nu, step * g_.ny), tp, CUFFT_INVERSE, s);
+      fft_exec<T>(fft_cols<T>(g_, step), tp, CUFFT_INVERSE, fft_work, s);
     }
     bool first = pg0 == 0, last = pg0 + n >= nplanes;
     {
@@ -3085,14 +3116,16 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
   const size_t plane = (size_t)g_.nu * g_.nv;
   const size_t tplane = (size_t)g_.ny * g_.nu;  // a plane's image columns, transposed
   size_t group = 0;
-  DevBuf grids, img, cols;
+  DevBuf grids, img, cols, fft_work;
   bool batched = false;
+  const int rows = touched_row_count(urows_, g_.nu);
   auto take = [&](bool ask) {
     group = plane_group(plane * cell, tplane * cell + npix * sizeof(T), ask, {nplanes * plane * cell});
     batched = batch_planes((int)group, plane, tplane, cell);
     grids.alloc(group * plane * cell, s);
     img.alloc(npix * sizeof(T), s);
     cols.alloc((batched ? group : 1) * tplane * cell, s);
+    fft_work.alloc(fft_work_bytes<T>(g_, rows, batched, group, nplanes), s);
   };
   try {
     take(false);
@@ -3113,7 +3146,6 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
       std::max<int>(1, (int)(SMEM_WINDOW_BYTES / ((size_t)g_.L * Lp * sizeof(cplx<T>)))),
       (int)std::min<size_t>(nplanes, 64));
   const int smem = gmax * g_.L * Lp * (int)sizeof(cplx<T>);
-  const int rows = touched_row_count(urows_, g_.nu);
   const dim3 tgrid((unsigned)((g_.nu + 31) / 32), (unsigned)((g_.ny + 31) / 32)), tblock(32, 8);
   for (size_t pg0 = 0; pg0 < nplanes; pg0 += group) {
     int n = (int)std::min(group, nplanes - pg0);
@@ -3129,13 +3161,13 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
       }
       check_cuda(cudaGetLastError(), "place");
       StageTimer timer_(ST_FFT, s, 3);
-      fft_exec<T>(fft_plan<T>(g_.nu, step * g_.ny), cols.as<cplx<T>>(), CUFFT_FORWARD, s);
+      fft_exec<T>(fft_cols<T>(g_, step), cols.as<cplx<T>>(), CUFFT_FORWARD, fft_work, s);
       k_t_to_cols<T><<<dim3(tgrid.x, tgrid.y, (unsigned)step), tblock, 0, s>>>(g_, cols.as<cplx<T>>(), rows, pl);
       check_cuda(cudaGetLastError(), "transpose");
       if (batched)
-        fft_exec<T>(fft_plan<T>(g_.nv, n * g_.nu), pl, CUFFT_FORWARD, s);
+        fft_exec<T>(fft_rows<T>(g_, rows, n), pl, CUFFT_FORWARD, fft_work, s);
       else
-        fft_touched_rows<T>(pl, g_.nu, g_.nv, rows, CUFFT_FORWARD, s);
+        fft_touched_rows<T>(fft_rows<T>(g_, rows, 0), pl, g_.nu, g_.nv, rows, CUFFT_FORWARD, fft_work, s);
     }
     bool first = pg0 == 0, last = pg0 + n >= nplanes;
     auto run = [&](auto S) {

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <functional>
 #include <map>
@@ -184,8 +185,11 @@ __global__ void k_gauss_spectrum(cufftComplex* __restrict__ f, int nx, int ny, d
   }
 }
 
+// Plans without a work area of their own: calls on several streams may be in
+// flight at once, and each brings its own (`work` bytes, for either plan).
 struct LowpassPlans {
   cufftHandle fwd = 0, inv = 0;
+  size_t work = 0;
   std::mutex mu;
 };
 
@@ -196,10 +200,16 @@ LowpassPlans& lowpass_plans(int dev, int nx, int ny) {
   LowpassPlans*& p = plans[{dev, nx, ny}];
   if (!p) {
     auto* q = new LowpassPlans();
-    if (cufftPlan2d(&q->fwd, nx, ny, CUFFT_R2C) != CUFFT_SUCCESS || cufftPlan2d(&q->inv, nx, ny, CUFFT_C2R) != CUFFT_SUCCESS) {
+    size_t wf = 0, wi = 0;
+    auto make = [&](cufftHandle& h, cufftType type, size_t& w) {
+      return cufftCreate(&h) == CUFFT_SUCCESS && cufftSetAutoAllocation(h, 0) == CUFFT_SUCCESS &&
+             cufftMakePlan2d(h, nx, ny, type, &w) == CUFFT_SUCCESS;
+    };
+    if (!make(q->fwd, CUFFT_R2C, wf) || !make(q->inv, CUFFT_C2R, wi)) {
       delete q;
       throw DeviceError("cuFFT plan for the low-pass failed");
     }
+    q->work = std::max(wf, wi);
     p = q;
   }
   return *p;
@@ -274,10 +284,13 @@ int32_t rang_b200_gaussian_lowpass(size_t nx, size_t ny, const float* in, float*
     int dev = 0;
     check_cuda(cudaGetDevice(&dev), "device");
     LowpassPlans& p = lowpass_plans(dev, (int)nx, (int)ny);
-    DevBuf spec(nx * (ny / 2 + 1) * sizeof(cufftComplex), s);
+    DevBuf spec(nx * (ny / 2 + 1) * sizeof(cufftComplex), s), work(p.work, s);
     std::lock_guard<std::mutex> lock(p.mu);
     if (cufftSetStream(p.fwd, s) != CUFFT_SUCCESS || cufftSetStream(p.inv, s) != CUFFT_SUCCESS)
       throw DeviceError("cuFFT stream");
+    if (p.work && (cufftSetWorkArea(p.fwd, work.get()) != CUFFT_SUCCESS ||
+                   cufftSetWorkArea(p.inv, work.get()) != CUFFT_SUCCESS))
+      throw DeviceError("cuFFT work area");
     if (cufftExecR2C(p.fwd, const_cast<float*>(in), spec.as<cufftComplex>()) != CUFFT_SUCCESS)
       throw DeviceError("cuFFT forward transform");
     const uint64_t total = (uint64_t)nx * (ny / 2 + 1);

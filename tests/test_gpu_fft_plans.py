@@ -1,0 +1,87 @@
+"""The Fourier transforms' plans, which calls of one size share: passes in
+flight at the same time on several threads and streams (lengths with a large
+prime factor, whose transforms need a work area), against the same passes one
+after the other."""
+
+from concurrent.futures import ThreadPoolExecutor
+
+import numpy as np
+import pytest
+
+from rang import gridder, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _kernel(supp, single):
+    rows = [(abs(r[1] - 2.0), i) for i, r in enumerate(gridder.kernel_table())
+            if r[0] == supp and r[5] == 3 and r[6] == single]
+    return min(rows)[1]
+
+
+def _case(seed, n, cell, wmax, single):
+    rng = np.random.default_rng(seed)
+    uvw = np.stack([rng.uniform(-0.45, 0.45, n) / cell, rng.uniform(-0.45, 0.45, n) / cell,
+                    rng.uniform(-wmax, wmax, n)], axis=1) * (synth.C_LIGHT / 1e9)
+    vis = rng.standard_normal((n, 1)) + 1j * rng.standard_normal((n, 1))
+    return uvw, vis.astype(np.complex64) if single else vis
+
+
+@pytest.mark.parametrize("single", [True, False])
+@pytest.mark.parametrize("n", [256, 1018])  # 1018 = 2 x 509
+def test_threads_share_plans_but_not_work_areas(single, n):
+    cell, freq = 2e-4, np.array([1e9])
+    kw = dict(freq=freq, pixsize_x=cell, pixsize_y=cell, epsilon=1e-3, kernel=(_kernel(4, single), n, n))
+    cases = [_case(s, 2000, cell, 40.0, single) for s in range(6)]
+    imgs = [np.random.default_rng(s).standard_normal((n // 4 * 2, n // 4 * 2)).astype(np.float32 if single else np.float64)
+            for s in range(6)]
+
+    def both(k):
+        uvw, vis = cases[k]
+        return (gridder.vis2dirty(uvw=uvw, vis=vis, npix_x=n // 4 * 2, npix_y=n // 4 * 2, **kw),
+                gridder.dirty2vis(uvw=uvw, dirty=imgs[k], **kw))
+
+    want = [both(k) for k in range(6)]
+    with ThreadPoolExecutor(6) as pool:
+        for _ in range(4):
+            for k, (d, v) in enumerate(pool.map(both, range(6))):
+                assert np.array_equal(d, want[k][0]) and np.array_equal(v, want[k][1])
+
+
+def test_streams_share_plans_but_not_work_areas():
+    import torch
+
+    from rang import core, wgrid_torch
+    from rang.fista import gaussian_lowpass
+
+    cell, n = 2e-4, 1018
+    kw = dict(npix_x=n // 4 * 2, npix_y=n // 4 * 2, pixsize_x=cell, pixsize_y=cell, epsilon=1e-3, kernel=(_kernel(4, True), n, n))
+    plans, vis, imgs = [], [], []
+    for k in range(4):
+        uvw, v = _case(k, 20000, cell, 40.0, True)
+        plans.append(wgrid_torch.DevicePlan(torch.from_numpy(uvw).cuda(), np.array([1e9]), **kw))
+        vis.append(torch.from_numpy(v).cuda())
+        imgs.append(torch.randn(n // 4 * 2, n // 4 * 2, device="cuda"))
+    want = [(p.grid(v), p.degrid(i)) for p, v, i in zip(plans, vis, imgs)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in plans]
+    for _ in range(5):
+        got = []
+        for p, v, i, s in zip(plans, vis, imgs, streams):
+            with torch.cuda.stream(s):
+                got.append((p.grid(v), p.degrid(i)))
+        torch.cuda.synchronize()
+        for (a, b), (c, d) in zip(got, want):
+            assert torch.equal(a, c) and torch.equal(b, d)
+    low = [gaussian_lowpass(i, 3.0) for i in imgs]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        got = []
+        for i, s in zip(imgs, streams):
+            with torch.cuda.stream(s):
+                got.append(gaussian_lowpass(i, 3.0))
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, low))
+    for p in plans:
+        p.close()
+    assert core.extension().wgridder_release_cached() == 0
