@@ -199,8 +199,11 @@ void rang_b200_wgridder_plan_release_work(RangWgridPlan* plan);
  * returns them, and the pool's unused memory, to the device, and the pinned
  * host buffers that copies of pageable arrays go through (32 MB at most) to
  * the host (status 0, 2 on a CUDA error), after the work already queued that
- * uses them. */
+ * uses them. It also drops the plans of the Fourier transforms, of which the
+ * library keeps 64 at most (rang_b200_wgridder_fft_plans: how many now, on all
+ * devices), except those that a captured graph may use. */
 size_t rang_b200_wgridder_cached_bytes(void);
+size_t rang_b200_wgridder_fft_plans(void);
 int32_t rang_b200_wgridder_release_cached(void);
 /* `plan` and `gridding_footprint` (wgridder.rs:3527-3588) on HOST arrays:
  * the kernel and grid a call would choose (info, 14 doubles; the activity as

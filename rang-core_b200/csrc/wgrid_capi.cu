@@ -632,12 +632,15 @@ size_t rang_b200_wgridder_cached_bytes(void) {
   return cached_free_bytes(dev);
 }
 
+size_t rang_b200_wgridder_fft_plans(void) { return fft_plan_count(); }
+
 int32_t rang_b200_wgridder_release_cached(void) {
   return guarded([&] {
     int dev = 0;
     check_cuda(cudaGetDevice(&dev), "no CUDA device");
     flush_cache(dev);  // frees in stream order and waits for those frees
     release_host_buffers();
+    release_fft_plans(dev);
     cudaMemPool_t pool;
     check_cuda(cudaDeviceGetDefaultMemPool(&pool, dev), "memory pool");
     check_cuda(cudaMemPoolTrimTo(pool, 0), "memory pool");

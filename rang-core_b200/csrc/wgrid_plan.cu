@@ -1889,44 +1889,99 @@ struct FftTraits<double> {
   }
 };
 
+void check_fft(cufftResult r, const char* what) {
+  if (r != CUFFT_SUCCESS) throw DeviceError(std::string("cuFFT ") + what + " failed (" + std::to_string((int)r) + ")");
+}
+
 // A plan without a work area of its own: executions of one plan may be in
 // flight on several streams at once, so each caller brings its own (`work`
 // bytes, fft_exec).
 struct FftPlan {
   cufftHandle h = 0;
   size_t work = 0;
+  int dev = 0;
+  std::atomic<bool> captured{false};  // a graph may hold its kernels
   std::mutex mu;
-};
 
-void check_fft(cufftResult r, const char* what) {
-  if (r != CUFFT_SUCCESS) throw DeviceError(std::string("cuFFT ") + what + " failed (" + std::to_string((int)r) + ")");
+  ~FftPlan() {  // after the transforms in flight
+    if (!h) return;
+    int cur = dev;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
+    cudaDeviceSynchronize();
+    cufftDestroy(h);
+    if (cur != dev) cudaSetDevice(cur);
+  }
+};
+using FftPlanPtr = std::shared_ptr<FftPlan>;
+
+// The plans kept, the least recently used first: at most FFT_PLANS_MAX, and none
+// that a graph may hold is dropped. (Never destroyed: the driver may be gone
+// before static objects are.)
+constexpr size_t FFT_PLANS_MAX = 64;
+struct FftPlans {
+  struct Entry {
+    std::tuple<int, int, int, int> key;  // device, type, length, batch
+    FftPlanPtr plan;
+  };
+  std::mutex mu;
+  std::vector<Entry> entries;
+};
+FftPlans& fft_plans() {
+  static FftPlans* const p = new FftPlans;
+  return *p;
+}
+// Takes the plans out that `drop` names, to be destroyed without the lock.
+template <class F>
+std::vector<FftPlans::Entry> take_fft_plans(F&& drop) {
+  FftPlans& c = fft_plans();
+  std::vector<FftPlans::Entry> out;
+  std::lock_guard<std::mutex> lock(c.mu);
+  for (size_t i = 0; i < c.entries.size();)
+    if (!c.entries[i].plan->captured.load() && drop(c.entries[i], c.entries.size())) {
+      out.push_back(std::move(c.entries[i]));
+      c.entries.erase(c.entries.begin() + (std::ptrdiff_t)i);
+    } else {
+      i++;
+    }
+  return out;
 }
 
-// `batch` consecutive transforms of length `n`, per device, kept for the life
-// of the process (touched-row batches are rounded up to 64 so that few exist).
+// `batch` consecutive transforms of length `n` on the current device (touched-row
+// batches are rounded up to 64 rows, batches of planes by fft_planes, so that
+// few exist).
 template <class T>
-FftPlan& fft_plan(int n, int batch) {
-  static std::mutex mu;
-  static std::map<std::tuple<int, int, int>, std::unique_ptr<FftPlan>> cache;
+FftPlanPtr fft_plan(int n, int batch) {
   int dev = 0;
   check_cuda(cudaGetDevice(&dev), "device");
-  std::lock_guard<std::mutex> lock(mu);
-  auto& slot = cache[std::make_tuple(dev, n, batch)];
-  if (!slot) {
-    auto p = std::make_unique<FftPlan>();
+  const auto key = std::make_tuple(dev, (int)FftTraits<T>::type, n, batch);
+  FftPlans& c = fft_plans();
+  FftPlanPtr p;
+  {
+    std::lock_guard<std::mutex> lock(c.mu);
+    for (size_t i = c.entries.size(); i-- > 0;)
+      if (c.entries[i].key == key) {
+        std::rotate(c.entries.begin() + (std::ptrdiff_t)i, c.entries.begin() + (std::ptrdiff_t)i + 1, c.entries.end());
+        return c.entries.back().plan;
+      }
+    p = std::make_shared<FftPlan>();
+    p->dev = dev;
     int len[1] = {n};
     check_fft(cufftCreate(&p->h), "plan");
     check_fft(cufftSetAutoAllocation(p->h, 0), "plan");
     check_fft(cufftMakePlanMany(p->h, 1, len, nullptr, 1, n, nullptr, 1, n, FftTraits<T>::type, batch, &p->work),
               "plan");
-    slot = std::move(p);
+    c.entries.push_back({key, p});
   }
-  return *slot;
+  take_fft_plans([](const FftPlans::Entry&, size_t count) { return count > FFT_PLANS_MAX; });
+  return p;
 }
 
 // The transforms of `p` on `s`; `work` holds f.work bytes of `s` until they are done.
 template <class T>
 void fft_exec(FftPlan& f, cplx<T>* p, int dir, const DevBuf& work, cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone) f.captured = true;
   std::lock_guard<std::mutex> lock(f.mu);
   check_fft(cufftSetStream(f.h, s), "stream");
   if (f.work) check_fft(cufftSetWorkArea(f.h, work.get()), "work area");
@@ -1958,27 +2013,42 @@ bool batch_planes(int n, size_t plane, size_t tplane, size_t cell) {
   return (size_t)n * (plane + tplane) * cell <= BATCH_BYTES && (size_t)n * std::max(plane, tplane) < (1u << 30);
 }
 
-// A pass's transforms: along v, all rows of `n` planes (batched) or, n 0, of
-// the touched rows of one plane (fft_touched_rows); along u, the image columns
-// of n planes, transposed.
-template <class T>
-FftPlan& fft_rows(const Geom<T>& g, int rows, int n) {
-  return fft_plan<T>(g.nv, n ? n * g.nu : rows ? rows : g.nu);
+// Planes that the transforms of n planes run over: n rounded up to four sizes an
+// octave. The number of planes follows the range of w, and with plans for each
+// a snapshot of 69 k visibilities took 0.95 ms where its plane count was new and
+// 0.41 where not (medians of 26 counts from 7 to 32); 0.50 so. The planes added,
+// a quarter at most, hold no values and nothing reads them.
+int fft_planes(int n) {
+  int step = 1;
+  while (n > 8 * step) step *= 2;
+  return (n + step - 1) / step * step;
 }
+
+// A pass's transforms, kept for its length: along v, all rows of the planes of a
+// group (batched) or the touched rows of one plane (fft_touched_rows); along
+// u, the image columns, transposed, of a group or of one plane. `whole` for
+// groups of `group` planes, `rest` for the last group of fewer.
 template <class T>
-FftPlan& fft_cols(const Geom<T>& g, int n) {
-  return fft_plan<T>(g.nu, n * g.ny);
-}
-// The largest work area of a pass of `nplanes` planes, `group` at a time (the
-// last group may be smaller).
-template <class T>
-size_t fft_work_bytes(const Geom<T>& g, int rows, bool batched, size_t group, size_t nplanes) {
-  if (!batched) return std::max(fft_rows<T>(g, rows, 0).work, fft_cols<T>(g, 1).work);
-  size_t w = 0;
-  for (size_t n : {group, nplanes % group})
-    if (n) w = std::max({w, fft_rows<T>(g, rows, (int)n).work, fft_cols<T>(g, (int)n).work});
-  return w;
-}
+struct PassFfts {
+  struct Pair {
+    FftPlanPtr rows, cols;
+  };
+  Pair whole, rest;
+  size_t work = 0;  // the largest work area
+  PassFfts() = default;
+  PassFfts(const Geom<T>& g, int touched, bool batched, size_t group, size_t nplanes) {
+    auto make = [&](Pair& p, int planes) {
+      p.rows = fft_plan<T>(g.nv, batched ? fft_planes(planes) * g.nu : touched ? touched : g.nu);
+      p.cols = fft_plan<T>(g.nu, (batched ? fft_planes(planes) : 1) * g.ny);
+      work = std::max({work, p.rows->work, p.cols->work});
+    };
+    make(whole, (int)group);
+    if (batched && nplanes % group)
+      make(rest, (int)(nplanes % group));
+    else
+      rest = whole;
+  }
+};
 
 template <class T, int S>
 void launch_grid(int smem, unsigned nblocks, cudaStream_t s, const Geom<T>& g, const Inputs& in, int mode,
@@ -2309,6 +2379,15 @@ void free_cached(const CachedBuf& b, cudaStream_t s) {
   cudaFreeAsync(b.p, s);
 }
 }  // namespace
+
+size_t fft_plan_count() {
+  std::lock_guard<std::mutex> lock(fft_plans().mu);
+  return fft_plans().entries.size();
+}
+
+void release_fft_plans(int dev) {
+  take_fft_plans([dev](const FftPlans::Entry& e, size_t) { return e.plan->dev == dev; });
+}
 
 size_t cached_free_bytes(int dev) {
   std::lock_guard<std::mutex> lock(g_cache_mu);
@@ -2859,15 +2938,18 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
   const size_t tplane = (size_t)g_.ny * g_.nu;  // a plane's image columns, transposed
   size_t plane_bytes, fixed, group;
   DevBuf grids, fpl, cols, fft_work;  // the fixed-point planes; planes being transformed; their image columns
+  PassFfts<T> ffts;
   bool batched = false;
   const int rows = touched_row_count(urows_, g_.nu);
   auto take = [&](bool ask) {
     grid_sizes(plane_bytes, fixed, group, ask);
     batched = batch_planes((int)group, plane, tplane, cell);
     grids.alloc(group * plane * sizeof(FixCell), s);
-    fpl.alloc((batched ? group : 1) * plane * cell, s);
-    cols.alloc(group * tplane * cell, s);
-    fft_work.alloc(fft_work_bytes<T>(g_, rows, batched, group, nplanes), s);
+    const size_t padded = batched ? (size_t)fft_planes((int)group) : 1;
+    fpl.alloc(padded * plane * cell, s);
+    cols.alloc(std::max(group, padded) * tplane * cell, s);
+    ffts = PassFfts<T>(g_, rows, batched, group, nplanes);
+    fft_work.alloc(ffts.work, s);
   };
   try {
     take(false);
@@ -3003,13 +3085,14 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
       }
       check_cuda(cudaGetLastError(), "fixed point");
       StageTimer timer_(ST_FFT, s, 3);
+      const auto& f = n == (int)group ? ffts.whole : ffts.rest;
       if (batched)
-        fft_exec<T>(fft_rows<T>(g_, rows, n), pl, CUFFT_INVERSE, fft_work, s);
+        fft_exec<T>(*f.rows, pl, CUFFT_INVERSE, fft_work, s);
       else
-        fft_touched_rows<T>(fft_rows<T>(g_, rows, 0), pl, g_.nu, g_.nv, rows, CUFFT_INVERSE, fft_work, s);
+        fft_touched_rows<T>(*f.rows, pl, g_.nu, g_.nv, rows, CUFFT_INVERSE, fft_work, s);
       k_cols_to_t<T><<<dim3(tgrid.x, tgrid.y, (unsigned)step), tblock, 0, s>>>(g_, pl, rows, tp);
       check_cuda(cudaGetLastError(), "transpose");
-      fft_exec<T>(fft_cols<T>(g_, step), tp, CUFFT_INVERSE, fft_work, s);
+      fft_exec<T>(*f.cols, tp, CUFFT_INVERSE, fft_work, s);
     }
     bool first = pg0 == 0, last = pg0 + n >= nplanes;
     {
@@ -3117,15 +3200,18 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
   const size_t tplane = (size_t)g_.ny * g_.nu;  // a plane's image columns, transposed
   size_t group = 0;
   DevBuf grids, img, cols, fft_work;
+  PassFfts<T> ffts;
   bool batched = false;
   const int rows = touched_row_count(urows_, g_.nu);
   auto take = [&](bool ask) {
     group = plane_group(plane * cell, tplane * cell + npix * sizeof(T), ask, {nplanes * plane * cell});
     batched = batch_planes((int)group, plane, tplane, cell);
-    grids.alloc(group * plane * cell, s);
+    const size_t padded = batched ? (size_t)fft_planes((int)group) : 1;
+    grids.alloc(std::max(group, padded) * plane * cell, s);
     img.alloc(npix * sizeof(T), s);
-    cols.alloc((batched ? group : 1) * tplane * cell, s);
-    fft_work.alloc(fft_work_bytes<T>(g_, rows, batched, group, nplanes), s);
+    cols.alloc(padded * tplane * cell, s);
+    ffts = PassFfts<T>(g_, rows, batched, group, nplanes);
+    fft_work.alloc(ffts.work, s);
   };
   try {
     take(false);
@@ -3161,13 +3247,14 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
       }
       check_cuda(cudaGetLastError(), "place");
       StageTimer timer_(ST_FFT, s, 3);
-      fft_exec<T>(fft_cols<T>(g_, step), cols.as<cplx<T>>(), CUFFT_FORWARD, fft_work, s);
+      const auto& f = n == (int)group ? ffts.whole : ffts.rest;
+      fft_exec<T>(*f.cols, cols.as<cplx<T>>(), CUFFT_FORWARD, fft_work, s);
       k_t_to_cols<T><<<dim3(tgrid.x, tgrid.y, (unsigned)step), tblock, 0, s>>>(g_, cols.as<cplx<T>>(), rows, pl);
       check_cuda(cudaGetLastError(), "transpose");
       if (batched)
-        fft_exec<T>(fft_rows<T>(g_, rows, n), pl, CUFFT_FORWARD, fft_work, s);
+        fft_exec<T>(*f.rows, pl, CUFFT_FORWARD, fft_work, s);
       else
-        fft_touched_rows<T>(fft_rows<T>(g_, rows, 0), pl, g_.nu, g_.nv, rows, CUFFT_FORWARD, fft_work, s);
+        fft_touched_rows<T>(*f.rows, pl, g_.nu, g_.nv, rows, CUFFT_FORWARD, fft_work, s);
     }
     bool first = pg0 == 0, last = pg0 + n >= nplanes;
     auto run = [&](auto S) {

@@ -39,6 +39,10 @@ constexpr size_t CACHED_MIN = (size_t)64 << 20;
 size_t cached_free_bytes(int dev);
 // Returns the cached buffers of device `dev` to the pool.
 void flush_cache(int dev);
+// The Fourier transforms' plans kept, on all devices, and dropping those of `dev`
+// (but for any that a captured graph may hold).
+size_t fft_plan_count();
+void release_fft_plans(int dev);
 
 // Device memory taken from the stream-ordered pool and returned on release.
 // Buffers of CACHED_MIN bytes or more are kept on release in a cache by

@@ -1,14 +1,15 @@
 """The Fourier transforms' plans, which calls of one size share: passes in
 flight at the same time on several threads and streams (lengths with a large
 prime factor, whose transforms need a work area), against the same passes one
-after the other."""
+after the other; and how many plans calls with ever other w ranges leave."""
 
 from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
 
-from rang import gridder, synth
+import oracle
+from rang import core, gridder, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -51,7 +52,7 @@ def test_threads_share_plans_but_not_work_areas(single, n):
 def test_streams_share_plans_but_not_work_areas():
     import torch
 
-    from rang import core, wgrid_torch
+    from rang import wgrid_torch
     from rang.fista import gaussian_lowpass
 
     cell, n = 2e-4, 1018
@@ -85,3 +86,42 @@ def test_streams_share_plans_but_not_work_areas():
     for p in plans:
         p.close()
     assert core.extension().wgridder_release_cached() == 0
+
+
+@pytest.mark.parametrize("single", [True, False])
+def test_plane_counts_share_plans(single):
+    """Passes of 4 to 70 planes, whose transforms run together, over sizes rounded
+    up: each against the CPU oracle."""
+    ext = core.extension()
+    assert ext.wgridder_release_cached() == 0 and ext.wgridder_fft_plans() == 0
+    cell, n, freq = 2e-3, 32, np.array([1e9])
+    planes, sizes = set(), set()
+    tol = 2e-5 if single else 1e-12
+    for k in range(67):
+        uvw, vis = _case(k, 200, cell, 1.0, single)
+        uvw[0, 2], uvw[1, 2] = 0.0, (k + 0.5) * 480.0 * synth.C_LIGHT / 1e9
+        kw = dict(uvw=uvw, freq=freq, pixsize_x=cell, pixsize_y=cell, epsilon=1e-3, kernel=(_kernel(4, single), 64, 64))
+        got = gridder.vis2dirty(vis=vis, npix_x=n, npix_y=n, **kw)
+        ref = oracle.vis2dirty(vis=vis, npix_x=n, npix_y=n, **kw)
+        assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+        img = np.random.default_rng(k).standard_normal((n, n)).astype(np.float32 if single else np.float64)
+        got = gridder.dirty2vis(dirty=img, **kw)
+        ref = oracle.dirty2vis(dirty=img, **kw)
+        assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+        p = int(gridder.plan(vis=vis, npix_x=n, npix_y=n, single=single, **kw)["nplanes"])
+        planes.add(p)
+        step = max(1, 1 << max(0, (p - 1).bit_length() - 3))
+        sizes.add(-(-p // step) * step)
+    assert len(planes) >= 60 and min(planes) <= 5 and max(planes) >= 64
+    assert ext.wgridder_fft_plans() <= 2 * len(sizes) <= 40
+    assert ext.wgridder_release_cached() == 0 and ext.wgridder_fft_plans() == 0
+
+
+def test_plans_are_bounded():
+    ext = core.extension()
+    for k in range(40):  # two sizes a call
+        uvw, vis = _case(k, 50, 2e-3, 1.0, True)
+        gridder.vis2dirty(uvw=uvw, vis=vis, freq=np.array([1e9]), npix_x=16, npix_y=16, pixsize_x=2e-3,
+                          pixsize_y=2e-3, epsilon=1e-3, kernel=(_kernel(4, True), 32 + 2 * k, 34 + 2 * k))
+    assert 0 < ext.wgridder_fft_plans() <= 64
+    assert ext.wgridder_release_cached() == 0 and ext.wgridder_fft_plans() == 0
