@@ -278,6 +278,9 @@ int64_t rang_b200_wgridder_launch_count(void);
  * RANG_WGRIDDER_GPU_METHOD=int8|fp32|tf32x3|bf16x3 sets the initial value.
  * Other values select 3. Returns the previous method. */
 int32_t rang_b200_wgridder_set_method(int32_t method);
+/* For tests, in the calling thread: with no_pinned, no pinned buffer can be had
+ * for the copies of pageable arrays. 0 ends it. */
+void rang_b200_wgridder_test_limits(int32_t no_pinned);
 void rang_b200_wgridder_profile(int32_t on);
 int32_t rang_b200_wgridder_profile_read(int64_t* launches, double* ms, int32_t n);
 const char* rang_b200_wgridder_stage_name(int32_t index);

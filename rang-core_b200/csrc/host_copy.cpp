@@ -1,6 +1,7 @@
 #include "host_copy.h"
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -11,6 +12,11 @@
 namespace wg {
 
 void check_cuda(cudaError_t e, const char* what);
+
+TestLimits& test_limits() {
+  static thread_local TestLimits l;
+  return l;
+}
 
 namespace {
 
@@ -26,16 +32,20 @@ struct Buffer {
   int dev = -1;
 };
 
+// The buffers no copy is using (a fixed array: the worker threads that give
+// them back must not throw).
 std::mutex g_mu;
-std::vector<Buffer> g_free;
+std::array<Buffer, POOL_MAX> g_free;
+size_t g_nfree = 0;
 
-cudaError_t acquire(int dev, Buffer& b) {
+cudaError_t acquire(int dev, bool no_pinned, Buffer& b) {
+  if (no_pinned) return cudaErrorMemoryAllocation;
   {
     std::lock_guard<std::mutex> lock(g_mu);
-    for (size_t i = g_free.size(); i-- > 0;)
+    for (size_t i = g_nfree; i-- > 0;)
       if (g_free[i].dev == dev) {
         b = g_free[i];
-        g_free.erase(g_free.begin() + (std::ptrdiff_t)i);
+        g_free[i] = g_free[--g_nfree];
         return cudaSuccess;
       }
   }
@@ -62,8 +72,8 @@ void give_back(Buffer& b) {
   }
   {
     std::lock_guard<std::mutex> lock(g_mu);
-    if (g_free.size() < POOL_MAX) {
-      g_free.push_back(b);
+    if (g_nfree < POOL_MAX) {
+      g_free[g_nfree++] = b;
       return;
     }
   }
@@ -79,9 +89,10 @@ bool pageable(const void* p) {
   return a.type == cudaMemoryTypeUnregistered;
 }
 
-// One worker: takes pieces by the shared counter, two buffers in turn.
+// One worker: takes pieces by the shared counter, two buffers in turn. A piece
+// for which no buffer can be had goes as the driver copies pageable arrays.
 void work(bool to_device, unsigned char* dst, const unsigned char* src, size_t bytes, int dev, cudaStream_t s,
-          std::atomic<size_t>& next, std::atomic<int>& error) {
+          bool no_pinned, std::atomic<size_t>& next, std::atomic<int>& error) {
   auto fail = [&](cudaError_t e) {
     int none = cudaSuccess;
     if (e != cudaSuccess) error.compare_exchange_strong(none, (int)e);
@@ -89,6 +100,7 @@ void work(bool to_device, unsigned char* dst, const unsigned char* src, size_t b
   };
   if (fail(cudaSetDevice(dev))) return;
   Buffer buf[2];
+  bool plain = false;
   size_t held[2] = {0, 0}, at[2] = {0, 0};  // bytes on their way to the host, and where they go
   for (int k = 0; error.load() == cudaSuccess; k ^= 1) {
     Buffer& b = buf[k];
@@ -103,9 +115,19 @@ void work(bool to_device, unsigned char* dst, const unsigned char* src, size_t b
       continue;
     }
     const size_t n = std::min(PIECE, bytes - o);
+    if (!b.p && !plain) {
+      if (acquire(dev, no_pinned, b) != cudaSuccess) {
+        cudaGetLastError();
+        destroy(b);
+        plain = true;
+      } else if (fail(cudaEventSynchronize(b.ev))) {
+        break;
+      }
+    }
     if (!b.p) {
-      if (fail(acquire(dev, b))) break;
-      if (fail(cudaEventSynchronize(b.ev))) break;
+      if (fail(cudaMemcpyAsync(dst + o, src + o, n, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, s)))
+        break;
+      continue;
     }
     if (to_device) {
       std::memcpy(b.p, src + o, n);
@@ -115,7 +137,10 @@ void work(bool to_device, unsigned char* dst, const unsigned char* src, size_t b
       held[k] = n;
       at[k] = o;
     }
-    if (fail(cudaEventRecord(b.ev, s))) break;
+    if (fail(cudaEventRecord(b.ev, s))) {
+      cudaStreamSynchronize(s);  // the copy in flight still uses the buffer
+      break;
+    }
   }
   for (Buffer& b : buf)
     if (b.p || b.ev) give_back(b);
@@ -127,11 +152,12 @@ void staged(bool to_device, void* dst, const void* src, size_t bytes, cudaStream
   const size_t pieces = (bytes + PIECE - 1) / PIECE;
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
   const unsigned n = (unsigned)std::min<size_t>(pieces, std::min(hw, MAX_THREADS));
+  const bool no_pinned = test_limits().no_pinned;  // the calling thread's
   std::atomic<size_t> next{0};
   std::atomic<int> error{cudaSuccess};
   auto run = [&] {
-    work(to_device, static_cast<unsigned char*>(dst), static_cast<const unsigned char*>(src), bytes, dev, s, next,
-         error);
+    work(to_device, static_cast<unsigned char*>(dst), static_cast<const unsigned char*>(src), bytes, dev, s, no_pinned,
+         next, error);
   };
   std::vector<std::thread> threads;
   threads.reserve(n);
@@ -162,12 +188,15 @@ void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
 }
 
 void release_host_buffers() {
-  std::vector<Buffer> out;
+  std::array<Buffer, POOL_MAX> out;
+  size_t n;
   {
     std::lock_guard<std::mutex> lock(g_mu);
-    out.swap(g_free);
+    out = g_free;
+    n = g_nfree;
+    g_nfree = 0;
   }
-  for (Buffer& b : out) destroy(b);
+  for (size_t i = 0; i < n; i++) destroy(out[i]);
 }
 
 }  // namespace wg

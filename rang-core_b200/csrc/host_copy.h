@@ -13,9 +13,17 @@ namespace wg {
 // output included, against 55 GB/s of the link. copy_to_device returns once
 // `src` has been read, copy_to_host once `dst` is complete when the array is
 // pageable, as cudaMemcpyAsync does; pinned arrays are copied asynchronously.
-// Errors throw (check_cuda).
+// Where no pinned buffer can be had the copy is the driver's. Errors throw
+// (check_cuda).
 void copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
 void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
+// What the tests make scarce, in the calling thread
+// (rang_b200_wgridder_test_limits).
+struct TestLimits {
+  bool no_pinned = false;  // no pinned buffer can be had
+};
+TestLimits& test_limits();
 
 // Frees the pinned buffers that no copy is using.
 void release_host_buffers();

@@ -378,6 +378,7 @@ PYBIND11_MODULE(_core, m) {
     return out;
   });
   m.def("wgridder_cached_bytes", []() { return rang_b200_wgridder_cached_bytes(); });
+  m.def("wgridder_test_limits", [](int no_pinned) { rang_b200_wgridder_test_limits(no_pinned); });
   m.def("wgridder_fft_plans", []() { return rang_b200_wgridder_fft_plans(); });
   m.def("wgridder_release_cached", []() { return rang_b200_wgridder_release_cached(); });
   m.def("wgridder_plan_release_work",

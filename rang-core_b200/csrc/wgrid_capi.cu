@@ -632,6 +632,8 @@ size_t rang_b200_wgridder_cached_bytes(void) {
   return cached_free_bytes(dev);
 }
 
+void rang_b200_wgridder_test_limits(int32_t no_pinned) { test_limits().no_pinned = no_pinned != 0; }
+
 size_t rang_b200_wgridder_fft_plans(void) { return fft_plan_count(); }
 
 int32_t rang_b200_wgridder_release_cached(void) {

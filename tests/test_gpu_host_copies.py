@@ -45,3 +45,26 @@ def test_host_arrays_give_the_device_tensors_results(nvis, threads):
     assert core.extension().wgridder_release_cached() == 0
     d, y = both(0)
     assert np.array_equal(d, want_img) and np.array_equal(y, want_vis)
+
+
+def test_copies_without_pinned_buffers_are_the_drivers():
+    uvw, freq = meerkat_like(nant=24, ntime=4, nchan=1, seed=3)
+    nvis = (5 << 17) + 77
+    rows = np.resize(uvw, (nvis, 3)) * np.linspace(0.9, 1.0, nvis)[:, None]
+    rng = np.random.default_rng(1)
+    vis = (rng.standard_normal((nvis, 1)) + 1j * rng.standard_normal((nvis, 1))).astype(np.complex64)
+    img = rng.standard_normal((128, 96)).astype(np.float32)
+    kw = dict(uvw=rows, freq=freq, pixsize_x=4e-5, pixsize_y=4e-5, epsilon=1e-4)
+    ext = core.extension()
+
+    def both():
+        return gridder.vis2dirty(vis=vis, npix_x=128, npix_y=96, **kw), gridder.dirty2vis(dirty=img, **kw)
+
+    want = both()
+    assert ext.wgridder_release_cached() == 0
+    ext.wgridder_test_limits(1)
+    try:
+        got = both()
+    finally:
+        ext.wgridder_test_limits(0)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
