@@ -279,8 +279,10 @@ int64_t rang_b200_wgridder_launch_count(void);
  * Other values select 3. Returns the previous method. */
 int32_t rang_b200_wgridder_set_method(int32_t method);
 /* For tests, in the calling thread: with no_pinned, no pinned buffer can be had
- * for the copies of pageable arrays. 0 ends it. */
-void rang_b200_wgridder_test_limits(int32_t no_pinned);
+ * for the copies of pageable arrays; a pass takes at most `planes` w planes at
+ * once (0: as many as fit); the fail_work-th buffer of a pass's work space from
+ * now on cannot be had, once (0: none). All 0 ends it. */
+void rang_b200_wgridder_test_limits(int32_t no_pinned, int32_t planes, int32_t fail_work);
 void rang_b200_wgridder_profile(int32_t on);
 int32_t rang_b200_wgridder_profile_read(int64_t* launches, double* ms, int32_t n);
 const char* rang_b200_wgridder_stage_name(int32_t index);

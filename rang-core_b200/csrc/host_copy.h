@@ -22,6 +22,8 @@ void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
 // (rang_b200_wgridder_test_limits).
 struct TestLimits {
   bool no_pinned = false;  // no pinned buffer can be had
+  size_t planes = 0;       // planes in a group at most (0: as many as fit)
+  int fail_work = 0;       // the work-space buffer that cannot be had, counted from now (0: none)
 };
 TestLimits& test_limits();
 

@@ -378,7 +378,9 @@ PYBIND11_MODULE(_core, m) {
     return out;
   });
   m.def("wgridder_cached_bytes", []() { return rang_b200_wgridder_cached_bytes(); });
-  m.def("wgridder_test_limits", [](int no_pinned) { rang_b200_wgridder_test_limits(no_pinned); });
+  m.def("wgridder_test_limits", [](int no_pinned, int planes, int fail_work) {
+    rang_b200_wgridder_test_limits(no_pinned, planes, fail_work);
+  });
   m.def("wgridder_fft_plans", []() { return rang_b200_wgridder_fft_plans(); });
   m.def("wgridder_release_cached", []() { return rang_b200_wgridder_release_cached(); });
   m.def("wgridder_plan_release_work",

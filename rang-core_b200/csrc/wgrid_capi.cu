@@ -632,7 +632,9 @@ size_t rang_b200_wgridder_cached_bytes(void) {
   return cached_free_bytes(dev);
 }
 
-void rang_b200_wgridder_test_limits(int32_t no_pinned) { test_limits().no_pinned = no_pinned != 0; }
+void rang_b200_wgridder_test_limits(int32_t no_pinned, int32_t planes, int32_t fail_work) {
+  test_limits() = TestLimits{no_pinned != 0, (size_t)std::max(planes, 0), fail_work};
+}
 
 size_t rang_b200_wgridder_fft_plans(void) { return fft_plan_count(); }
 

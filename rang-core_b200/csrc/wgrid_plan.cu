@@ -37,6 +37,7 @@
 #include <tuple>
 #include <type_traits>
 
+#include "host_copy.h"
 #include "wgrid_plan.h"
 
 namespace wg {
@@ -2852,6 +2853,7 @@ void Plan<T>::corrections(cudaStream_t s) {
 template <class T>
 size_t Plan<T>::plane_group(size_t plane_bytes, size_t fixed, bool ask, std::initializer_list<size_t> whole) const {
   size_t nplanes = (size_t)std::max(g_.nplanes, 1);
+  if (const size_t most = test_limits().planes; most && most < nplanes) return most;
   if (!ask) {
     const size_t need = nplanes * plane_bytes + fixed;
     if (need <= ((size_t)64 << 20)) return nplanes;
@@ -2899,6 +2901,12 @@ void zero_touched(void* grids, size_t cell_bytes, int n, int nu, int nv, int row
   }
 }
 
+// Takes a buffer of a pass's work space (the tests make one of them fail).
+void work_alloc(DevBuf& b, size_t bytes, cudaStream_t s) {
+  if (int& n = test_limits().fail_work; n > 0 && --n == 0) throw DeviceError("device memory: none for the test");
+  b.alloc(bytes, s);
+}
+
 // A gridding pass's work space: per plane of a group its fixed-point grid and
 // its image columns (transposed), and whatever the group the floating-point
 // plane being transformed and the image accumulator.
@@ -2944,17 +2952,18 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
   auto take = [&](bool ask) {
     grid_sizes(plane_bytes, fixed, group, ask);
     batched = batch_planes((int)group, plane, tplane, cell);
-    grids.alloc(group * plane * sizeof(FixCell), s);
+    work_alloc(grids, group * plane * sizeof(FixCell), s);
     const size_t padded = batched ? (size_t)fft_planes((int)group) : 1;
-    fpl.alloc(padded * plane * cell, s);
-    cols.alloc(std::max(group, padded) * tplane * cell, s);
+    work_alloc(fpl, padded * plane * cell, s);
+    work_alloc(cols, std::max(group, padded) * tplane * cell, s);
     ffts = PassFfts<T>(g_, rows, batched, group, nplanes);
-    fft_work.alloc(ffts.work, s);
+    work_alloc(fft_work, ffts.work, s);
   };
   try {
     take(false);
   } catch (const DeviceError&) {
     cudaGetLastError();
+    for (DevBuf* b : {&grids, &fpl, &cols, &fft_work}) b->release();  // what is held counts as used
     take(true);
   }
   DevBuf acc(group < nplanes ? npix * sizeof(T) : 0, s);
@@ -3207,16 +3216,17 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
     group = plane_group(plane * cell, tplane * cell + npix * sizeof(T), ask, {nplanes * plane * cell});
     batched = batch_planes((int)group, plane, tplane, cell);
     const size_t padded = batched ? (size_t)fft_planes((int)group) : 1;
-    grids.alloc(std::max(group, padded) * plane * cell, s);
-    img.alloc(npix * sizeof(T), s);
-    cols.alloc(padded * tplane * cell, s);
+    work_alloc(grids, std::max(group, padded) * plane * cell, s);
+    work_alloc(img, npix * sizeof(T), s);
+    work_alloc(cols, padded * tplane * cell, s);
     ffts = PassFfts<T>(g_, rows, batched, group, nplanes);
-    fft_work.alloc(ffts.work, s);
+    work_alloc(fft_work, ffts.work, s);
   };
   try {
     take(false);
   } catch (const DeviceError&) {
     cudaGetLastError();
+    for (DevBuf* b : {&grids, &img, &cols, &fft_work}) b->release();  // what is held counts as used
     take(true);
   }
   const double* corr = corr_.as<double>();

@@ -62,9 +62,9 @@ def test_copies_without_pinned_buffers_are_the_drivers():
 
     want = both()
     assert ext.wgridder_release_cached() == 0
-    ext.wgridder_test_limits(1)
+    ext.wgridder_test_limits(1, 0, 0)
     try:
         got = both()
     finally:
-        ext.wgridder_test_limits(0)
+        ext.wgridder_test_limits(0, 0, 0)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
