@@ -1,8 +1,12 @@
-"""The retry after a buffer of a pass's work space could not be had."""
+"""Passes that take their w planes in several groups (as where they do not all
+fit in memory): every kernel family, direction and the fused residual against
+the CPU oracle, with footprints across the groups' edges; and the retry after a
+buffer of the work space could not be had."""
 
 import numpy as np
 import pytest
 
+import oracle
 from rang import core, gridder, synth
 
 pytestmark = pytest.mark.gpu
@@ -46,6 +50,50 @@ def _case(supp, nu, nv, single, n=3000):
     kw = dict(uvw=uvw, freq=np.array([1e9]), wgt=wgt, pixsize_x=CELL, pixsize_y=CELL, epsilon=1e-3, center_x=0.01,
               center_y=-0.02, kernel=(_kernel(supp, single), nu, nv))
     return vis, img, kw
+
+
+@pytest.mark.parametrize("chunks", [1, 3])
+@pytest.mark.parametrize("planes", [1, 2, 5])
+@pytest.mark.parametrize("single,supp,nu,nv", [(True, 4, 84, 80), (True, 7, 90, 100), (True, 8, 84, 96),
+                                               (False, 4, 84, 80), (False, 8, 90, 100), (False, 11, 96, 84)])
+def test_plane_groups_match_the_oracle(limits, monkeypatch, single, supp, nu, nv, planes, chunks):
+    monkeypatch.setenv("RANG_WGRIDDER_ROW_CHUNKS", str(chunks))
+    vis, img, kw = _case(supp, nu, nv, single)
+    total = gridder.plan(vis=vis, npix_x=NX, npix_y=NY, single=single, **kw)["nplanes"]
+    assert total > planes + supp
+    groups = -(-total // planes)
+    tol = 2e-5 if single else 1e-12  # the parity tests' bound; float64 sums of a few thousand terms
+    limits(0, planes, 0)
+    got, n = _launches(lambda: gridder.vis2dirty(vis=vis, npix_x=NX, npix_y=NY, **kw))
+    assert n["grid"] == groups * chunks
+    ref = oracle.vis2dirty(vis=vis, npix_x=NX, npix_y=NY, **kw)
+    assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+    got, n = _launches(lambda: gridder.dirty2vis(dirty=img, **kw))
+    assert n["degrid"] == groups * chunks
+    ref = oracle.dirty2vis(dirty=img, **kw)
+    assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("planes", [1, 3])
+@pytest.mark.parametrize("single,supp", [(True, 5), (True, 8), (False, 6)])
+def test_residual_in_plane_groups(limits, single, supp, planes):
+    import torch
+
+    from rang import wgrid_torch
+
+    vis, img, kw = _case(supp, 84, 90, single)
+    wgt = kw.pop("wgt")
+    bare = oracle.dirty2vis(dirty=img, **kw)
+    ref = oracle.vis2dirty(vis=(vis - bare).astype(vis.dtype), npix_x=NX, npix_y=NY, wgt=wgt, **kw)
+    misfit = (wgt.astype(np.float64) * np.abs(vis.astype(np.complex128) - bare) ** 2).sum()
+    w = torch.from_numpy(wgt).cuda()
+    plan = wgrid_torch.DevicePlan(torch.from_numpy(kw.pop("uvw")).cuda(), kw.pop("freq"), npix_x=NX, npix_y=NY, wgt=w,
+                                  single=single, **kw)
+    limits(0, planes, 0)
+    got, q = plan.residual(torch.from_numpy(vis).cuda(), w, model=torch.from_numpy(img).cuda())
+    tol = 4e-5 if single else 1e-12
+    assert np.abs(got.cpu().numpy() - ref).max() <= tol * np.abs(ref).max()
+    assert abs(float(q) - misfit) <= tol * misfit
 
 
 @pytest.mark.parametrize("buffer", [1, 2, 3])
