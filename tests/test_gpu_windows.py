@@ -49,9 +49,9 @@ def test_windows_match_the_oracle(single, supp, n):
               kernel=(_kernel(supp, single), nu, nv))
     got = gridder.vis2dirty(vis=vis, npix_x=nx, npix_y=ny, **kw)
     ref = oracle.vis2dirty(vis=vis, npix_x=nx, npix_y=ny, **kw)
-    # The parity tests' bounds: factors in 23 bits (single) or float64, random
+    # Factors in 23 bits (single: the parity tests' bound) or float64 throughout, random
     # signs, no wide-field correction at this field.
-    tol = 2e-5 if single else 1e-9
+    tol = 2e-5 if single else 1e-12
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
     got = gridder.dirty2vis(dirty=img, **kw)
     ref = oracle.dirty2vis(dirty=img, **kw)
