@@ -1978,14 +1978,14 @@ FftPlanPtr fft_plan(int n, int batch) {
   return p;
 }
 
-// The transforms of `p` on `s`; `work` holds f.work bytes of `s` until they are done.
+// The transforms of `p` on `s`; `work` holds f.work bytes until they are done.
 template <class T>
-void fft_exec(FftPlan& f, cplx<T>* p, int dir, const DevBuf& work, cudaStream_t s) {
+void fft_exec(FftPlan& f, cplx<T>* p, int dir, void* work, cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone) f.captured = true;
   std::lock_guard<std::mutex> lock(f.mu);
   check_fft(cufftSetStream(f.h, s), "stream");
-  if (f.work) check_fft(cufftSetWorkArea(f.h, work.get()), "work area");
+  if (f.work) check_fft(cufftSetWorkArea(f.h, work), "work area");
   check_fft(FftTraits<T>::exec(f.h, p, dir), "transform");
 }
 
@@ -1999,7 +1999,7 @@ int touched_row_count(int urows, int nu) {
 // The v transforms of the rows footprints can touch: storage rows [0, b)
 // and [nu - b, nu), b = touched_row_count (every row when b is 0).
 template <class T>
-void fft_touched_rows(FftPlan& f, cplx<T>* plane, int nu, int nv, int b, int dir, const DevBuf& work, cudaStream_t s) {
+void fft_touched_rows(FftPlan& f, cplx<T>* plane, int nu, int nv, int b, int dir, void* work, cudaStream_t s) {
   fft_exec<T>(f, plane, dir, work, s);
   if (b) fft_exec<T>(f, plane + (size_t)(nu - b) * nv, dir, work, s);
 }
@@ -2945,8 +2945,11 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
   const size_t plane = (size_t)g_.nu * g_.nv;
   const size_t tplane = (size_t)g_.ny * g_.nu;  // a plane's image columns, transposed
   size_t plane_bytes, fixed, group;
-  DevBuf grids, fpl, cols, fft_work;  // the fixed-point planes; planes being transformed; their image columns
+  // The fixed-point planes; planes being transformed, then the transforms' work
+  // area; their image columns.
+  DevBuf grids, fpl, cols;
   PassFfts<T> ffts;
+  void* fft_work = nullptr;
   bool batched = false;
   const int rows = touched_row_count(urows_, g_.nu);
   auto take = [&](bool ask) {
@@ -2954,16 +2957,17 @@ void Plan<T>::grid(const Inputs& data, ValueMode mode, T* image, cudaStream_t s,
     batched = batch_planes((int)group, plane, tplane, cell);
     work_alloc(grids, group * plane * sizeof(FixCell), s);
     const size_t padded = batched ? (size_t)fft_planes((int)group) : 1;
-    work_alloc(fpl, padded * plane * cell, s);
-    work_alloc(cols, std::max(group, padded) * tplane * cell, s);
     ffts = PassFfts<T>(g_, rows, batched, group, nplanes);
-    work_alloc(fft_work, ffts.work, s);
+    const size_t at = (padded * plane * cell + 255) / 256 * 256;
+    work_alloc(fpl, at + ffts.work, s);
+    fft_work = fpl.as<unsigned char>() + at;
+    work_alloc(cols, std::max(group, padded) * tplane * cell, s);
   };
   try {
     take(false);
   } catch (const DeviceError&) {
     cudaGetLastError();
-    for (DevBuf* b : {&grids, &fpl, &cols, &fft_work}) b->release();  // what is held counts as used
+    for (DevBuf* b : {&grids, &fpl, &cols}) b->release();  // what is held counts as used
     take(true);
   }
   DevBuf acc(group < nplanes ? npix * sizeof(T) : 0, s);
@@ -3208,8 +3212,9 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
   const size_t plane = (size_t)g_.nu * g_.nv;
   const size_t tplane = (size_t)g_.ny * g_.nu;  // a plane's image columns, transposed
   size_t group = 0;
-  DevBuf grids, img, cols, fft_work;
+  DevBuf grids, img, cols;  // cols: the image columns, then the transforms' work area
   PassFfts<T> ffts;
+  void* fft_work = nullptr;
   bool batched = false;
   const int rows = touched_row_count(urows_, g_.nu);
   auto take = [&](bool ask) {
@@ -3218,15 +3223,16 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
     const size_t padded = batched ? (size_t)fft_planes((int)group) : 1;
     work_alloc(grids, std::max(group, padded) * plane * cell, s);
     work_alloc(img, npix * sizeof(T), s);
-    work_alloc(cols, padded * tplane * cell, s);
     ffts = PassFfts<T>(g_, rows, batched, group, nplanes);
-    work_alloc(fft_work, ffts.work, s);
+    const size_t at = (padded * tplane * cell + 255) / 256 * 256;
+    work_alloc(cols, at + ffts.work, s);
+    fft_work = cols.as<unsigned char>() + at;
   };
   try {
     take(false);
   } catch (const DeviceError&) {
     cudaGetLastError();
-    for (DevBuf* b : {&grids, &img, &cols, &fft_work}) b->release();  // what is held counts as used
+    for (DevBuf* b : {&grids, &img, &cols}) b->release();  // what is held counts as used
     take(true);
   }
   const double* corr = corr_.as<double>();
