@@ -242,25 +242,38 @@ __device__ __forceinline__ cplx<double> cis_turns(double t, double) {
   return {c, s};
 }
 
+// The same through sincos of the rounded angle, turned by what the rounding
+// left (within 1.8e-16 where sincospi is within 1.3e-16), for the tile gridder in
+// double precision, whose few staging threads wait on this chain: 82 ms with
+// sincospi, 70 so, for 0.3 M visibilities of support 13 within 70 x 70 cells.
+__device__ __forceinline__ cplx<float> cis_turns_staged(double t, float) { return cis_turns(t, 0.0f); }
+__device__ __forceinline__ cplx<double> cis_turns_staged(double t, double) {
+  constexpr double HI = 6.283185307179586, LO = 2.4492935982947064e-16;  // 2 pi
+  const double r = t - rint(t), a = HI * r, d = fma(HI, r, -a) + LO * r;
+  double s, c;
+  sincos(a, &s, &c);
+  return {c - s * d, s + c * d};
+}
+
 template <class T>
 __device__ __forceinline__ cplx<T> cmul(cplx<T> a, cplx<T> b) {
   return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
 }
 
 // shift_phase (wgridder.rs:1395-1408) from the row's fixed coordinates.
-template <class T>
+template <class T, bool STAGED = false>
 __device__ __forceinline__ cplx<T> shift_phase(const Geom<T>& g, const double b[3], double imflip,
                                                double f_over_c, double sign) {
   double fct = sign * imflip * (b[0] * g.lshift + b[1] * g.mshift + b[2] * g.nshift);
-  return cis_turns(fct * f_over_c, (T)0);
+  return STAGED ? cis_turns_staged(fct * f_over_c, (T)0) : cis_turns(fct * f_over_c, (T)0);
 }
 
 // unit_value (wgridder.rs:1414-1424).
-template <class T>
+template <class T, bool STAGED = false>
 __device__ __forceinline__ cplx<T> unit_value(const Geom<T>& g, const double b[3], double imflip,
                                               double f_over_c, bool has_w, T w) {
   cplx<T> v{(T)1, (T)0};
-  if (g.shifting) v = cmul(v, shift_phase<T>(g, b, imflip, f_over_c, 1.0));
+  if (g.shifting) v = cmul(v, shift_phase<T, STAGED>(g, b, imflip, f_over_c, 1.0));
   if (has_w) v = {v.re * w, v.im * w};
   return {v.re, v.im * (T)imflip};
 }

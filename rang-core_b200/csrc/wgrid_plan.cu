@@ -892,7 +892,7 @@ __global__ void __launch_bounds__(GridLayout<S>::THREADS)
             const T x0 = (T)(-uf * 2.0 + ((double)S - 1.0));
             const T y0 = (T)(-vf * 2.0 + ((double)S - 1.0));
             eval_taps2<T, S>(g.coeff, g.ne, x0, y0, ku, kv);
-            cplx<T> val = unit_value<T>(g, b, imflip, f, in.wgt_kind != WGT_NONE, wgt_get<T>(in, idx));
+            cplx<T> val = unit_value<T, true>(g, b, imflip, f, in.wgt_kind != WGT_NONE, wgt_get<T>(in, idx));
             if (mode == VALUE_DATA) val = data_value<T>(vis_get<T>(in, idx), val, (T)imflip);
 #pragma unroll
             for (int j = 0; j < S; j++) {

@@ -58,6 +58,27 @@ def test_windows_match_the_oracle(single, supp, n):
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("supp", [9, 13, 16])
+def test_wider_supports_far_from_the_centre(supp):
+    """The tile kernels' phases: a field off the centre and long baselines, tens
+    of turns each."""
+    n, nx, ny, cell = 3000, 48, 40, 2e-4
+    uvw = _uv(n, 216, 150, cell, supp)
+    uvw[:, 2] *= 50.0
+    freq = np.array([1e9])
+    rng = np.random.default_rng(supp)
+    vis = rng.standard_normal((n, 1)) + 1j * rng.standard_normal((n, 1))
+    img = rng.standard_normal((nx, ny))
+    kw = dict(uvw=uvw, freq=freq, pixsize_x=cell, pixsize_y=cell, epsilon=1e-9, center_x=0.03, center_y=-0.02,
+              kernel=(_kernel(supp, False), 216, 150))
+    # Both sides' phases in float64; the oracle's angle is rounded before it is
+    # reduced, 2^-53 of 100 turns (1e-13).
+    for got, ref in ((gridder.vis2dirty(vis=vis, npix_x=nx, npix_y=ny, **kw),
+                      oracle.vis2dirty(vis=vis, npix_x=nx, npix_y=ny, **kw)),
+                     (gridder.dirty2vis(dirty=img, **kw), oracle.dirty2vis(dirty=img, **kw))):
+        assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("single", [True, False])
 @pytest.mark.parametrize("supp,nu,nv,nx,ny", [(4, 4, 4, 2, 2), (4, 4, 14, 2, 6), (4, 6, 4, 2, 2), (5, 6, 6, 2, 2),
                                               (5, 8, 6, 4, 2), (6, 6, 8, 2, 4), (7, 8, 8, 4, 2), (8, 8, 10, 4, 4)])
