@@ -33,6 +33,11 @@ visibilities and mask: the reference's two stateless calls.
   harness runs it (a fresh process per repeat, three repeats, the median, all
   threads and one, peak RSS and output SHA256).
 
+The one line on stdout holds the headline (`headline`: the keys above
+`accuracy`, its default method's errors, and one figure of each other leg);
+the whole report, legs included, goes to stderr as one line of JSON after it
+is complete, and to the file that `--details` names.
+
 `--impl reference` times the CPU oracle alone, on the same workload sample.
 Multi-GPU (`--gpus N` under torchrun): independent replicas, one per GPU.
 """
@@ -95,6 +100,7 @@ def parse():
     ap.add_argument("--no-msv4", action="store_true")
     ap.add_argument("--learned-patches", type=int, default=20000)
     ap.add_argument("--learned-steps", type=int, default=2500)
+    ap.add_argument("--details", default=None, metavar="PATH", help="write the whole report (every leg) to PATH")
     ap.add_argument("--trace-e2e", default=None, metavar="PATH",
                     help="after the e2e leg, one more e2e step under the PyTorch profiler (CUDA activity), "
                          "its trace written to PATH (Chrome trace JSON)")
@@ -1016,6 +1022,45 @@ def run_config1(dev, args):
     return out
 
 
+# ------------------------------------------------------------------ the report
+
+
+def headline(report):
+    """The report's headline: every key that says what was timed and how, and of
+    the legs one figure each. Short, so that a log that keeps the last few
+    kilobytes keeps the line whole."""
+
+    def short(o):  # seven significant digits
+        if isinstance(o, dict):
+            return {k: short(v) for k, v in o.items()}
+        if isinstance(o, (list, tuple)):
+            return [short(v) for v in o]
+        return float(f"{o:.7g}") if isinstance(o, float) else o
+
+    def some(d, *keys):
+        return None if d is None else {k: d[k] for k in keys if k in d}
+
+    legs = ("accuracy", "config1", "fista", "imaging_weights", "msv4_ingest")
+    head = {k: v for k, v in report.items() if k not in legs and k != "stages_ms"}
+    roof = dict(report["roofline"])
+    roof.pop("traffic_source", None)
+    roof["compute"] = some(roof["compute"], "achieved_tflops", "fp32_fma_peak_tflops", "frac")
+    head["roofline"] = roof
+    cpu = report["cpu_baseline"]
+    head["cpu_baseline"] = some(cpu, "value", "unit", "cores", "kind", "sample", "cpu_model", "simd")
+    if cpu and "two_sample_model" in cpu:
+        head["cpu_baseline"]["whole_workload"] = cpu["two_sample_model"]["whole_workload_mvis_per_s"]
+    if report["accuracy"]:
+        head["accuracy"] = some(report["accuracy"]["methods"][0], "method", "epsilon", "dirty_border_linf",
+                                "dirty_interior_linf", "dirty_rms", "vis_linf", "vis_rms")
+    if report["fista"]:
+        f = report["fista"]
+        head["fista"] = some(f, "target_rms", "time_to_target_s")
+        if f.get("learned"):
+            head["fista"]["learned_time_to_target_s"] = f["learned"].get("time_to_target_s")
+    return short(head)
+
+
 # ------------------------------------------------------------------ GPU
 
 
@@ -1132,7 +1177,10 @@ def run_b200(args):
                      + npix * npix * vb // 2)
     alg = {"grid": per_direction, "degrid": per_direction}
     dom = max(("grid", "degrid"), key=lambda k: prof[k][1])
-    kernel = ({"grid": "k_grid_i8", "degrid": "k_degrid_h"} if single else {"grid": "k_grid_f64", "degrid": "k_degrid"})[dom]
+    if single:
+        kernel = {"grid": "k_grid_i8", "degrid": "k_degrid_h"}[dom]
+    else:
+        kernel = {"grid": "k_grid_f64", "degrid": "k_degrid_f64"}[dom] if supp <= 8 else {"grid": "k_grid", "degrid": "k_degrid"}[dom]
     dom_launches, dom_ms = prof[dom]
     per_launch_s = dom_ms / max(dom_launches, 1) / 1e3
     achieved = alg[dom] / per_launch_s / 1e9
@@ -1272,7 +1320,7 @@ def run_b200(args):
         msv4_leg = run_msv4()
 
     if rank == 0:
-        line = {
+        report = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": args.precision, "data": "synthetic",
@@ -1283,7 +1331,11 @@ def run_b200(args):
             "msv4_ingest": msv4_leg,
             "stages_ms": {k: round(v[1], 3) for k, v in prof.items() if v[0]},
         }
-        print(json.dumps(line, default=_plain), flush=True)
+        whole = json.dumps(report, default=_plain)
+        if args.details:
+            Path(args.details).write_text(whole + "\n")
+        print(whole, file=sys.stderr, flush=True)
+        print(json.dumps(headline(json.loads(whole))), flush=True)
     if dist is not None:
         dist.barrier()
         dist.destroy_process_group()

@@ -96,3 +96,43 @@ def test_reference_sample_is_as_large_as_the_run_allows():
     assert bench.reference_stride(20, 3) == 16
     assert bench.reference_stride(40, 3) == 32
     assert bench.reference_stride(100, 5) == 64
+
+
+def test_the_headline_line_is_short_and_whole():
+    """One line of less than 2.5 kB with every key that says what was timed,
+    whatever the legs hold."""
+    import json
+
+    bench = _bench()
+    x = 1234.567890123456
+    report = {"metric": bench.METRIC, "value": x, "unit": bench.UNIT, "n_gpus": 8, "steps": 20, "warmup": 5,
+              "ms_per_step": x, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
+              "data": "synthetic",
+              "config": bench.workload_config(bench.synth.WORKLOADS[bench.WORKLOAD], bench.WORKLOAD, 1e-5, 8, "f32"),
+              "plan": dict.fromkeys(("kernel_index", "supp", "nu", "nv", "nplanes", "active"), 1056964608),
+              "roofline": {"bound": "hbm", "kernel": "k_degrid_h", "achieved": x, "peak": x, "unit": "GB/s", "frac": x,
+                           "peak_kind": "measured", "traffic": 1e12 * x, "traffic_source": "t" * 300,
+                           "algorithmic_bytes_per_launch": 23834301376, "avg_launch_ms": x, "share_of_step": x,
+                           "compute": {"useful_tflop_per_launch": x, "achieved_tflops": x, "fp32_fma_peak_tflops": x,
+                                       "peak_kind": "p" * 50, "frac": x}},
+              "cpu_baseline": {"value": x, "unit": bench.UNIT, "cores": 224, "kind": "port", "sample": "s" * 250,
+                               "cpu_model": "c" * 60, "simd": "avx512", "step_s": [x] * 3,
+                               "two_sample_model": {"whole_workload_mvis_per_s": x, "note": "n" * 100}},
+              "e2e": {"value": x, "unit": bench.UNIT, "h2d_bytes_per_step": 10686316544,
+                      "d2h_bytes_per_step": 8522825728, "ms_per_step": x},
+              "gpu_launches": 2220, "clocks": {"sm_mhz": x, "sm_max_mhz": x, "reasons": ["sw_power_cap"], "samples": 99},
+              "accuracy": {"methods": [{"method": "int8", "epsilon": 1e-5, "dirty_border_linf": x / 1e9,
+                                        "dirty_interior_linf": x / 1e9, "dirty_rms": x / 1e9, "vis_linf": x / 1e9,
+                                        "vis_rms": x / 1e9, "stages_per_round_trip": {str(i): x for i in range(99)}}] * 9},
+              "config1": {str(i): x for i in range(200)}, "imaging_weights": {"a": x}, "msv4_ingest": None,
+              "fista": {"target_rms": 0.06, "time_to_target_s": x, "rms_trajectory": [x] * 300,
+                        "learned": {"time_to_target_s": x, "conv3_kernels": [x] * 300}},
+              "stages_ms": {str(i): x for i in range(14)}}
+    head = bench.headline(report)
+    assert len(json.dumps(head)) < 2500
+    for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+              "vs_baseline", "dtype", "data", "config", "roofline", "cpu_baseline", "e2e", "gpu_launches", "clocks"):
+        assert k in head
+    assert head["value"] == 1234.568 and head["gpu_launches"] == 2220 and head["e2e"]["h2d_bytes_per_step"] == 10686316544
+    report.update(accuracy=None, fista=None, cpu_baseline=None, e2e={"unavailable": "pinned host memory"})
+    assert bench.headline(report)["e2e"] == {"unavailable": "pinned host memory"}
