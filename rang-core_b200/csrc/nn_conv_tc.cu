@@ -4,10 +4,10 @@
 // the accumulators in tensor memory (TMEM), operands in shared memory, fetched
 // by the tensor memory accelerator (TMA).
 //
-// What bounds it is the traffic from L2 into shared memory (about 38 bytes per
-// clock and SM here): a tile fetched anew for each of the nine taps, with its
-// weights, took 30 % of the tensor peak on the widest layers and 15 % on the
-// narrow ones. So a K step is one horizontal shift (dx) of KC = 64 or 32 input
+// What bounded it was the traffic from L2 into shared memory (about 38 bytes per
+// clock and SM): a tile fetched anew for each of the nine taps, with its weights,
+// reached 30 % of the tensor peak on the widest layers and 15 % on the narrow ones.
+// So a K step is one horizontal shift (dx) of KC = 64 or 32 input
 // channels: one 4-D TMA box (KC channels, 8 columns, 18 rows, 1 image) from a
 // row above the patch, in the 128- or 64-byte swizzled K-major layout. A row
 // of eight pixels is one 8-row group of that layout, so the three vertical
@@ -33,6 +33,11 @@
 // mask, bf16) while the next patches are multiplied into the other half of
 // TMEM. Four epilogue warps, one per scheduler, took longer over their chains
 // of dependent instructions than the loads and MMAs of a narrow layer.
+//
+// No unit is full now: at batch 8 the tcgen05 pipe is active 54 % of the time on
+// 256^2 x 32 -> 32 channels and 56 % on 64^2 x 384 -> 128, L2 into the SMs takes 7
+// and 18 % of its rate. What is left is the latency of loads, MMAs and epilogue
+// over the few groups of patches that a block has.
 //
 // The weight gradient (k_conv3_dw_tc, further down) is the same machinery with
 // K = pixels and both operands read channel-contiguous (MN-major).

@@ -815,8 +815,9 @@ __device__ __forceinline__ void block_sync() {
 // half the depth. The next round's records and values are loaded while the
 // current round is contracted.
 //
-// It is bound by issue and by latency at 11 warps per SM (59 % of the issue
-// slots, the integer tensor pipe 21 %). 1.06 G visibilities of support 6 took
+// It is bound by the latency of its own chains at 11 warps per SM: on 106 M
+// active visibilities of support 6 54 % of the issue slots and 24 % of the
+// integer tensor pipe are used. 1.06 G visibilities of support 6 took
 // 31.3 ms while every bin flushed its whole window and staging ran on scalar
 // multiply-adds in blocks of 8192 records, 26.2 now; 54 M of support 8, where
 // bins are sparse and the flush's atomics were the bound, 19.6 and 6.1.
@@ -1030,10 +1031,11 @@ struct DegridOut {
 // registers) and 20 (96), and as fast as 28. The w contraction before the u
 // taps and one output lane per record (two lanes of each quad) measured 10 %
 // faster than u first and one lane writing both records. From support 7, 16
-// (128 registers) against 12 took 5.5 ms against 6.1 at 54 M visibilities.
-// It is bound by issue (69 % of the slots, the FP16 tensor pipe 45 %). That
+// (128 registers) against 12 took 5.5 ms against 6.1 at 54 M visibilities. That
 // call took 12.5 ms while a warp read the whole window of every bin; 1.06 G
-// visibilities of support 6, 27.6 then and 26.3 now.
+// visibilities of support 6, 27.6 then and 26.3 now. It is bound by issue and the
+// FP16 tensor pipe: 65 % of the slots and 51 % of the pipe on 106 M active
+// visibilities of support 6.
 template <int S>
 __global__ void __launch_bounds__(H16_BATCH, h16_blocks(S))
     k_degrid_h(const __grid_constant__ Geom<float> g, Inputs wts, const VisRecord* __restrict__ rec,

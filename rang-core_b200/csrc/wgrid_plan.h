@@ -169,7 +169,7 @@ class Plan {
   int kernel_errors(cudaStream_t s) const;
 
   // For the tests: per visibility (row-major) the reference's bin key
-  // tile * nbuckets + first plane (0xffffffff inactive), and the sorted order.
+  // tile * max(nplanes, 1) + first plane (0xffffffff inactive), and the sorted order.
   void export_binning(uint32_t* key_host, uint32_t* sorted_host, cudaStream_t s) const;
   // Per visibility iu0, iv0 (int64) from the device arithmetic, for the tests.
   void export_pixels(const Inputs& act, bool with_vis, int64_t* iu0_host, int64_t* iv0_host, cudaStream_t s) const;
@@ -249,8 +249,8 @@ class Plan {
 // rounded into the fixed-point grid, also order-independent). The float
 // tensor-core methods sum blocks of visibilities inside the tensor core, so
 // their results depend on the sorted order, which the counting sort's
-// atomics leave free. Double precision always uses FP64 CUDA-core products
-// rounded into the fixed-point grid. The environment variable
+// atomics leave free. Double precision always uses FP64 products (tensor cores
+// up to support 8) rounded into the fixed-point grid. The environment variable
 // RANG_WGRIDDER_GPU_METHOD (int8 | fp32 | tf32x3 | bf16x3) sets the default.
 enum GridMethod : int { GRID_FP32 = 0, GRID_TF32X3 = 1, GRID_BF16X3 = 2, GRID_INT8 = 3 };
 int grid_method();
