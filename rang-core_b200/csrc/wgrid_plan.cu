@@ -2630,9 +2630,7 @@ template <class T>
 void Plan<T>::build_layout(const Inputs& act, bool with_vis, const uint32_t* bits, cudaStream_t s) {
   ntiles_ = (size_t)g_.ntu * g_.ntv;
   nbins_ = ntiles_ * (size_t)g_.nbuckets * (size_t)g_.nsub;
-  // The limit counts every plane as a first plane, as the keys of the binning's export do.
-  if (ntiles_ * (size_t)std::max(g_.nplanes, 1) * (size_t)g_.nsub >= 0xffffffffull)
-    throw InvalidArgument("too many uv tiles and w-planes for one call");
+  if (too_many_bins()) throw InvalidArgument("too many uv tiles and w-planes for one call");
   if ((size_t)nchunk_ * nbins_ >= 0xffffffffull) {
     // Row chunks are an optimisation: as many as the 32-bit key space holds
     // (chunks x bins keys, below the inactive key), down to one.
@@ -3148,7 +3146,7 @@ void Plan<T>::degrid_to(const T* image, const Inputs& wts, T* vis, const void* f
     const size_t np = (size_t)std::max(g_.nplanes, 1), pl = (size_t)g_.nu * g_.nv;
     const size_t npx = (size_t)o_.nx * o_.ny, tpl = (size_t)g_.ny * g_.nu;
     stream_bins = sizeof(T) == 4 && !fused && windows() && nchunk_ > 1 &&
-                  (size_t)nchunk_ * nb < 0xffffffffull &&
+                  (size_t)nchunk_ * nb < 0xffffffffull && !too_many_bins() &&
                   plane_group(pl * sizeof(cplx<T>), tpl * sizeof(cplx<T>) + npx * sizeof(T)) >= np;
     if (stream_bins) {
       ntiles_ = (size_t)g_.ntu * g_.ntv;

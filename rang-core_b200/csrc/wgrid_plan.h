@@ -175,6 +175,11 @@ class Plan {
   void export_pixels(const Inputs& act, bool with_vis, int64_t* iu0_host, int64_t* iv0_host, cudaStream_t s) const;
 
  private:
+  // Whether the bins pass the 32-bit keys. Every plane counts as a first plane, as
+  // in the keys of the binning's export.
+  bool too_many_bins() const {
+    return (size_t)g_.ntu * g_.ntv * (size_t)std::max(g_.nplanes, 1) * (size_t)g_.nsub >= 0xffffffffull;
+  }
   void build_layout(const Inputs& act, bool with_vis, const uint32_t* bits, cudaStream_t s);
   // Per row the binning's coordinates and sign (double4, nrow_ of them).
   void row_coords(DevBuf& out, cudaStream_t s) const;

@@ -122,3 +122,20 @@ def test_chunked_vis2dirty_regrids_when_the_bound_changes(chunks, k, change):
     assert np.array_equal(out.view(np.uint8), ref.view(np.uint8))
     oref = oracle.vis2dirty(vis=vis, wgt=wgt, mask=mask, **kw)
     assert rel_linf(out, oref) < TOL[True]
+
+
+@pytest.mark.parametrize("k", [1, 2])
+def test_more_bins_than_keys_are_refused_in_every_form(chunks, k):
+    """A grid of 24576^2 at support 8: the streamed binning refuses what the whole
+    one refuses."""
+    from rang import gridder
+
+    chunks(k)
+    kernel = next(i for i, r in enumerate(gridder.kernel_table()) if r[0] == 8 and r[5] == 3 and r[6])
+    rng = np.random.default_rng(0)
+    uvw, freq = rng.uniform(-100.0, 100.0, (64, 3)), np.array([1e9])
+    kw = dict(uvw=uvw, freq=freq, pixsize_x=1e-5, pixsize_y=1e-5, epsilon=1e-3, kernel=(kernel, 24576, 24576))
+    with pytest.raises(ValueError, match="too many uv tiles"):
+        gridder.dirty2vis(dirty=np.ones((32, 32), np.float32), **kw)
+    with pytest.raises(ValueError, match="too many uv tiles"):
+        gridder.vis2dirty(vis=np.ones((64, 1), np.complex64), npix_x=32, npix_y=32, **kw)
