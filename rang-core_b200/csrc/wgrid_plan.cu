@@ -1904,8 +1904,8 @@ struct FftPlan {
   std::atomic<bool> captured{false};  // a graph may hold its kernels
   std::mutex mu;
 
-  ~FftPlan() {  // after the transforms in flight
-    if (!h) return;
+  ~FftPlan() {  // after the transforms in flight; not where a graph may run more
+    if (!h || captured.load()) return;
     int cur = dev;
     cudaGetDevice(&cur);
     if (cur != dev) cudaSetDevice(dev);
